@@ -271,8 +271,8 @@ extern "C" int p3m_destroy(p3m_ctx *ctx)
                     s.cell_sub,
                     s.nlist, s.rebuild, s.rb_list, s.pos_ref, s.pp_tables,
                     s.nnb_in, s.nlist_in, s.prune, s.pos_pref, s.prune_count,
-                    s.acc_pp, s.brick_key, s.brick_count, s.brick_start, s.brick_cursor,
-                    s.brick_perm, s.brick_slot, s.brick_hist, s.tiles, s.spec, s.ek, s.green, s.efield,
+                    s.acc_pp, s.brick_key, s.brick_rank, s.brick_count, s.brick_start,
+                    s.brick_slot, s.slot_pt, s.slot_q, s.tiles, s.spec, s.ek, s.green, s.efield,
                     s.acc_pm, s.twiddle, s.u_pp_part, s.u_pm_part, s.kin_part, s.rep_out,
                     s.status, ctx->counters, ctx->ring, ctx->qmult, ctx->nqt_part, ctx->snap,
                     ctx->snap_steps,
@@ -306,6 +306,8 @@ template <typename T> static int alloc_bulk(p3m_ctx *ctx)
     CK(valloc(&s.acc_pp, (size_t)s.ntot * sizeof(T4)));
     if (s.has_mesh) {
         CK(valloc(&s.acc_pm, (size_t)s.ntot * sizeof(T4)));
+        CK(valloc(&s.slot_pt, (size_t)s.ntot * sizeof(T4)));
+        CK(valloc(&s.slot_q, (size_t)s.ntot * sizeof(T)));
         CK(valloc(&s.spec, (size_t)s.nspec * sizeof(C)));
         CK(valloc(&s.ek, (size_t)3 * s.nspec * sizeof(C)));
         CK(valloc(&s.green, (size_t)s.nspec * sizeof(T)));
@@ -374,15 +376,7 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     s.nrep = n_reps;
     s.has_mesh = with_mesh;
     ctx->rh.resize(n_reps);
-    long long mesh = 0, spec = 0, tile = 0, hist = 0;
-    int nchunk = 0, max_bricks = 0;
-    // brick-sort chunks: about 4 per SM over the whole batch (one warp each
-    // places its particles), 256 to 4096 particles, a multiple of 32
-    long long ntot_all = 0;
-    for (int r = 0; r < n_reps; ++r) ntot_all += reps[r].n;
-    int sort_ch = (int)std::min<long long>(4096, std::max<long long>(256, (ntot_all + 591) / 592));
-    sort_ch = (sort_ch + 31) / 32 * 32;
-    s.sort_ch = sort_ch;
+    long long mesh = 0, spec = 0, tile = 0;
     int p = 0, cell = 0, brick = 0, wc_cap = 0, blk = 0, maxm = 0;
     for (int r = 0; r < n_reps; ++r) {
         const p3m_replica_desc &d = reps[r];
@@ -414,11 +408,6 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
             R.mesh_off = mesh;
             R.spec_off = spec;
             R.tile_off = tile;
-            R.sc_off = nchunk;
-            R.sh_off = hist;
-            nchunk += (d.n + sort_ch - 1) / sort_ch;
-            hist += (long long)((d.n + sort_ch - 1) / sort_ch) * R.nb * R.nb * R.nb;
-            if (R.nb * R.nb * R.nb > max_bricks) max_bricks = R.nb * R.nb * R.nb;
             brick += R.nb * R.nb * R.nb;
             mesh += (long long)M * M * M;
             spec += (long long)(M / 2 + 1) * M * M;
@@ -452,6 +441,7 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     s.ntile = tile;
     s.plane_max = plane_max_mesh();
     s.gather_mode = 1;
+    s.assign_parts = assign_parts_for(brick);
     plan_mesh_passes(ctx);
     s.nblk = blk;
     s.max_mesh = maxm;
@@ -517,13 +507,9 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(dalloc(&s.cell_perm, (size_t)p));
     CKC(dalloc(&s.cell_slot, (size_t)p));
     CKC(dalloc(&s.brick_key, (size_t)p));
-    CKC(dalloc(&s.brick_count, (size_t)brick));
+    CKC(dalloc(&s.brick_rank, (size_t)p));
+    CKC(dalloc(&s.brick_count, (size_t)brick * BRICK_CNT_STRIDE));
     CKC(dalloc(&s.brick_start, (size_t)brick + 1));
-    CKC(dalloc(&s.brick_cursor, (size_t)brick));
-    CKC(dalloc(&s.brick_perm, (size_t)p));
-    s.nchunk = nchunk;
-    s.max_bricks = max_bricks;
-    CKC(dalloc(&s.brick_hist, (size_t)hist));
     CKC(dalloc(&s.brick_slot, (size_t)p));
     if (with_mesh)
         CKC(valloc(&s.tiles, (size_t)tile * (precision == P3M_FP32 ? sizeof(float) : sizeof(double))));
@@ -582,8 +568,8 @@ template <typename T> static void seq_sort(p3m_ctx *ctx, bool keys)
     launch_build_lists<T>(s, ctx->st);  // from those coordinates (rebuild steps)
     ctx->launches += 5;
     if (s.has_mesh) {
-        launch_sort_bricks(s, ctx->st);
-        ctx->launches += 3;
+        launch_place_bricks<T>(s, ctx->st);
+        ctx->launches++;
     }
 }
 
@@ -668,8 +654,8 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
                 launch_scan(s, st2, 1);
-                launch_sort_bricks(s, st2);
-                ctx->launches += 4;
+                launch_place_bricks<T>(s, st2);
+                ctx->launches += 2;
                 seq_pm<T>(ctx, false, st2);
                 e = cudaEventRecord(ctx->ev_join, st2);
             }

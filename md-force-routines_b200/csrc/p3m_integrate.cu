@@ -35,8 +35,8 @@ __device__ __forceinline__ double wrap_once(double x, double L)
 __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                              double *__restrict__ pos, double *__restrict__ vel,
                              const double *__restrict__ acc, const double *__restrict__ pos_ref,
-                             int ntot, int *__restrict__ brick_key, int *__restrict__ brick_count,
-                             int has_mesh, int *rebuild, int *status,
+                             int ntot, int *__restrict__ brick_key, int *__restrict__ brick_rank,
+                             int *__restrict__ brick_count, int has_mesh, int *rebuild, int *status,
                              const double *__restrict__ pos_pref, int *prune)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
@@ -71,7 +71,7 @@ __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restr
         particle_keys(R, x[0], x[1], x[2], has_mesh, nullptr, &b, status);
         if (b >= 0) {
             brick_key[i] = b;
-            atomicAdd(&brick_count[b], 1);
+            brick_rank[i] = atomicAdd(&brick_count[b * BRICK_CNT_STRIDE], 1);
         }
     }
 }
@@ -561,7 +561,7 @@ void launch_kick_drift(const DevState &s, cudaStream_t st)
 {
     const bool inner = s.prune_buf > 0.0;
     k_kick_drift<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
-                                                s.ntot, s.brick_key, s.brick_count, s.has_mesh,
+                                                s.ntot, s.brick_key, s.brick_rank, s.brick_count, s.has_mesh,
                                                 s.rebuild, s.status, inner ? s.pos_pref : nullptr,
                                                 s.prune);
 }

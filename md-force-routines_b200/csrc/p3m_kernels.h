@@ -56,10 +56,13 @@ struct DevState {
     float4 *pp_tables = nullptr; // FP32 pair tables: cubic of psi = phi r, [nrep][PP_TABLE_N]
     void *acc_pp = nullptr;      // V4<T> PP acceleration, cell-sorted order
     // brick sort
-    int *brick_key = nullptr, *brick_count = nullptr, *brick_start = nullptr;
-    int *brick_cursor = nullptr, *brick_perm = nullptr, *brick_slot = nullptr;
-    int *brick_hist = nullptr;   // [replica][chunk][brick] counts, then chunk offsets
-    int nchunk = 0, max_bricks = 0, sort_ch = 2048;  // chunks, bricks of the largest mesh, chunk size
+    int *brick_key = nullptr, *brick_rank = nullptr;  // per particle: brick, arrival rank in it
+    int *brick_count = nullptr;  // [nbrick * BRICK_CNT_STRIDE], zero between sorts
+    int *brick_start = nullptr, *brick_slot = nullptr;
+    // the particles in brick order: V4<T> (stencil offsets x, y, z, packed
+    // base in the brick) and T charge per slot
+    void *slot_pt = nullptr, *slot_q = nullptr;
+    int assign_parts = 1;        // CTAs per brick in the charge assignment (z ranges of its tile)
     // mesh
     void *tiles = nullptr;       // T assignment tiles [brick][TILE^3]
     void *spec = nullptr;        // C2<T> half spectrum rho_k / phi_k, [kx][z][y]
@@ -87,13 +90,14 @@ void launch_cell_keys(const DevState &s, cudaStream_t st);
 void launch_scan(const DevState &s, cudaStream_t st, int part = -1);  // -1 both, 0 cells, 1 bricks
 void launch_scatter(const DevState &s, cudaStream_t st);
 template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st);
-void launch_sort_bricks(const DevState &s, cudaStream_t st);  // 3 kernels
+template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t st);
 template <typename T> void launch_quantize(const DevState &s, cudaStream_t st);
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st);
 template <typename T> void launch_pp(const DevState &s, cudaStream_t st);
 int pp_particles_per_block(int tpi);
 void launch_reduce_pp(const DevState &s, cudaStream_t st);
 
+int assign_parts_for(int nbrick);
 template <typename T> void launch_assign(const DevState &s, cudaStream_t st);
 template <typename T> void launch_fft_forward(const DevState &s, cudaStream_t st);
 template <typename T> void launch_fft_inverse(const DevState &s, cudaStream_t st);

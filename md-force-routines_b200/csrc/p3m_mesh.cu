@@ -23,10 +23,9 @@
 //   efield  T     [3][z][y][x]      real field meshes, x fastest
 //
 // Assignment is deterministic: each CTA owns one brick of BRICK^3 base
-// cells and adds its particles' 216-node stencils into a shared-memory tile
-// of TILE^3 nodes, in FP64 in a fixed particle order without atomics
-// (k_assign), or in FP32 with order-independent integer atomics
-// (k_assign_i32).
+// cells (or a z range of its tile) and adds its particles' 216-node stencils
+// into a shared-memory tile of TILE^3 nodes with fixed-point integer atomics,
+// whose sums do not depend on the order of the adds (k_assign).
 // Overlapping tile halos are summed in a fixed order when the first FFT pass
 // reads the mesh.
 //
@@ -176,198 +175,142 @@ __device__ __forceinline__ void fft_lines_t(cplx<T> *buf, int ls, int es, int lo
 // Charge assignment
 // ---------------------------------------------------------------------------
 
-// Order-6 weights at node offset x (yukawa_pm_ord6.py:29-34).
+// Order-6 weights at node offset x (yukawa_pm_ord6.py:29-34), from the even
+// and odd parts that mirrored nodes share: w[5 - c](x) = w[c](-x), and the
+// outermost are (1 -+ 2x)^5 / 3840. Coefficients are divided by 3840 and 1920
+// beforehand (the six divisions per axis were a third of the instructions of
+// an FP64 stencil).
 template <typename T>
 __device__ __forceinline__ void weights6(T x, T *w)
 {
-    T x2 = x * x, x3 = x2 * x, x4 = x3 * x, x5 = x4 * x;
-    w[0] = ((T)1 - (T)10 * x + (T)40 * x2 - (T)80 * x3 + (T)80 * x4 - (T)32 * x5) / (T)3840;
-    w[1] = ((T)237 - (T)750 * x + (T)840 * x2 - (T)240 * x3 - (T)240 * x4 + (T)160 * x5) / (T)3840;
-    w[2] = ((T)841 - (T)770 * x - (T)440 * x2 + (T)560 * x3 + (T)80 * x4 - (T)160 * x5) / (T)1920;
-    w[3] = ((T)841 + (T)770 * x - (T)440 * x2 - (T)560 * x3 + (T)80 * x4 + (T)160 * x5) / (T)1920;
-    w[4] = ((T)237 + (T)750 * x + (T)840 * x2 + (T)240 * x3 - (T)240 * x4 - (T)160 * x5) / (T)3840;
-    w[5] = ((T)1 + (T)10 * x + (T)40 * x2 + (T)80 * x3 + (T)80 * x4 + (T)32 * x5) / (T)3840;
+    const T x2 = x * x;
+    const T a = (T)1 - (T)2 * x, b = (T)1 + (T)2 * x;
+    const T a2 = a * a, b2 = b * b;
+    w[0] = a2 * a2 * (a * (T)(1.0 / 3840));
+    w[5] = b2 * b2 * (b * (T)(1.0 / 3840));
+    const T e1 = (T)(237.0 / 3840) + x2 * ((T)(840.0 / 3840) + x2 * (T)(-240.0 / 3840));
+    const T o1 = x * ((T)(750.0 / 3840) + x2 * ((T)(240.0 / 3840) + x2 * (T)(-160.0 / 3840)));
+    w[1] = e1 - o1;
+    w[4] = e1 + o1;
+    const T e2 = (T)(841.0 / 1920) + x2 * ((T)(-440.0 / 1920) + x2 * (T)(80.0 / 1920));
+    const T o2 = x * ((T)(770.0 / 1920) + x2 * ((T)(-560.0 / 1920) + x2 * (T)(160.0 / 1920)));
+    w[2] = e2 - o2;
+    w[3] = e2 + o2;
 }
 
-// Base index (unwrapped) and offset along one axis (yukawa_pm_ord6.py:17-27).
-__device__ __forceinline__ int base_offset(double p, double h, double &off)
-{
-    int ix = (int)floor(p / h);
-    off = (p - (ix + 0.5) * h) / h;
-    return ix;
-}
-
-__device__ __forceinline__ int wrapM(int i, int M)
-{
-    i %= M;
-    return i < 0 ? i + M : i;
-}
-
-// One CTA of A_WARPS warps per brick. The brick's particles come in a fixed
-// order (ascending particle index, from the brick sort); their weights are
-// computed once per chunk; then warp w adds the stencils of all particles,
-// in that order, to the tile planes z = w (mod 6) only -- exactly one of each
-// particle's six planes, 36 nodes, spread over the lanes. No two warps
-// touch the same node and each warp adds its particles one after another, so
-// every node receives its contributions in the same order on every run and
-// no atomics are needed.
-constexpr int A_WARPS = 6;
-constexpr int A_THREADS = 32 * A_WARPS;
-constexpr int A_CHUNK = 128;   // particles per weight chunk
-
-template <typename T> struct AssignW {
-    T wx[6], wy[6], wz[6];  // wx carries the charge
-    int base;               // (lz * TILE + ly) * TILE + lx, or -1
-    int lz;
-};
-
-template <typename T> constexpr size_t assign_smem()
-{
-    return (size_t)TILE3 * sizeof(T) + (size_t)A_CHUNK * sizeof(AssignW<T>);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(A_THREADS)
-k_assign(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
-         const int *__restrict__ brick_perm, const double *__restrict__ pos,
-         const double *__restrict__ charge, T *__restrict__ tiles, int nbrick, int *status)
-{
-    extern __shared__ __align__(16) unsigned char a_smem[];
-    T *tile = reinterpret_cast<T *>(a_smem);
-    AssignW<T> *W = reinterpret_cast<AssignW<T> *>(a_smem + (size_t)TILE3 * sizeof(T));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // this lane's nodes (dy, dx) of a particle's plane: node = lane + 32 pass < 36
-    const int n0 = lane, n1 = lane + 32;
-    const int off0 = (n0 / 6) * TILE + n0 % 6, off1 = (n1 / 6) * TILE + n1 % 6;
-    const bool has1 = n1 < 36;
-    for (int b = blockIdx.x; b < nbrick; b += gridDim.x) {
-        const int r = find_rep(b, nrep, [&](int k) { return reps[k].brick_off; });
-        const RepDev &R = reps[r];
-        const int nb = R.nb, M = R.M, local = b - R.brick_off;
-        const int bx = (local % nb) * BRICK, by = ((local / nb) % nb) * BRICK,
-                  bz = (local / (nb * nb)) * BRICK;
-        const int p0 = brick_start[b];
-        const int n = brick_start[b + 1] - p0;
-        __syncthreads();
-        for (int k = threadIdx.x; k < TILE3; k += A_THREADS) tile[k] = (T)0;
-        for (int c0 = 0; c0 < n; c0 += A_CHUNK) {
-            const int cn = min(A_CHUNK, n - c0);
-            __syncthreads();
-            for (int k = threadIdx.x; k < cn; k += A_THREADS) {
-                const int i = brick_perm[p0 + c0 + k];
-                double ox, oy, oz;
-                const int ix = base_offset(pos[3 * i + 0], R.h, ox);
-                const int iy = base_offset(pos[3 * i + 1], R.h, oy);
-                const int iz = base_offset(pos[3 * i + 2], R.h, oz);
-                const int lx = wrapM(ix, M) - bx, ly = wrapM(iy, M) - by, lz = wrapM(iz, M) - bz;
-                AssignW<T> w;
-                // a particle outside [-L, 2L) was filed under brick 0 and
-                // flagged by the key pass; it must not reach outside the tile
-                if ((unsigned)lx < (unsigned)BRICK && (unsigned)ly < (unsigned)BRICK &&
-                    (unsigned)lz < (unsigned)BRICK) {
-                    weights6<T>((T)ox, w.wx);
-                    weights6<T>((T)oy, w.wy);
-                    weights6<T>((T)oz, w.wz);
-                    const T q = (T)charge[i];
-#pragma unroll
-                    for (int c = 0; c < 6; ++c) w.wx[c] *= q;
-                    w.base = (lz * TILE + ly) * TILE + lx;
-                    w.lz = lz;
-                } else {
-                    w.base = -1;
-                    w.lz = 0;
-                }
-                W[k] = w;
-            }
-            __syncthreads();
-            for (int k = 0; k < cn; ++k) {
-                const AssignW<T> &w = W[k];
-                if (w.base < 0) continue;  // uniform over the block
-                // this warp's plane of the particle: lz <= lz + d < lz + 6
-                const int d = ((warp - w.lz) % A_WARPS + A_WARPS) % A_WARPS;
-                T *plane = tile + w.base + d * TILE * TILE;
-                const T wz = w.wz[d];
-                plane[off0] += wz * w.wy[n0 / 6] * w.wx[n0 % 6];
-                if (has1) plane[off1] += wz * w.wy[n1 / 6] * w.wx[n1 % 6];
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        T *dst = tiles + R.tile_off + (long long)local * TILE3;
-        for (int k = threadIdx.x; k < TILE3; k += A_THREADS) dst[k] = tile[k];
-    }
-}
-
-// FP32 path: one CTA of 256 threads per brick, thread per particle, the 216
-// contributions added to a shared tile with 32-bit integer atomics -- integer
-// sums do not depend on the order of the adds, so the result is the same on
-// every run. Each contribution q w is scaled by S = 2^k, the largest power of
-// two with 0.17 n |q|max S <= 2^22 for the brick's n particles (0.17 bounds a
-// product of three order-6 weights), so no node sum can exceed 2^22 in
-// magnitude. t = q w S is split exactly into an integer part and an fb-bit
+// One CTA of 256 threads per brick, a thread per particle, the 216
+// contributions added to a shared tile with integer atomics -- integer sums
+// do not depend on the order of the adds, so the result is the same on every
+// run, and the brick sort need not order a brick's particles. Each
+// contribution q w is scaled by S = 2^k, the largest power of two with
+// 0.17 n |q|max S <= 2^B for the brick's n particles (0.17 bounds a product
+// of three order-6 weights; |q|max of the replica, in FP64 of the brick), so
+// no node sum can exceed 2^B in magnitude. A node is two int32 words:
+//
+// FP32, B = 22: t = q w S is split exactly into an integer part and an fb-bit
 // fraction with the 1.5 * 2^23 rounding constant (exact for |t| < 2^22, no
-// float <-> int conversions) and the two parts go to two int32 tiles: the node
-// value is (hi + lo / 2^fb) / S, resolved to 2^-fb / S. fb = 16, or fewer for
-// bricks of more than 2^14 particles, so that the n fractions of a node (each
-// at most 2^fb) cannot overflow: n 2^fb <= 2^30.
-constexpr int A32_THREADS = 256;
+// float <-> int conversions); the node value is (hi + lo / 2^fb) / S,
+// resolved to 2^-fb / S. fb = 16, or fewer for bricks of more than 2^14
+// particles, so that the n fractions of a node (each at most 2^fb) cannot
+// overflow: n 2^fb <= 2^30.
+//
+// FP64, B = 62: t rounded to a 64-bit integer, added as its low word and --
+// with the carry of that add -- its high word; the number of carries does not
+// depend on the order either. A contribution is kept to 2^-62 of the bound on
+// a node sum (156 unit charges: 2^-57), finer than an FP64 sum's rounding.
+// Shared memory has no 64-bit add (a
+// compare-and-swap loop: 33 us for the 64 bricks of 1e4 particles, against
+// 14 with the two words; the ordered FP64 sum it replaced took 34).
+//
+// Bound: the shared-memory atomics (a warp's add every two cycles; 1280
+// bricks of 157 particles 50 -> 42 us without the second pass over positions
+// and with shared weight terms, 1e6 particles on 256^3 190 -> 174), in small
+// systems as much the CTA's set-up and write-out. With parts > 1, that many
+// CTAs share a brick: each owns a z range of the tile's planes, takes the
+// particles whose stencils reach it, and writes its planes -- no sums between
+// CTAs.
+constexpr int A_THREADS = 256;
 constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
 constexpr int kRoundBits = 0x4B400000;
 
-__global__ void __launch_bounds__(A32_THREADS)
-k_assign_i32(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
-             const int *__restrict__ brick_perm, const double *__restrict__ pos,
-             const double *__restrict__ charge, float *__restrict__ tiles, int nbrick)
+static size_t assign_smem(int parts)
 {
-    extern __shared__ __align__(16) int a32_smem[];
-    int *thi = a32_smem;
-    int *tlo = a32_smem + TILE3;
-    __shared__ int a_src[A32_THREADS];  // the chunk's particle slot of each thread, or -1
+    return (size_t)((TILE + parts - 1) / parts) * TILE * TILE * 2 * sizeof(int);
+}
+
+template <typename T, bool SPLIT>
+__global__ void __launch_bounds__(A_THREADS)
+k_assign(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
+         const typename V4<T>::t *__restrict__ slot_pt, const T *__restrict__ slot_q,
+         T *__restrict__ tiles, int nbrick, int parts)
+{
+    extern __shared__ __align__(16) int a_smem[];
+    __shared__ int a_src[A_THREADS];  // the chunk's particle slot of each thread, or -1
     __shared__ int a_cnt[32];
+    __shared__ double a_qmax[sizeof(T) == 8 ? A_THREADS / 32 : 1];
     const int lane = threadIdx.x & 31;
-    for (int b = blockIdx.x; b < nbrick; b += gridDim.x) {
+    const int np_max = SPLIT ? (TILE + parts - 1) / parts : TILE;  // planes of a full part
+    int *thi = a_smem, *tlo = a_smem + np_max * TILE * TILE;
+    for (int it = blockIdx.x; it < nbrick * (SPLIT ? parts : 1); it += gridDim.x) {
+        const int b = SPLIT ? it / parts : it;
+        const int z0 = SPLIT ? (it % parts) * np_max : 0;
+        const int np = SPLIT ? min(np_max, TILE - z0) : TILE;  // this item's planes z0 .. z0 + np
+        if (SPLIT && np <= 0) continue;
+        const int nnode = np * TILE * TILE;
         const int r = find_rep(b, nrep, [&](int k) { return reps[k].brick_off; });
         const RepDev &R = reps[r];
-        const int nb = R.nb, M = R.M, local = b - R.brick_off;
-        const int bx = (local % nb) * BRICK, by = ((local / nb) % nb) * BRICK,
-                  bz = (local / (nb * nb)) * BRICK;
+        const int local = b - R.brick_off;
         const int p0 = brick_start[b], n = brick_start[b + 1] - p0;
-        // S = 2^k with 0.17 n qmax S <= 2^22
-        const double bound = 0.17 * (double)(n > 0 ? n : 1) * R.qmax;
-        const int kexp = (int)floor(22.0 - log2(bound > 1e-300 ? bound : 1e-300));
-        const float S = ldexpf(1.0f, max(-100, min(kexp, 100)));
-        int nbits = 0;
-        while ((1 << nbits) <= n && nbits < 30) ++nbits;  // n < 2^nbits
-        const int fb = max(0, min(16, 30 - nbits));
-        const float F = ldexpf(1.0f, fb);
+        double qmax = R.qmax;
+        if constexpr (sizeof(T) == 8) {  // the brick's own largest |q|
+            qmax = 0.0;
+            for (int k = threadIdx.x; k < n; k += A_THREADS) qmax = fmax(qmax, fabs((double)slot_q[p0 + k]));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) qmax = fmax(qmax, __shfl_xor_sync(0xffffffffu, qmax, o));
+            __syncthreads();  // the previous item is done with a_qmax
+            if (lane == 0) a_qmax[threadIdx.x >> 5] = qmax;
+            __syncthreads();
+            for (int k = 0; k < A_THREADS / 32; ++k) qmax = fmax(qmax, a_qmax[k]);
+        }
+        // S = 2^k with 0.17 n qmax S <= 2^B, k = B - ceil(log2(0.17 n qmax))
+        const double bound = fmax(0.17 * (double)(n > 0 ? n : 1) * qmax, 1e-300);
+        const long long bits = __double_as_longlong(bound);
+        const int ceil2 = (int)(bits >> 52) - 1023 + ((bits & 0xFFFFFFFFFFFFFll) != 0 ? 1 : 0);
+        constexpr int B = sizeof(T) == 4 ? 22 : 62, KMAX = sizeof(T) == 4 ? 100 : 1000;
+        const int kexp = max(-KMAX, min(B - ceil2, KMAX));
+        const double Sd = __longlong_as_double((long long)(kexp + 1023) << 52);
+        const T S = (T)Sd;
+        const double inv = __longlong_as_double((long long)(1023 - kexp) << 52);  // 1 / S
+        const int fb = max(0, min(16, 30 - (32 - __clz(n))));  // n < 2^(32 - clz n)
+        const float F = (float)(1 << fb);
         __syncthreads();
-        for (int k = threadIdx.x; k < TILE3; k += A32_THREADS) {
+        for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
             thi[k] = 0;
             tlo[k] = 0;
         }
         __syncthreads();
-        for (int c0 = p0; c0 < p0 + n; c0 += A32_THREADS) {
+        for (int c0 = p0; c0 < p0 + n; c0 += A_THREADS) {
             // The lanes of a warp add at the same offsets from their
             // particles' stencil bases: lanes whose bases share a shared-memory
-            // bank conflict on every atomic. The chunk's particles are ranked
-            // by bank (from floor(x / h) by multiplication: only the balance
-            // depends on it) and dealt round-robin to the warps. Integer sums
-            // do not depend on which thread adds what.
-            const int nch = min(A32_THREADS, p0 + n - c0);
+            // bank conflict on every atomic. The chunk's particles (of those
+            // that reach this item's planes) are ranked by bank and dealt
+            // round-robin to the warps. Integer sums do not depend on which
+            // thread adds what.
+            const int c = c0 + threadIdx.x;
             int bank = 0, rank = 0;
-            if (threadIdx.x < nch) {
-                const int i = brick_perm[c0 + threadIdx.x];
-                const int qx = wrapM((int)floor(pos[3 * i + 0] * R.inv_h), M) - bx;
-                const int qy = wrapM((int)floor(pos[3 * i + 1] * R.inv_h), M) - by;
-                const int qz = wrapM((int)floor(pos[3 * i + 2] * R.inv_h), M) - bz;
-                bank = (int)((((unsigned)qz * TILE + (unsigned)qy) * TILE + (unsigned)qx) & 31u);
+            bool use = false;
+            if (c < p0 + n) {
+                const int pb = unpack_base(slot_pt[c].w);  // -1: filed under brick 0 and flagged
+                const int lz = (pb >> 8) & 15;
+                use = pb >= 0 && (!SPLIT || (lz + HALO >= z0 && lz < z0 + np));
+                bank = (((lz * TILE + ((pb >> 4) & 15)) * TILE) + (pb & 15)) & 31;
             }
             __syncthreads();  // the previous chunk is done with a_src
             a_src[threadIdx.x] = -1;
             if (threadIdx.x < 32) a_cnt[threadIdx.x] = 0;
             __syncthreads();
-            if (threadIdx.x < nch) rank = atomicAdd(&a_cnt[bank], 1);
-            __syncthreads();
+            if (use) rank = atomicAdd(&a_cnt[bank], 1);
+            const int nch = __syncthreads_count(use);
             if (threadIdx.x < 32) {  // exclusive scan of the bank counts
                 const int v = a_cnt[lane];
                 int x = v;
@@ -379,54 +322,58 @@ k_assign_i32(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ 
                 a_cnt[lane] = x - v;
             }
             __syncthreads();
-            if (threadIdx.x < nch) {
+            if (use) {
                 const int q = a_cnt[bank] + rank, nw = (nch + 31) >> 5;
-                a_src[(q % nw) * 32 + q / nw] = c0 + threadIdx.x;
+                a_src[(q % nw) * 32 + q / nw] = c;
             }
             __syncthreads();
             const int p = a_src[threadIdx.x];
             if (p < 0) continue;
-            const int i = brick_perm[p];
-            double ox, oy, oz;
-            const int ix = base_offset(pos[3 * i + 0], R.h, ox);
-            const int iy = base_offset(pos[3 * i + 1], R.h, oy);
-            const int iz = base_offset(pos[3 * i + 2], R.h, oz);
-            const int lx = wrapM(ix, M) - bx, ly = wrapM(iy, M) - by, lz = wrapM(iz, M) - bz;
-            // a particle outside [-L, 2L) was filed under brick 0 and flagged
-            if ((unsigned)lx >= (unsigned)BRICK || (unsigned)ly >= (unsigned)BRICK ||
-                (unsigned)lz >= (unsigned)BRICK)
-                continue;
-            float wx[6], wy[6], wz[6];
-            weights6<float>((float)ox, wx);
-            weights6<float>((float)oy, wy);
-            weights6<float>((float)oz, wz);
-            const float qs = (float)charge[i] * S;
-            const int base = (lz * TILE + ly) * TILE + lx;
+            const typename V4<T>::t v = slot_pt[p];
+            const int pb = unpack_base(v.w), lz = pb >> 8;
+            T wx[6], wy[6], wz[6];
+            weights6<T>(v.x, wx);
+            weights6<T>(v.y, wy);
+            weights6<T>(v.z, wz);
+            const T qs = slot_q[p] * S;
+            const int base = ((lz - z0) * TILE + ((pb >> 4) & 15)) * TILE + (pb & 15);
 #pragma unroll
             for (int g = 0; g < 6; ++g) {
+                if (SPLIT && (unsigned)(lz + g - z0) >= (unsigned)np) continue;
 #pragma unroll
                 for (int a = 0; a < 6; ++a) {
-                    const float qzy = qs * wz[g] * wy[a];
+                    const T qzy = qs * wz[g] * wy[a];
                     const int row = base + (g * TILE + a) * TILE;
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        const float t = qzy * wx[c];
-                        const float hb = (t - 0.5f) + kRound;       // floor(t), as a float
-                        const int hi = __float_as_int(hb) - kRoundBits;
-                        const float frac = t - (hb - kRound);         // in [0, 1], exact
-                        const int lo = __float_as_int(frac * F + kRound) - kRoundBits;
-                        atomicAdd(thi + row + c, hi);
-                        atomicAdd(tlo + row + c, lo);
+                    for (int cx = 0; cx < 6; ++cx) {
+                        const T t = qzy * wx[cx];
+                        if constexpr (sizeof(T) == 4) {
+                            const float hb = (t - 0.5f) + kRound;    // floor(t), as a float
+                            const int hi = __float_as_int(hb) - kRoundBits;
+                            const float frac = t - (hb - kRound);      // in [0, 1], exact
+                            const int lo = __float_as_int(frac * F + kRound) - kRoundBits;
+                            atomicAdd(thi + row + cx, hi);
+                            atomicAdd(tlo + row + cx, lo);
+                        } else {
+                            const long long i = __double2ll_rn(t);
+                            const unsigned lo = (unsigned)i;
+                            const unsigned old = atomicAdd((unsigned *)tlo + row + cx, lo);
+                            atomicAdd(thi + row + cx, (int)(i >> 32) + (old + lo < lo ? 1 : 0));
+                        }
                     }
                 }
             }
         }
         __syncthreads();
-        float *dst = tiles + R.tile_off + (long long)local * TILE3;
-        const double inv = 1.0 / (double)S;
-        const double invF = 1.0 / (double)F;  // exact: F is a power of two
-        for (int k = threadIdx.x; k < TILE3; k += A32_THREADS)
-            dst[k] = (float)(((double)thi[k] + (double)tlo[k] * invF) * inv);
+        T *dst = tiles + R.tile_off + (long long)local * TILE3 + z0 * TILE * TILE;
+        // exact as integers, rounded once by the conversion
+        const T unit = sizeof(T) == 4 ? (T)(inv / (double)F) : (T)inv;
+        for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
+            if constexpr (sizeof(T) == 4)
+                dst[k] = (float)(((long long)thi[k] << fb) + tlo[k]) * unit;
+            else
+                dst[k] = (T)(((long long)thi[k] << 32) | (unsigned)tlo[k]) * unit;
+        }
     }
 }
 
@@ -915,17 +862,13 @@ constexpr int GTILE = TILE * TILE * GTX;
 template <typename T, int NB, int NC>
 __global__ void __launch_bounds__(G_THREADS, sizeof(T) == 4 ? (NB == 1 ? 4 : 1) : 2)
 k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
-         const int *__restrict__ brick_perm, const double *__restrict__ pos,
-         const double *__restrict__ charge, const T *__restrict__ efield, long long nmesh,
+         const typename V4<T>::t *__restrict__ slot_pt, const T *__restrict__ slot_q,
+         const T *__restrict__ efield, long long nmesh,
          typename V4<T>::t *__restrict__ acc_pm, int nbrick)
 {
     extern __shared__ __align__(16) unsigned char g_smem[];
     T *tile = reinterpret_cast<T *>(g_smem);
-    // per thread of the chunk: its particle (slot p, or -1), node offsets,
-    // local tile offset of the stencil's first node (or -1)
-    __shared__ int g_src[G_THREADS];
-    __shared__ T g_o[3][G_THREADS];
-    __shared__ int g_base[G_THREADS];
+    __shared__ int g_src[G_THREADS];  // per thread of the chunk: its particle's slot, or -1
     __shared__ int g_cnt[32];
     const int lane = threadIdx.x & 31;
     static_assert(NC == 3 || NC == 1, "a whole brick or one component per CTA");
@@ -946,24 +889,10 @@ k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
             // warps: each warp gets bases spread over the banks. Which thread
             // handles a particle does not change its sums.
             const int nch = min(G_THREADS, p1 - c0);
-            int bank = 0, rank = 0, base0 = -1;
-            T ox0 = 0, oy0 = 0, oz0 = 0;
+            int bank = 0, rank = 0;
             if (threadIdx.x < nch) {
-                const int i = brick_perm[c0 + threadIdx.x];
-                double ox, oy, oz;
-                const int ix = base_offset(pos[3 * i + 0], R.h, ox);
-                const int iy = base_offset(pos[3 * i + 1], R.h, oy);
-                const int iz = base_offset(pos[3 * i + 2], R.h, oz);
-                const int lx = wrapM(ix, M) - bx, ly = wrapM(iy, M) - by, lz = wrapM(iz, M) - bz;
-                // (a particle outside [-L, 2L) was flagged by the key pass)
-                if ((unsigned)lx < (unsigned)BRICK && (unsigned)ly < (unsigned)BRICK &&
-                    (unsigned)lz < (unsigned)BRICK) {
-                    base0 = (lz * TILE + ly) * GTX + lx;
-                    bank = base0 & 31;
-                }
-                ox0 = (T)ox;
-                oy0 = (T)oy;
-                oz0 = (T)oz;
+                const int pb = max(0, unpack_base(slot_pt[c0 + threadIdx.x].w));
+                bank = (((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15)) & 31;
             }
             __syncthreads();  // the previous chunk / brick is done with g_* and the buffers
             g_src[threadIdx.x] = -1;
@@ -984,22 +913,20 @@ k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
             __syncthreads();
             if (threadIdx.x < nch) {
                 const int q = g_cnt[bank] + rank, nw = (nch + 31) >> 5;
-                const int tgt = (q % nw) * 32 + q / nw;
-                g_src[tgt] = c0 + threadIdx.x;
-                g_o[0][tgt] = ox0;
-                g_o[1][tgt] = oy0;
-                g_o[2][tgt] = oz0;
-                g_base[tgt] = base0;
+                g_src[(q % nw) * 32 + q / nw] = c0 + threadIdx.x;
             }
             __syncthreads();
             const int p = g_src[threadIdx.x];
             T wx[6], wy[6], wz[6];
-            const int base = p >= 0 ? g_base[threadIdx.x] : -1;
+            int base = -1;
             T e[3] = {(T)0, (T)0, (T)0};
-            if (base >= 0) {
-                weights6<T>(g_o[0][threadIdx.x], wx);
-                weights6<T>(g_o[1][threadIdx.x], wy);
-                weights6<T>(g_o[2][threadIdx.x], wz);
+            if (p >= 0) {
+                const typename V4<T>::t v = slot_pt[p];
+                const int pb = unpack_base(v.w);  // -1: flagged by the key pass
+                if (pb >= 0) base = ((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15);
+                weights6<T>(v.x, wx);
+                weights6<T>(v.y, wy);
+                weights6<T>(v.z, wz);
             }
             // component tiles through the NB buffers
             auto issue = [&](int comp) {
@@ -1060,12 +987,12 @@ k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
                     out.x = e[0];
                     out.y = e[1];
                     out.z = e[2];
-                    out.w = (T)charge[brick_perm[p]];
+                    out.w = slot_q[p];
                     acc_pm[p] = out;
                 } else {
                     T *o = reinterpret_cast<T *>(acc_pm + p);  // (Ex, Ey, Ez, Z)
                     o[cfirst] = e[cfirst];
-                    if (cfirst == 0) o[3] = (T)charge[brick_perm[p]];
+                    if (cfirst == 0) o[3] = slot_q[p];
                 }
             }
         }
@@ -1175,8 +1102,8 @@ static int grid_items(int n, int cap = 148 * 8) { return n < cap ? (n > 0 ? n : 
 
 template <typename T> void configure_mesh_kernels()
 {
-    set_smem(k_assign<T>, assign_smem<T>());
-    set_smem(k_assign_i32, 2 * TILE3 * sizeof(int));
+    set_smem(k_assign<T, false>, assign_smem(1));
+    set_smem(k_assign<T, true>, assign_smem(1));
     set_smem(k_fft_x_r2c<T>, x_smem<T>(256));
     set_smem(k_fft_y<T>, fft_smem<T>(256, 1));
     set_smem(k_fft_z_green<T>, fft_smem<T>(256, 2));
@@ -1187,18 +1114,26 @@ template <typename T> void configure_mesh_kernels()
     set_smem(k_fft_plane<T>, plane_smem<T>(PLANE_MAX));
 }
 
+// CTAs per brick of the assignment: two for up to 32 bricks (FP32, one
+// against two CTAs: 12.4 / 10.3 us at 8 bricks of 250 particles, 12.4 / 11.8
+// at 32), one from there on, where the repeated set-up costs as much as the
+// halved atomics save (8.3 / 8.3 us at 64 bricks, 9.2 / 10.3 at 128, 22 / 27
+// at 512; three or more CTAs nowhere better than two).
+int assign_parts_for(int nbrick) { return nbrick <= 32 ? 2 : 1; }
+
 template <typename T> void launch_assign(const DevState &s, cudaStream_t st)
 {
-    if (sizeof(T) == 4) {
-        k_assign_i32<<<grid_items(s.nbrick, 148 * 16), A32_THREADS, 2 * TILE3 * sizeof(int), st>>>(
-            s.reps, s.nrep, s.brick_start, s.brick_perm, s.pos, s.charge, (float *)s.tiles,
-            s.nbrick);
-        return;
-    }
-    const size_t smem = assign_smem<T>();
-    k_assign<T><<<grid_items(s.nbrick, 148 * 16), A_THREADS, smem, st>>>(
-        s.reps, s.nrep, s.brick_start, s.brick_perm, s.pos, s.charge, (T *)s.tiles, s.nbrick,
-        s.status);
+    using A = typename V4<T>::t;
+    const int parts = s.assign_parts;
+    const int grid = grid_items(s.nbrick * parts, 148 * 16);
+    if (parts > 1)
+        k_assign<T, true><<<grid, A_THREADS, assign_smem(parts), st>>>(
+            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (T *)s.tiles,
+            s.nbrick, parts);
+    else
+        k_assign<T, false><<<grid, A_THREADS, assign_smem(1), st>>>(
+            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (T *)s.tiles,
+            s.nbrick, parts);
 }
 
 template <typename T> void launch_fft_forward(const DevState &s, cudaStream_t st)
@@ -1242,15 +1177,15 @@ template <typename T> void launch_gather(const DevState &s, cudaStream_t st)
     using A = typename V4<T>::t;
     if (sizeof(T) == 4 && s.gather_mode == 2)
         k_gather<T, 2, 3><<<grid_items(s.nbrick, 148 * 16), G_THREADS, 2 * GTILE * sizeof(T), st>>>(
-            s.reps, s.nrep, s.brick_start, s.brick_perm, s.pos, s.charge, (const T *)s.efield,
+            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (const T *)s.efield,
             s.nmesh, (A *)s.acc_pm, s.nbrick);
     else if (s.gather_mode == 0)
         k_gather<T, 1, 1><<<grid_items(3 * s.nbrick, 148 * 16), G_THREADS, GTILE * sizeof(T), st>>>(
-            s.reps, s.nrep, s.brick_start, s.brick_perm, s.pos, s.charge, (const T *)s.efield,
+            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (const T *)s.efield,
             s.nmesh, (A *)s.acc_pm, s.nbrick);
     else
         k_gather<T, 1, 3><<<grid_items(s.nbrick, 148 * 16), G_THREADS, GTILE * sizeof(T), st>>>(
-            s.reps, s.nrep, s.brick_start, s.brick_perm, s.pos, s.charge, (const T *)s.efield,
+            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (const T *)s.efield,
             s.nmesh, (A *)s.acc_pm, s.nbrick);
 }
 

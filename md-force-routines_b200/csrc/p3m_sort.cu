@@ -14,14 +14,17 @@
 // lists, and its rounding, do not depend on the other replicas of a batch. It is deterministic: counts and offsets
 // come from integer atomics and a scan; the order inside a cell is then
 // fixed by sorting each cell's particle indices ascending (rank sort), so
-// every rerun builds the same lists. The brick sort runs every step and puts
-// each brick's particles in ascending index order, so the assignment adds
-// them in a fixed order: a stable counting sort over chunks of `ch`
-// consecutive particles of one replica (ch sized at context creation so that
-// there are a few chunks per SM) (per-chunk counts per brick, a scan of
-// each brick's counts over the chunks, then one warp per chunk placing its
-// particles in index order). Its work is linear in the particle count however
-// many particles share a brick.
+// every rerun builds the same lists. The brick sort runs every step: the
+// drift (or key) pass takes each particle's arrival rank in its brick from
+// the atomic that counts it, a scan gives the bricks' first slots, and one
+// pass writes every particle's stencil offsets and charge to its slot. The
+// order inside a brick is whatever the atomics gave; nothing depends on it
+// (the assignment sums integers, the gather works per particle). Against a
+// stable sort (chunk histograms, a column scan and a warp per chunk placing
+// its particles in index order) that is two kernels and two passes fewer:
+// per step 14.5 -> 6.4 us of drift and
+// sort kernels for 1e4 particles on 64^3, 43 -> 14 for 1e5 on 128^3, 153 -> 65
+// for 1e6 on 256^3.
 #include "p3m_kernels.h"
 
 namespace p3m {
@@ -30,8 +33,8 @@ template <typename T>
 __global__ void k_keys(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                        const double *__restrict__ pos, int ntot, int *__restrict__ cell_key,
                        int *__restrict__ cell_sub, int *__restrict__ cell_count,
-                       int *__restrict__ brick_key, int *__restrict__ brick_count, int has_mesh,
-                       int *status)
+                       int *__restrict__ brick_key, int *__restrict__ brick_rank,
+                       int *__restrict__ brick_count, int has_mesh, int *status)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const RepDev &R = reps[prep[i]];
@@ -43,7 +46,7 @@ __global__ void k_keys(const RepDev *__restrict__ reps, const int *__restrict__ 
         atomicAdd(&cell_count[c], 1);
         if (b >= 0) {
             brick_key[i] = b;
-            atomicAdd(&brick_count[b], 1);
+            brick_rank[i] = atomicAdd(&brick_count[b * BRICK_CNT_STRIDE], 1);
         }
     }
 }
@@ -66,15 +69,17 @@ __global__ void k_cell_keys(const RepDev *__restrict__ reps, const int *__restri
     }
 }
 
-// Exclusive scan of count[0..n) into start[0..n], offset by `base` (single
-// block), zeroing the counts and the scatter cursors for the next use.
+// Exclusive scan of count[0], count[STRIDE], ... (n of them) into start[0..n],
+// offset by `base` (single block), zeroing the counts and the scatter cursors
+// (may be NULL) for the next use.
+template <int STRIDE>
 __device__ void block_scan_array(int *count, int *start, int *cursor, int n, int base, int *sm)
 {
     int carry = base;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     for (int b0 = 0; b0 < n; b0 += blockDim.x) {
         int i = b0 + tid;
-        int v = (i < n) ? count[i] : 0;
+        int v = (i < n) ? count[i * STRIDE] : 0;
         int x = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -96,8 +101,8 @@ __device__ void block_scan_array(int *count, int *start, int *cursor, int n, int
         int excl = carry + x - v + (w > 0 ? sm[32 + w - 1] : 0);
         if (i < n) {
             start[i] = excl;
-            count[i] = 0;
-            cursor[i] = 0;
+            count[i * STRIDE] = 0;
+            if (cursor) cursor[i] = 0;
         }
         carry += sm[32 + nw - 1];
         __syncthreads();
@@ -109,7 +114,7 @@ __device__ void block_scan_array(int *count, int *start, int *cursor, int n, int
 // its own particle range [p_off, p_off + n). Block 1: all bricks.
 __global__ void k_scan(const RepDev *__restrict__ reps, int nrep, int *cell_count,
                        int *cell_start, int *cell_cursor, int *brick_count, int *brick_start,
-                       int *brick_cursor, int nbrick, const int *__restrict__ rebuild,
+                       int nbrick, const int *__restrict__ rebuild,
                        int *__restrict__ rb_list, int first_part)
 {
     __shared__ int sm[64];
@@ -119,7 +124,7 @@ __global__ void k_scan(const RepDev *__restrict__ reps, int nrep, int *cell_coun
             if (!rebuild[r]) continue;
             const RepDev &R = reps[r];
             const int c0 = R.cell_off, nc = R.nc * R.nc * R.nc;
-            block_scan_array(cell_count + c0, cell_start + c0, cell_cursor + c0, nc, R.p_off, sm);
+            block_scan_array<1>(cell_count + c0, cell_start + c0, cell_cursor + c0, nc, R.p_off, sm);
             if (threadIdx.x == 0) {
                 rb_list[1 + k] = r;
                 rb_list[nrep + 1 + k] = cells;
@@ -133,7 +138,7 @@ __global__ void k_scan(const RepDev *__restrict__ reps, int nrep, int *cell_coun
             rb_list[nrep + 1 + k] = cells;
         }
     } else if (nbrick > 0) {
-        block_scan_array(brick_count, brick_start, brick_cursor, nbrick, 0, sm);
+        block_scan_array<BRICK_CNT_STRIDE>(brick_count, brick_start, nullptr, nbrick, 0, sm);
     }
 }
 
@@ -194,91 +199,55 @@ __global__ void k_fix_cells(const RepDev *__restrict__ reps, int nrep,
 
 // ---- brick sort ----------------------------------------------------------
 
-__device__ __forceinline__ int sort_chunks(const RepDev &R, int ch) { return (R.n + ch - 1) / ch; }
-
-// One block per chunk: hist[chunk][k] = particles of the chunk in the
-// replica's brick k (shared-memory integer counts).
-__global__ void __launch_bounds__(256)
-k_brick_hist(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_key,
-             int *__restrict__ hist, int nchunk, int ch)
+// Base index (unwrapped) and offset along one axis (yukawa_pm_ord6.py:17-27).
+__device__ __forceinline__ int base_offset(double p, double h, double &off)
 {
-    extern __shared__ int hcount[];
-    for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
-        const RepDev &R = reps[find_rep(c, nrep, [&](int k) { return reps[k].sc_off; })];
-        const int nbr = R.nb * R.nb * R.nb;
-        const int cl = c - R.sc_off;
-        const int p0 = R.p_off + cl * ch, n = min(ch, R.n - cl * ch);
-        for (int k = threadIdx.x; k < nbr; k += blockDim.x) hcount[k] = 0;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-            atomicAdd(&hcount[brick_key[p0 + i] - R.brick_off], 1);
-        __syncthreads();
-        int *row = hist + R.sh_off + (long long)cl * nbr;
-        for (int k = threadIdx.x; k < nbr; k += blockDim.x) row[k] = hcount[k];
-        __syncthreads();
-    }
+    int ix = (int)floor(p / h);
+    off = (p - (ix + 0.5) * h) / h;
+    return ix;
 }
 
-// One warp per brick: its counts over the replica's chunks become the
-// chunks' first slots (exclusive scan from brick_start), 32 chunks a pass.
-__global__ void k_brick_colscan(const RepDev *__restrict__ reps, int nrep,
-                                const int *__restrict__ brick_start, int *__restrict__ hist,
-                                int nbrick, int ch)
+__device__ __forceinline__ int wrapM(int i, int M)
 {
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (int b = blockIdx.x * wpb + (threadIdx.x >> 5); b < nbrick; b += gridDim.x * wpb) {
-        const RepDev &R = reps[find_rep(b, nrep, [&](int k) { return reps[k].brick_off; })];
-        const int nbr = R.nb * R.nb * R.nb;
-        const int nch = sort_chunks(R, ch);
-        int *col = hist + R.sh_off + (b - R.brick_off);
-        int carry = brick_start[b];
-        for (int c0 = 0; c0 < nch; c0 += 32) {
-            const int cl = c0 + lane;
-            const int t = cl < nch ? col[(long long)cl * nbr] : 0;
-            int x = t;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (cl < nch) col[(long long)cl * nbr] = carry + x - t;
-            carry += __shfl_sync(0xffffffffu, x, 31);
-        }
-    }
+    i %= M;
+    return i < 0 ? i + M : i;
 }
 
-// One warp per chunk, 32 particles at a time in index order: lanes with the
-// same brick take consecutive slots in lane order (__match_any_sync), then
-// the group's last lane advances the brick's next slot.
-__global__ void __launch_bounds__(32)
-k_brick_place(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_key,
-              const int *__restrict__ hist, int *__restrict__ brick_perm,
-              int *__restrict__ brick_slot, int nchunk, int ch)
+// One thread per particle: its slot in brick order, and there its stencil
+// offsets (FP64 arithmetic, stored in the bulk precision), its base inside
+// the brick and its charge -- what the assignment and the gather read,
+// contiguous per brick and computed once for both.
+template <typename T>
+__global__ void k_brick_place(const RepDev *__restrict__ reps, const int *__restrict__ prep,
+                              const double *__restrict__ pos, const double *__restrict__ charge,
+                              const int *__restrict__ brick_key, const int *__restrict__ brick_rank,
+                              const int *__restrict__ brick_start, int *__restrict__ brick_slot,
+                              typename V4<T>::t *__restrict__ slot_pt, T *__restrict__ slot_q,
+                              int ntot)
 {
-    extern __shared__ int next_slot[];
-    const int lane = threadIdx.x;
-    for (int c = blockIdx.x; c < nchunk; c += gridDim.x) {
-        const RepDev &R = reps[find_rep(c, nrep, [&](int k) { return reps[k].sc_off; })];
-        const int nbr = R.nb * R.nb * R.nb;
-        const int cl = c - R.sc_off;
-        const int p0 = R.p_off + cl * ch, n = min(ch, R.n - cl * ch);
-        const int *row = hist + R.sh_off + (long long)cl * nbr;
-        for (int k = lane; k < nbr; k += 32) next_slot[k] = row[k];
-        __syncwarp();
-        for (int e0 = 0; e0 < n; e0 += 32) {
-            const int e = e0 + lane;
-            const bool valid = e < n;
-            const int key = valid ? brick_key[p0 + e] - R.brick_off : -1;
-            const unsigned peers = __match_any_sync(0xffffffffu, key);
-            if (valid) {
-                const int slot = next_slot[key] + __popc(peers & ((1u << lane) - 1u));
-                brick_perm[slot] = p0 + e;
-                brick_slot[p0 + e] = slot;
-            }
-            __syncwarp();
-            if (valid && lane == 31 - __clz(peers)) next_slot[key] += __popc(peers);
-            __syncwarp();
-        }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
+        const RepDev &R = reps[prep[i]];
+        const int b = brick_key[i], local = b - R.brick_off, nb = R.nb, M = R.M;
+        const int slot = brick_start[b] + brick_rank[i];
+        double ox, oy, oz;
+        const int ix = base_offset(pos[3 * i + 0], R.h, ox);
+        const int iy = base_offset(pos[3 * i + 1], R.h, oy);
+        const int iz = base_offset(pos[3 * i + 2], R.h, oz);
+        const int lx = wrapM(ix, M) - (local % nb) * BRICK,
+                  ly = wrapM(iy, M) - ((local / nb) % nb) * BRICK,
+                  lz = wrapM(iz, M) - (local / (nb * nb)) * BRICK;
+        // a particle outside [-L, 2L) was filed under brick 0 and flagged; it
+        // must not reach outside the tile
+        const bool in = (unsigned)lx < (unsigned)BRICK && (unsigned)ly < (unsigned)BRICK &&
+                        (unsigned)lz < (unsigned)BRICK;
+        typename V4<T>::t v;
+        v.x = (T)ox;
+        v.y = (T)oy;
+        v.z = (T)oz;
+        v.w = pack_base<T>(in ? lx | (ly << 4) | (lz << 8) : -1);
+        brick_slot[i] = slot;
+        slot_pt[slot] = v;
+        slot_q[slot] = (T)charge[i];
     }
 }
 
@@ -293,7 +262,8 @@ template <typename T> void launch_keys(const DevState &s, cudaStream_t st)
 {
     k_keys<T><<<grid_for(s.ntot, 256), 256, 0, st>>>(s.reps, s.prep, s.pos, s.ntot, s.cell_key,
                                                       s.cell_sub, s.cell_count, s.brick_key,
-                                                      s.brick_count, s.has_mesh, s.status);
+                                                      s.brick_rank, s.brick_count, s.has_mesh,
+                                                      s.status);
 }
 
 void launch_cell_keys(const DevState &s, cudaStream_t st)
@@ -309,8 +279,7 @@ void launch_scan(const DevState &s, cudaStream_t st, int part)
 {
     const int first = part == 1 ? 1 : 0, nblocks = part < 0 ? 2 : 1;
     k_scan<<<nblocks, 1024, 0, st>>>(s.reps, s.nrep, s.cell_count, s.cell_start, s.cell_cursor,
-                                     s.brick_count, s.brick_start, s.brick_cursor,
-                                     s.has_mesh ? s.nbrick : 0, s.rebuild, s.rb_list, first);
+                                     s.brick_count, s.brick_start, s.has_mesh ? s.nbrick : 0, s.rebuild, s.rb_list, first);
 }
 
 void launch_scatter(const DevState &s, cudaStream_t st)
@@ -319,16 +288,11 @@ void launch_scatter(const DevState &s, cudaStream_t st)
                                                       s.cell_tmp, s.ntot, s.prep, s.rebuild);
 }
 
-void launch_sort_bricks(const DevState &s, cudaStream_t st)
+template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t st)
 {
-    const size_t smem = (size_t)s.max_bricks * sizeof(int);
-    k_brick_hist<<<grid_for(s.nchunk, 1), 256, smem, st>>>(s.reps, s.nrep, s.brick_key,
-                                                            s.brick_hist, s.nchunk, s.sort_ch);
-    k_brick_colscan<<<grid_for(s.nbrick, 8), 256, 0, st>>>(s.reps, s.nrep, s.brick_start,
-                                                              s.brick_hist, s.nbrick, s.sort_ch);
-    k_brick_place<<<grid_for(s.nchunk, 1), 32, smem, st>>>(s.reps, s.nrep, s.brick_key,
-                                                           s.brick_hist, s.brick_perm,
-                                                           s.brick_slot, s.nchunk, s.sort_ch);
+    k_brick_place<T><<<grid_for(s.ntot, 256), 256, 0, st>>>(
+        s.reps, s.prep, s.pos, s.charge, s.brick_key, s.brick_rank, s.brick_start, s.brick_slot,
+        (typename V4<T>::t *)s.slot_pt, (T *)s.slot_q, s.ntot);
 }
 
 template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st)
@@ -342,6 +306,8 @@ template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st)
 
 template void launch_keys<float>(const DevState &, cudaStream_t);
 template void launch_keys<double>(const DevState &, cudaStream_t);
+template void launch_place_bricks<float>(const DevState &, cudaStream_t);
+template void launch_place_bricks<double>(const DevState &, cudaStream_t);
 template void launch_fix_cells<float>(const DevState &, cudaStream_t);
 template void launch_fix_cells<double>(const DevState &, cudaStream_t);
 
