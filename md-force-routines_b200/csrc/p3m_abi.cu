@@ -175,6 +175,80 @@ static void build_pp_table(const p3m_replica_desc &d, float4 *out)
     }
 }
 
+// psi(r) and g(r) in extended precision, from the same expressions.
+static void pair_g_psi_l(long double r, long double k, long double a, long double *g, long double *psi)
+{
+    const long double up = a * r + 0.5L * k / a, um = a * r - 0.5L * k / a;
+    const long double ep = expl(k * r) * erfcl(up), em = expl(-k * r) * erfcl(um);
+    const long double gauss = expl(-a * a * r * r - 0.25L * k * k / (a * a));
+    *psi = 0.5L * (ep + em);
+    *g = 0.5L * (ep * (1.0L - k * r) + em * (1.0L + k * r)) +
+         2.0L * a * r * gauss / sqrtl(3.141592653589793238462643383279502884L);
+}
+
+// FP64 pair table of one replica with N intervals: psi on interval i as a
+// degree-7 polynomial in u in [-1/2, 1/2] about its middle, through eight
+// Chebyshev points (Newton's divided differences, expanded); out[k * N + i] =
+// coefficients 2k, 2k + 1. Returns the largest error of psi and of g = psi - r
+// psi' (as the kernel forms them) at points between the nodes, in units of
+// psi(0) = 1; stops early once it exceeds `limit`. Nodes are in extended
+// precision: psi' divides their noise by the interval width.
+static double build_pp_table64(const p3m_replica_desc &d, int N, double limit, double2 *out)
+{
+    constexpr int K = 8;
+    const long double h = (long double)d.rc / N;
+    long double x[K];
+    for (int j = 0; j < K; ++j) x[j] = 0.5L * cosl((2 * j + 1) * 3.141592653589793238462643383279502884L / (2 * K));
+    double worst = 0.0;
+    for (int i = 0; i < N; ++i) {
+        long double f[K], g, c[K] = {0};
+        for (int j = 0; j < K; ++j) pair_g_psi_l((i + 0.5L + x[j]) * h, d.kappa, d.alpha, &g, &f[j]);
+        for (int m = 1; m < K; ++m)
+            for (int j = K - 1; j >= m; --j) f[j] = (f[j] - f[j - 1]) / (x[j] - x[j - m]);
+        for (int m = K - 1; m >= 0; --m) {  // c = c (u - x[m]) + f[m]
+            for (int j = K - 1; j > 0; --j) c[j] = c[j - 1] - x[m] * c[j];
+            c[0] = f[m] - x[m] * c[0];
+        }
+        for (int k = 0; k < K / 2; ++k) out[k * N + i] = make_double2((double)c[2 * k], (double)c[2 * k + 1]);
+        for (int j = 0; j < 3; ++j) {  // the ends and the middle
+            const long double u = 0.5L * (j - 1), t = i + 0.5L + u;
+            long double p = 0.0L, dp = 0.0L, gt, pt;
+            for (int k = K - 1; k >= 0; --k) {
+                dp = dp * u + p;
+                p = p * u + (k % 2 ? out[k / 2 * N + i].y : out[k / 2 * N + i].x);
+            }
+            pair_g_psi_l(t * h, d.kappa, d.alpha, &gt, &pt);
+            const double e = (double)fmaxl(fabsl(p - pt), fabsl(p - t * dp - gt));
+            if (!(e <= limit)) return 1.0;
+            worst = fmax(worst, e);
+        }
+    }
+    return worst;
+}
+
+// FP64 pair tables of all replicas with one interval count, the smallest that
+// keeps every replica's error within 4e-16 (a few units in the last place of
+// psi(0) = 1: below the rounding of the pair sums); 0 intervals when none
+// does. Replicas of equal parameters share the work.
+static int build_pp_tables64(const p3m_replica_desc *reps, int n_reps, std::vector<double2> &tab)
+{
+    for (int N = 128; N <= PP64_MAX_N; N *= 2) {
+        tab.assign((size_t)n_reps * N * 4, make_double2(0.0, 0.0));
+        bool ok = true;
+        for (int r = 0; r < n_reps && ok; ++r) {
+            double2 *out = tab.data() + (size_t)r * N * 4;
+            int same = -1;
+            for (int q = 0; q < r && same < 0; ++q)
+                if (reps[q].kappa == reps[r].kappa && reps[q].alpha == reps[r].alpha && reps[q].rc == reps[r].rc) same = q;
+            if (same >= 0) memcpy(out, tab.data() + (size_t)same * N * 4, sizeof(double2) * N * 4);
+            else ok = build_pp_table64(reps[r], N, 4e-16, out) <= 4e-16;
+        }
+        if (ok) return N;
+    }
+    tab.clear();
+    return 0;
+}
+
 // Work items of the mesh passes of every replica: x-pass items, and either
 // plane items (sides up to s.plane_max: the fused y/z plane kernel) or y and
 // z pencil items. Updates ctx->rh offsets and ctx->s totals; the caller
@@ -269,7 +343,7 @@ extern "C" int p3m_destroy(p3m_ctx *ctx)
     void *ptrs[] = {s.reps, s.pos, s.vel, s.acc, s.charge, s.prep, s.cell_key, s.cell_count,
                     s.cell_start, s.cell_cursor, s.cell_tmp, s.cell_perm, s.cell_slot, s.xq, s.nnb,
                     s.cell_sub,
-                    s.nlist, s.rebuild, s.rb_list, s.pos_ref, s.pp_tables,
+                    s.nlist, s.rebuild, s.rb_list, s.pos_ref, s.pp_tables, s.pp_tables64,
                     s.nnb_in, s.nlist_in, s.prune, s.pos_pref, s.prune_count,
                     s.acc_pp, s.brick_key, s.brick_rank, s.brick_count, s.brick_start,
                     s.brick_slot, s.slot_pt, s.slot_q, s.tiles, s.spec, s.ek, s.green, s.efield,
@@ -474,6 +548,14 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
         for (int r = 0; r < n_reps; ++r) build_pp_table(reps[r], tab.data() + (size_t)r * PP_TABLE_N);
         CKC(dalloc(&s.pp_tables, tab.size()));
         CKC(cudaMemcpy(s.pp_tables, tab.data(), sizeof(float4) * tab.size(), cudaMemcpyHostToDevice));
+    }
+    if (precision == P3M_FP64) {
+        std::vector<double2> tab;
+        s.pp64_n = build_pp_tables64(reps, n_reps, tab);
+        if (s.pp64_n > 0) {
+            CKC(dalloc(&s.pp_tables64, tab.size()));
+            CKC(cudaMemcpy(s.pp_tables64, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice));
+        }
     }
     CKC(dalloc(&s.pos, (size_t)3 * p));
     CKC(dalloc(&s.vel, (size_t)3 * p));

@@ -54,6 +54,8 @@ struct DevState {
     double *pos_pref = nullptr;  // positions at the last inner-list build (ntot,3)
     double *prune_count = nullptr;  // per replica: inner-list builds between outer rebuilds
     float4 *pp_tables = nullptr; // FP32 pair tables: cubic of psi = phi r, [nrep][PP_TABLE_N]
+    double2 *pp_tables64 = nullptr;  // FP64 path: [nrep][4][pp64_n] coefficient pairs
+    int pp64_n = 0;              // intervals of the FP64 tables (0: pair terms evaluated directly)
     void *acc_pp = nullptr;      // V4<T> PP acceleration, cell-sorted order
     // brick sort
     int *brick_key = nullptr, *brick_rank = nullptr;  // per particle: brick, arrival rank in it

@@ -28,15 +28,18 @@
 // either farther than rc + b at its build or missing from the Verlet list, so
 // it cannot come within rc before one of the two checks fires.
 //
-// Pair terms: the FP64 path evaluates the reference's formula directly,
-// written with the shared Gaussian factor
-//   e^{+-kr} erfc(u+-) = erfcx(u+-) exp(-(a^2 r^2 + k^2/4a^2)),  u+- = ar +- k/2a,
-// using CUDA's exp and erfcx. The FP32 path interpolates psi(r) = phi(r) r
-// (finite at r = 0), tabulated on [0, rc] from FP64 values computed on the
-// host, cubic per interval, and takes the force from the same cubic:
+// Pair terms: psi(r) = phi(r) r (finite at r = 0) is tabulated on [0, rc] as
+// one polynomial per interval, and the force comes from the same polynomial:
 //   g(r) = F(r) r^2 = -r^2 d(psi/r)/dr = psi - r psi',
 // F/r = g/r^3 and phi = psi/r -- one table read per pair, and a force that is
-// exactly minus the gradient of the interpolated potential.
+// exactly minus the gradient of the interpolated potential. FP32: cubics from
+// FP64 values. FP64: polynomials of degree 7 from extended-precision values,
+// with as many intervals as keep psi and g within a few 1e-16 of psi(0) = 1;
+// where the largest table does not reach that (very steep pair functions),
+// the reference's formula is evaluated directly, written with the shared
+// Gaussian factor
+//   e^{+-kr} erfc(u+-) = erfcx(u+-) exp(-(a^2 r^2 + k^2/4a^2)),  u+- = ar +- k/2a,
+// using CUDA's exp and erfcx.
 #include "p3m_kernels.h"
 
 namespace p3m {
@@ -292,22 +295,61 @@ __device__ __forceinline__ void pair_direct(double r2, const RepDev &R, double &
 // ---------------------------------------------------------------------------
 constexpr int PPL_THREADS = 256;
 
-// FP64 forces from the lists: the reference's pair terms (pair_direct) per
-// entry, TPI threads per particle, Kahan-compensated sums.
-template <int TPI>
+// FP64 pair terms of one entry from the table: tab[k * N + i] holds the
+// coefficients 2k, 2k + 1 of interval i (u in [-1/2, 1/2) about its middle),
+// so the 16-byte reads of a warp's lanes fall on random bank groups. Value and
+// derivative by one Horner recurrence; t = r / h, and g = p - t dp/du. The
+// caller passes r2 in (0, rc^2) (or rc^2, masked).
+__device__ __forceinline__ void pair_table64(double r2, double inv_h, int N, const double2 *tab,
+                                             double &f_over_r, double &phi)
+{
+    const double rinv = rsqrt(r2);
+    const double t = r2 * rinv * inv_h;
+    const int i = min((int)t, N - 1);
+    const double u = t - ((double)i + 0.5);
+    const double2 c67 = tab[3 * N + i], c45 = tab[2 * N + i], c23 = tab[N + i], c01 = tab[i];
+    double p = c67.y, d = c67.y;
+    p = fma(p, u, c67.x);
+    d = fma(d, u, p); p = fma(p, u, c45.y);
+    d = fma(d, u, p); p = fma(p, u, c45.x);
+    d = fma(d, u, p); p = fma(p, u, c23.y);
+    d = fma(d, u, p); p = fma(p, u, c23.x);
+    d = fma(d, u, p); p = fma(p, u, c01.y);
+    d = fma(d, u, p); p = fma(p, u, c01.x);
+    phi = p * rinv;
+    f_over_r = fma(-t, d, p) * rinv * (rinv * rinv);
+}
+
+// FP64 forces from the lists: TPI threads per particle, Kahan-compensated
+// sums. TAB: pair terms from the table (tab_n intervals), branch-free, so the
+// loads and the dependent chains of a pass overlap; otherwise pair_direct.
+//
+// Bound: the table and coordinate reads through L1 (96 bytes a pair), then
+// the FP64 pipe; pair_direct's exp and two erfcx, some 250 FP64 instructions
+// a pair, bound it there before (1e4 particles, rc 5.9: 162 -> 51 us with two
+// lanes per particle, 84 -> 35 with eight; 1e5: 531 -> 218 with eight).
+template <int TPI, bool TAB>
 __global__ void __launch_bounds__(PPL_THREADS)
 k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict__ xq,
          const int *__restrict__ nnb, const int *__restrict__ nlist, int maxnb,
-         double4 *__restrict__ acc_out, double *__restrict__ u_part)
+         const double2 *__restrict__ tables, int tab_n, double4 *__restrict__ acc_out,
+         double *__restrict__ u_part)
 {
     using T = double;
     using Q = ulonglong4;
     constexpr int PPB = PPL_THREADS / TPI;  // particles per block
     constexpr int CH = 32;                  // entries per Kahan flush
     __shared__ double red[32];
+    extern __shared__ __align__(16) double2 ppl_tab64[];
     const int b = blockIdx.x;
     const int r = find_rep(b, nrep, [&](int k) { return reps[k].pp_blk_off; });
     const RepDev &R = reps[r];
+    if constexpr (TAB) {
+        const double2 *src = tables + (long long)r * tab_n * 4;
+        for (int k = threadIdx.x; k < tab_n * 4; k += PPL_THREADS) cp_async16(ppl_tab64 + k, src + k);
+        cp_async_wait_all();
+        __syncthreads();
+    }
     const int sub = threadIdx.x % TPI;
     const int s = R.p_off + (b - R.pp_blk_off) * PPB + threadIdx.x / TPI;
     const bool have = s < R.p_off + R.n;
@@ -315,6 +357,7 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
     const double scd = R.L / Coord<T>::scale;
     const T sc = (T)scd, sc_lo = (T)(scd - (double)sc);
     const T rc2 = (T)(R.rc * R.rc);
+    const T inv_h = (T)(tab_n / R.rc);
 
     T fx = 0, fy = 0, fz = 0, gx = 0, gy = 0, gz = 0;
     double u = 0.0;
@@ -331,7 +374,7 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
             T px = 0, py = 0, pz = 0, pu = 0;
             for (int k0 = c0; k0 < c1; k0 += STEP) {
                 // independent loads first (padding points at the particle
-                // itself: r2 = 0 is skipped below)
+                // itself: r2 = 0 is masked below)
                 const int *lp = list_pass_at<TPI>(lg, k0);
                 int j[UNR];
 #pragma unroll
@@ -355,7 +398,16 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
                     const T dy = iy * sc + iy * sc_lo;
                     const T dz = iz * sc + iz * sc_lo;
                     const T r2 = dx * dx + dy * dy + dz * dz;
-                    if (r2 < rc2 && r2 > (T)0) {
+                    const bool in = r2 < rc2 && r2 > (T)0;
+                    if constexpr (TAB) {
+                        T fr, ph;
+                        pair_table64(in ? r2 : rc2, inv_h, tab_n, ppl_tab64, fr, ph);
+                        fr = in ? fr : (T)0;
+                        px += fr * dx;
+                        py += fr * dy;
+                        pz += fr * dz;
+                        pu += in ? ph : (T)0;
+                    } else if (in) {
                         T fr, ph;
                         pair_direct(r2, R, fr, ph);
                         px += fr * dx;
@@ -782,6 +834,8 @@ template <typename T> void configure_pp_kernels()
         set(k_pp_f32<1, PP_DYN>); set(k_pp_f32<2, PP_DYN>);
         set(k_pp_f32<4, PP_DYN>); set(k_pp_f32<8, PP_DYN>);
     }
+    // (the FP64 table, at most PP64_MAX_N intervals of 64 bytes, fits the default limit)
+    static_assert(PP64_MAX_N * 4 * sizeof(double2) <= 48 * 1024 - 1024, "FP64 table size");
 }
 
 template <typename T> void launch_quantize(const DevState &s, cudaStream_t st)
@@ -830,9 +884,14 @@ template <typename T, int TPI> static void launch_pp_tpi(const DevState &s, cuda
             s.reps, s.nrep, (const uint4 *)s.xq, s.nnb, s.nlist, s.maxnb, s.pp_tables,
             (float4 *)s.acc_pp, s.u_pp_part, pa);
     } else {
-        k_pp_f64<TPI><<<s.pp_nblk, PPL_THREADS, 0, st>>>(s.reps, s.nrep, (const Q *)s.xq, s.nnb,
-                                                         s.nlist, s.maxnb, (double4 *)s.acc_pp,
-                                                         s.u_pp_part);
+        if (s.pp64_n > 0)
+            k_pp_f64<TPI, true><<<s.pp_nblk, PPL_THREADS, s.pp64_n * 4 * sizeof(double2), st>>>(
+                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, s.pp_tables64, s.pp64_n,
+                (double4 *)s.acc_pp, s.u_pp_part);
+        else
+            k_pp_f64<TPI, false><<<s.pp_nblk, PPL_THREADS, 0, st>>>(
+                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, nullptr, 0,
+                (double4 *)s.acc_pp, s.u_pp_part);
     }
 }
 
