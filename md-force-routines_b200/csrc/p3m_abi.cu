@@ -519,7 +519,13 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     plan_mesh_passes(ctx);
     s.nblk = blk;
     s.max_mesh = maxm;
-    plan_lists(ctx, -1.0, p >= 148 * 256 * 2 ? 1 : (p >= 148 * 64 ? 2 : 4));
+    // Threads per particle, from step times (FP32, us per step with 1 / 2 / 4 / 8):
+    // 2e3 particles 61 / 54 / 54 / 53, 1e4 71 / 67 / 74 / 70, 1e5 335 / 318 /
+    // 340 / 364, 2e5 in 20 replicas 456 / 442 / 469 / 554, 1e6 2270 / 2107 /
+    // 2217 / 2698: four while two would leave most SMs without a block, then
+    // two -- one, though it fills the SMs from 7.6e4 particles on, ends with a
+    // longer last wave of longer blocks.
+    plan_lists(ctx, -1.0, p >= 148 * 64 ? 2 : 4);
 
     auto cleanup = [&](int code) {
         std::string e = ctx->err;
@@ -643,15 +649,15 @@ template <typename T> static void seq_sort(p3m_ctx *ctx, bool keys)
         launch_cell_keys(s, ctx->st);
         ctx->launches++;
     }
-    launch_scan(s, ctx->st);
+    launch_scan_cells(s, ctx->st);
     launch_scatter(s, ctx->st);
     launch_fix_cells<T>(s, ctx->st);
-    launch_quantize<T>(s, ctx->st);     // sorted coordinates of this step
-    launch_build_lists<T>(s, ctx->st);  // from those coordinates (rebuild steps)
-    ctx->launches += 5;
+    launch_build_lists<T>(s, ctx->st);  // rebuild steps
+    ctx->launches += 4;
     if (s.has_mesh) {
+        launch_scan_bricks(s, ctx->st);
         launch_place_bricks<T>(s, ctx->st);
-        ctx->launches++;
+        ctx->launches += 2;
     }
 }
 
@@ -725,7 +731,7 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
 {
     DevState &s = ctx->s;
     cudaStream_t st = ctx->st, st2 = ctx->st2;
-    launch_kick_drift(s, st);
+    launch_kick_drift<T>(s, st);
     ctx->launches++;
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
     const bool fork = s.has_mesh || rec;
@@ -735,7 +741,7 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
         if (e == cudaSuccess && s.has_mesh) {
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
-                launch_scan(s, st2, 1);
+                launch_scan_bricks(s, st2);
                 launch_place_bricks<T>(s, st2);
                 ctx->launches += 2;
                 seq_pm<T>(ctx, false, st2);
@@ -754,12 +760,11 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
         }
     }
     launch_cell_keys(s, st);
-    launch_scan(s, st, s.has_mesh ? 0 : -1);  // without a mesh branch: the bricks here too
+    launch_scan_cells(s, st);
     launch_scatter(s, st);
     launch_fix_cells<T>(s, st);
-    launch_quantize<T>(s, st);     // sorted coordinates of this step
-    launch_build_lists<T>(s, st);  // from those coordinates (rebuild steps)
-    ctx->launches += 6;
+    launch_build_lists<T>(s, st);  // rebuild steps
+    ctx->launches += 5;
     seq_pp<T>(ctx, false, st);
     if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
     if (e == cudaSuccess && rec) e = cudaStreamWaitEvent(st, ctx->ev_join3, 0);
@@ -1696,7 +1701,7 @@ template <typename T> static void enqueue_stage(p3m_ctx *ctx, int k)
     DevState &s = ctx->s;
     switch (k) {
     case 0:
-        launch_kick_drift(s, ctx->st);
+        launch_kick_drift<T>(s, ctx->st);
         seq_sort<T>(ctx, false);
         break;
     case 1: seq_sort<T>(ctx, true); break;

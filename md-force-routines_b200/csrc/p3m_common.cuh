@@ -169,6 +169,43 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Integer fixed-point coordinates of the pair stages (see p3m_pp.cu).
+template <typename T> struct Coord;
+template <> struct Coord<float> {
+    using Q = uint4;
+    using U = unsigned int;
+    using I = int;
+    static constexpr double scale = 4294967296.0;  // 2^32
+    __device__ static U q(double t) { return __double2uint_rz(t * scale); }
+};
+template <> struct Coord<double> {
+    using Q = ulonglong4;
+    using U = unsigned long long;
+    using I = long long;
+    static constexpr double scale = 18446744073709551616.0;  // 2^64
+    __device__ static U q(double t) { return __double2ull_rz(t * scale); }
+};
+
+// frac(x / L) in [0, 1)
+__device__ __forceinline__ double unit_coord(double x, double inv_L)
+{
+    double t = x * inv_L;
+    t -= floor(t);
+    return t < 1.0 ? t : 0.0;
+}
+
+// Integer coordinates of a position, the replica index in .w.
+template <typename T>
+__device__ __forceinline__ typename Coord<T>::Q quantize(double x, double y, double z, double inv_L, int r)
+{
+    typename Coord<T>::Q q;
+    q.x = Coord<T>::q(unit_coord(x, inv_L));
+    q.y = Coord<T>::q(unit_coord(y, inv_L));
+    q.z = Coord<T>::q(unit_coord(z, inv_L));
+    q.w = r;
+    return q;
+}
+
 // One periodic fold by a box length (positions are kept in [-L, 2L)).
 __device__ __forceinline__ double fold_box(double x, double L)
 {

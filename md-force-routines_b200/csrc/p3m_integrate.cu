@@ -32,12 +32,19 @@ __device__ __forceinline__ double wrap_once(double x, double L)
     return x;
 }
 
+// Also the coordinates of the pair stage, at the slots of the last cell sort
+// (a replica that rebuilds this step has them rewritten at its new slots by
+// k_fix_cells): a pass of its own read the positions again at random (1e6
+// particles: 40 us).
+template <typename T>
 __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                              double *__restrict__ pos, double *__restrict__ vel,
                              const double *__restrict__ acc, const double *__restrict__ pos_ref,
                              int ntot, int *__restrict__ brick_key, int *__restrict__ brick_rank,
                              int *__restrict__ brick_count, int has_mesh, int *rebuild, int *status,
-                             const double *__restrict__ pos_pref, int *prune)
+                             const double *__restrict__ pos_pref, int *prune,
+                             const int *__restrict__ cell_slot,
+                             typename Coord<T>::Q *__restrict__ xq)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int r = prep[i];
@@ -67,11 +74,13 @@ __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restr
         if (!vfin) raise_status(status, ST_NONFINITE);
         if (d2 > 0.25 * R.skin * R.skin && !rebuild[r]) atomicOr(rebuild + r, 1);
         if (pos_pref && d2p > 0.25 * R.pbuf * R.pbuf && !prune[r]) atomicOr(prune + r, 1);
-        int b;
+        int b, rank = 0;
         particle_keys(R, x[0], x[1], x[2], has_mesh, nullptr, &b, status);
+        if (b >= 0) rank = atomicAdd(&brick_count[b * BRICK_CNT_STRIDE], 1);
+        xq[cell_slot[i]] = quantize<T>(x[0], x[1], x[2], R.inv_L, r);  // while the atomic returns
         if (b >= 0) {
             brick_key[i] = b;
-            brick_rank[i] = atomicAdd(&brick_count[b * BRICK_CNT_STRIDE], 1);
+            brick_rank[i] = rank;
         }
     }
 }
@@ -557,13 +566,13 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
 // ---------------------------------------------------------------------------
 static int pgrid(int n) { int g = (n + 255) / 256; return g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g); }
 
-void launch_kick_drift(const DevState &s, cudaStream_t st)
+template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st)
 {
     const bool inner = s.prune_buf > 0.0;
-    k_kick_drift<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
+    k_kick_drift<T><<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
                                                 s.ntot, s.brick_key, s.brick_rank, s.brick_count, s.has_mesh,
                                                 s.rebuild, s.status, inner ? s.pos_pref : nullptr,
-                                                s.prune);
+                                                s.prune, s.cell_slot, (typename Coord<T>::Q *)s.xq);
 }
 
 void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
@@ -652,6 +661,7 @@ void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double
 int gf_opt_blocks(int M) { return (int)(((long long)M * M * M + 255) / 256); }
 
 #define P3M_INST(T)                                                                             \
+    template void launch_kick_drift<T>(const DevState &, cudaStream_t);                          \
     template void launch_kick_finish<T>(const DevState &, int, double *, cudaStream_t);          \
     template void launch_nqt<T>(const DevState &, const double *, const double *, int, int,      \
                                 double *, double *, const int *, int, cudaStream_t);            \

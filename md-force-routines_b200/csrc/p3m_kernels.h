@@ -42,7 +42,7 @@ struct DevState {
     int *cell_sub = nullptr;     // [particle] sub-cell Morton code (rebuild steps)
     int *nlist = nullptr;        // neighbour lists (sorted indices), in 16-entry group blocks (list_index)
     int *rebuild = nullptr;      // per-replica flags: rebuild cells and lists this step
-    // the replicas rebuilding this step (written by k_scan): [0] = count k,
+    // the replicas rebuilding this step (written by k_scan_cells): [0] = count k,
     // [1 .. k] replica indices, [nrep + 1 + j] = cells of the first j of them
     int *rb_list = nullptr;
     double *pos_ref = nullptr;   // positions at the last rebuild (ntot,3)
@@ -89,11 +89,11 @@ template <typename T> void configure_pp_kernels();
 template <typename T> void configure_mesh_kernels();
 template <typename T> void launch_keys(const DevState &s, cudaStream_t st);
 void launch_cell_keys(const DevState &s, cudaStream_t st);
-void launch_scan(const DevState &s, cudaStream_t st, int part = -1);  // -1 both, 0 cells, 1 bricks
+void launch_scan_cells(const DevState &s, cudaStream_t st);
+void launch_scan_bricks(const DevState &s, cudaStream_t st);
 void launch_scatter(const DevState &s, cudaStream_t st);
 template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st);
 template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t st);
-template <typename T> void launch_quantize(const DevState &s, cudaStream_t st);
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st);
 template <typename T> void launch_pp(const DevState &s, cudaStream_t st);
 int pp_particles_per_block(int tpi);
@@ -119,7 +119,7 @@ template <typename T> void launch_efield_from_mesh(const DevState &s, int rep,
 void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double L,
                    double *G_k, double *a_part, cudaStream_t st);
 
-void launch_kick_drift(const DevState &s, cudaStream_t st);
+template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st);
 template <typename T> void launch_kick_finish(const DevState &s, int do_kick, double *ep_out,
                                               cudaStream_t st);
 // Sums that k_step_reduce can take over from k_reduce_pp, k_reduce_pm and

@@ -45,51 +45,8 @@
 namespace p3m {
 
 // ---------------------------------------------------------------------------
-// coordinates
+// coordinates (Coord<T>, quantize: p3m_common.cuh)
 // ---------------------------------------------------------------------------
-template <typename T> struct Coord;
-template <> struct Coord<float> {
-    using Q = uint4;
-    using U = unsigned int;
-    using I = int;
-    static constexpr double scale = 4294967296.0;  // 2^32
-    __device__ static U q(double t) { return __double2uint_rz(t * scale); }
-};
-template <> struct Coord<double> {
-    using Q = ulonglong4;
-    using U = unsigned long long;
-    using I = long long;
-    static constexpr double scale = 18446744073709551616.0;  // 2^64
-    __device__ static U q(double t) { return __double2ull_rz(t * scale); }
-};
-
-// frac(x / L) in [0, 1)
-__device__ __forceinline__ double unit_coord(double x, double inv_L)
-{
-    double t = x * inv_L;
-    t -= floor(t);
-    return t < 1.0 ? t : 0.0;
-}
-
-// Sorted-order integer coordinates, every step: xq[s] = q(pos[cell_perm[s]]);
-// .w holds the replica index.
-template <typename T>
-__global__ void k_quantize(const RepDev *__restrict__ reps, const int *__restrict__ prep,
-                           const int *__restrict__ cell_perm, const double *__restrict__ pos,
-                           typename Coord<T>::Q *__restrict__ xq, int ntot)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ntot; s += gridDim.x * blockDim.x) {
-        const int i = cell_perm[s];
-        const int r = prep[i];
-        const double il = reps[r].inv_L;
-        typename Coord<T>::Q q;
-        q.x = Coord<T>::q(unit_coord(pos[3 * i + 0], il));
-        q.y = Coord<T>::q(unit_coord(pos[3 * i + 1], il));
-        q.z = Coord<T>::q(unit_coord(pos[3 * i + 2], il));
-        q.w = r;
-        xq[s] = q;
-    }
-}
 
 // dx of two coordinates (minimum image) in units of L / 2^B
 template <typename T>
@@ -112,7 +69,7 @@ constexpr int LB_SCAP = 1024;                 // candidates staged per window (1
 static_assert(cell_stencil(CELL_DIV_MAX) <= LB_THREADS, "one thread per stencil cell");
 static_assert(LB_TPI >= PP_LIST_PAD, "one pad entry per lane at most");
 
-// One CTA per cell of the replicas rebuilding this step (the list k_scan
+// One CTA per cell of the replicas rebuilding this step (the list k_scan_cells
 // wrote); cells are (rc + skin)/D wide (about 10 particles at D = 2 and unit
 // density 3/(4 pi), 80 at D = 1). The (2D+1)^3 neighbour cells'
 // coordinates are staged in shared memory in the fixed stencil order (x
@@ -813,8 +770,6 @@ __global__ void k_reduce_pp(const RepDev *__restrict__ reps, int nrep,
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-static int qgrid(int n) { int g = (n + 255) / 256; return g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g); }
-
 int pp_particles_per_block(int tpi) { return PPL_THREADS / tpi; }
 
 template <typename T> void configure_pp_kernels()
@@ -836,12 +791,6 @@ template <typename T> void configure_pp_kernels()
     }
     // (the FP64 table, at most PP64_MAX_N intervals of 64 bytes, fits the default limit)
     static_assert(PP64_MAX_N * 4 * sizeof(double2) <= 48 * 1024 - 1024, "FP64 table size");
-}
-
-template <typename T> void launch_quantize(const DevState &s, cudaStream_t st)
-{
-    k_quantize<T><<<qgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.cell_perm, s.pos,
-                                                 (typename Coord<T>::Q *)s.xq, s.ntot);
 }
 
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st)
@@ -914,7 +863,6 @@ void launch_reduce_pp(const DevState &s, cudaStream_t st)
 
 #define P3M_INST(T)                                                         \
     template void configure_pp_kernels<T>();                                 \
-    template void launch_quantize<T>(const DevState &, cudaStream_t);        \
     template void launch_build_lists<T>(const DevState &, cudaStream_t);     \
     template void launch_pp<T>(const DevState &, cudaStream_t);
 P3M_INST(float)

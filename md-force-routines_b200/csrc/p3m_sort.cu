@@ -22,9 +22,9 @@
 // (the assignment sums integers, the gather works per particle). Against a
 // stable sort (chunk histograms, a column scan and a warp per chunk placing
 // its particles in index order) that is two kernels and two passes fewer:
-// per step 14.5 -> 6.4 us of drift and
-// sort kernels for 1e4 particles on 64^3, 43 -> 14 for 1e5 on 128^3, 153 -> 65
-// for 1e6 on 256^3.
+// per
+// step 14.5 -> 6.4 us of drift and sort kernels for 1e4 particles on 64^3, 43
+// -> 14 for 1e5 on 128^3, 153 -> 65 for 1e6 on 256^3.
 #include "p3m_kernels.h"
 
 namespace p3m {
@@ -55,8 +55,11 @@ __global__ void k_keys(const RepDev *__restrict__ reps, const int *__restrict__ 
 __global__ void k_cell_keys(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                             const double *__restrict__ pos, int ntot, int *__restrict__ cell_key,
                             int *__restrict__ cell_sub, int *__restrict__ cell_count,
-                            const int *__restrict__ rebuild, int *status)
+                            const int *__restrict__ rebuild, int nrep, int *status)
 {
+    int any = 0;  // nothing to do on most steps
+    for (int r = threadIdx.x; r < nrep; r += blockDim.x) any |= rebuild[r];
+    if (!__syncthreads_or(any)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int r = prep[i];
         if (!rebuild[r]) continue;
@@ -69,83 +72,123 @@ __global__ void k_cell_keys(const RepDev *__restrict__ reps, const int *__restri
     }
 }
 
+// Exclusive sum over the block's threads of v; *total: the sum of all. sm: 33
+// ints. Ends with a barrier.
+__device__ int block_excl_scan(int v, int *total, int *sm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += t;
+    }
+    if (lane == 31) sm[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const int own = lane < nw ? sm[lane] : 0;
+        int s = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        sm[lane] = s - own;  // exclusive warp totals
+        if (lane == 31) sm[32] = s;
+    }
+    __syncthreads();
+    const int e = sm[w] + x - v;
+    *total = sm[32];
+    __syncthreads();
+    return e;
+}
+
 // Exclusive scan of count[0], count[STRIDE], ... (n of them) into start[0..n],
 // offset by `base` (single block), zeroing the counts and the scatter cursors
-// (may be NULL) for the next use.
+// (may be NULL) for the next use. Four entries per thread and round.
 template <int STRIDE>
 __device__ void block_scan_array(int *count, int *start, int *cursor, int n, int base, int *sm)
 {
     int carry = base;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-    for (int b0 = 0; b0 < n; b0 += blockDim.x) {
-        int i = b0 + tid;
-        int v = (i < n) ? count[i * STRIDE] : 0;
-        int x = v;
+    for (int b0 = 0; b0 < n; b0 += 4 * blockDim.x) {
+        const int i0 = b0 + 4 * threadIdx.x;
+        int v[4], sum = 0, total;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += t;
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i0 + k < n ? count[(i0 + k) * STRIDE] : 0;
+            sum += v[k];
         }
-        if (lane == 31) sm[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            int s = (lane < nw) ? sm[lane] : 0;
+        int e = carry + block_excl_scan(sum, &total, sm);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, s, o);
-                if (lane >= o) s += t;
+        for (int k = 0; k < 4; ++k) {
+            if (i0 + k < n) {
+                start[i0 + k] = e;
+                count[(i0 + k) * STRIDE] = 0;
+                if (cursor) cursor[i0 + k] = 0;
             }
-            sm[32 + lane] = s;  // inclusive warp totals
+            e += v[k];
         }
-        __syncthreads();
-        int excl = carry + x - v + (w > 0 ? sm[32 + w - 1] : 0);
-        if (i < n) {
-            start[i] = excl;
-            count[i * STRIDE] = 0;
-            if (cursor) cursor[i] = 0;
-        }
-        carry += sm[32 + nw - 1];
-        __syncthreads();
+        carry += total;
     }
-    if (tid == 0) start[n] = carry;
+    if (threadIdx.x == 0) start[n] = carry;
 }
 
-// Block 0: the cells of every replica whose rebuild flag is set, each within
-// its own particle range [p_off, p_off + n). Block 1: all bricks.
-__global__ void k_scan(const RepDev *__restrict__ reps, int nrep, int *cell_count,
-                       int *cell_start, int *cell_cursor, int *brick_count, int *brick_start,
-                       int nbrick, const int *__restrict__ rebuild,
-                       int *__restrict__ rb_list, int first_part)
+// Block r: replica r's cells, within its own particle range [p_off, p_off + n),
+// when its rebuild flag is set. Block 0 also writes the list of the rebuilding
+// replicas and their cells.
+__global__ void k_scan_cells(const RepDev *__restrict__ reps, int nrep, int *cell_count,
+                             int *cell_start, int *cell_cursor, const int *__restrict__ rebuild,
+                             int *__restrict__ rb_list)
 {
-    __shared__ int sm[64];
-    if (blockIdx.x + first_part == 0) {
+    __shared__ int sm[33];
+    if (blockIdx.x == 0) {
         int k = 0, cells = 0;
-        for (int r = 0; r < nrep; ++r) {
-            if (!rebuild[r]) continue;
-            const RepDev &R = reps[r];
-            const int c0 = R.cell_off, nc = R.nc * R.nc * R.nc;
-            block_scan_array<1>(cell_count + c0, cell_start + c0, cell_cursor + c0, nc, R.p_off, sm);
-            if (threadIdx.x == 0) {
-                rb_list[1 + k] = r;
-                rb_list[nrep + 1 + k] = cells;
+        for (int r0 = 0; r0 < nrep; r0 += blockDim.x) {
+            const int r = r0 + threadIdx.x;
+            const bool on = r < nrep && rebuild[r] != 0;
+            const int nc = on ? reps[r].nc : 0;
+            int nk, ncells;
+            const int ek = k + block_excl_scan(on ? 1 : 0, &nk, sm);
+            const int ec = cells + block_excl_scan(nc * nc * nc, &ncells, sm);
+            if (on) {
+                rb_list[1 + ek] = r;
+                rb_list[nrep + 1 + ek] = ec;
             }
-            ++k;
-            cells += nc;
-            __syncthreads();
+            k += nk;
+            cells += ncells;
         }
         if (threadIdx.x == 0) {
             rb_list[0] = k;
             rb_list[nrep + 1 + k] = cells;
         }
-    } else if (nbrick > 0) {
-        block_scan_array<BRICK_CNT_STRIDE>(brick_count, brick_start, nullptr, nbrick, 0, sm);
+    }
+    for (int r = blockIdx.x; r < nrep; r += gridDim.x) {
+        if (!rebuild[r]) continue;  // block-uniform
+        const RepDev &R = reps[r];
+        block_scan_array<1>(cell_count + R.cell_off, cell_start + R.cell_off,
+                            cell_cursor + R.cell_off, R.nc * R.nc * R.nc, R.p_off, sm);
+    }
+}
+
+// Block r: replica r's bricks (all its particles lie in them).
+__global__ void k_scan_bricks(const RepDev *__restrict__ reps, int nrep, int *brick_count,
+                              int *brick_start)
+{
+    __shared__ int sm[33];
+    for (int r = blockIdx.x; r < nrep; r += gridDim.x) {
+        const RepDev &R = reps[r];
+        block_scan_array<BRICK_CNT_STRIDE>(brick_count + R.brick_off * BRICK_CNT_STRIDE,
+                                           brick_start + R.brick_off, nullptr,
+                                           R.nb * R.nb * R.nb, R.p_off, sm);
     }
 }
 
 __global__ void k_scatter(const int *__restrict__ cell_key, const int *__restrict__ cell_start,
                           int *cell_cursor, int *__restrict__ cell_tmp, int ntot,
-                          const int *__restrict__ prep, const int *__restrict__ rebuild)
+                          const int *__restrict__ prep, const int *__restrict__ rebuild,
+                          const int *__restrict__ rb_list)
 {
+    if (rb_list[0] == 0) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         if (rebuild[prep[i]]) {
             int c = cell_key[i];
@@ -154,23 +197,32 @@ __global__ void k_scatter(const int *__restrict__ cell_key, const int *__restric
     }
 }
 
-// One warp per cell: order the cell's particles by (sub-cell Morton code,
-// index) -- z-order inside the cell, so the particles of one warp of the PP
-// kernel are neighbours in space and walk their (similar) lists in step,
-// reading nearby coordinates -- and remember every particle's position at
-// this rebuild (the reference point of the skin check).
+// One warp per cell of the rebuilding replicas: order the cell's particles by
+// (sub-cell Morton code, index) -- z-order inside the cell, so the particles
+// of one warp of the PP kernel are neighbours in space and walk their
+// (similar) lists in step, reading nearby coordinates -- and write, at their
+// new slots, the coordinates of the pair stage and the reference point of the
+// skin check.
+template <typename T>
 __global__ void k_fix_cells(const RepDev *__restrict__ reps, int nrep,
                             const int *__restrict__ cell_start, const int *__restrict__ cell_tmp,
                             const int *__restrict__ cell_sub, const double *__restrict__ pos,
                             int *__restrict__ cell_perm, int *__restrict__ cell_slot,
-                            double *__restrict__ pos_ref, int ncell,
-                            const int *__restrict__ rebuild)
+                            double *__restrict__ pos_ref, typename Coord<T>::Q *__restrict__ xq,
+                            const int *__restrict__ rb_list)
 {
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
+    const int nrb = rb_list[0];
+    if (nrb == 0) return;
+    const int *rb_cells = rb_list + nrep + 1;
     auto key = [&](int i) { return ((unsigned long long)cell_sub[i] << 32) | (unsigned)i; };
-    for (int c = blockIdx.x * wpb + (threadIdx.x >> 5); c < ncell; c += gridDim.x * wpb) {
-        if (!rebuild[find_rep(c, nrep, [&](int k) { return reps[k].cell_off; })]) continue;
+    for (int item = blockIdx.x * wpb + (threadIdx.x >> 5); item < rb_cells[nrb];
+         item += gridDim.x * wpb) {
+        const int k = find_rep(item, nrb, [&](int j) { return rb_cells[j]; });
+        const int r = rb_list[1 + k];
+        const int c = reps[r].cell_off + item - rb_cells[k];
+        const double inv_L = reps[r].inv_L;
         const int start = cell_start[c], n = cell_start[c + 1] - start;
         for (int e0 = 0; e0 < n; e0 += 32) {
             int e = e0 + lane;
@@ -186,12 +238,14 @@ __global__ void k_fix_cells(const RepDev *__restrict__ reps, int nrep,
                     rank += (__shfl_sync(0xffffffffu, kf, t) < kv) ? 1 : 0;
             }
             if (e < n) {
-                int s = start + rank;
+                const int s = start + rank;
+                const double x = pos[3 * v + 0], y = pos[3 * v + 1], z = pos[3 * v + 2];
                 cell_perm[s] = v;
                 cell_slot[v] = s;
-                pos_ref[3 * v + 0] = pos[3 * v + 0];
-                pos_ref[3 * v + 1] = pos[3 * v + 1];
-                pos_ref[3 * v + 2] = pos[3 * v + 2];
+                pos_ref[3 * v + 0] = x;
+                pos_ref[3 * v + 1] = y;
+                pos_ref[3 * v + 2] = z;
+                xq[s] = quantize<T>(x, y, z, inv_L, r);
             }
         }
     }
@@ -270,22 +324,27 @@ void launch_cell_keys(const DevState &s, cudaStream_t st)
 {
     k_cell_keys<<<grid_for(s.ntot, 256), 256, 0, st>>>(s.reps, s.prep, s.pos, s.ntot, s.cell_key,
                                                        s.cell_sub, s.cell_count, s.rebuild,
-                                                       s.status);
+                                                       s.nrep, s.status);
 }
 
-// Both scans (block 0: the cells of the rebuilding replicas, block 1: the
-// bricks), or one of them: part 0 / 1.
-void launch_scan(const DevState &s, cudaStream_t st, int part)
+void launch_scan_cells(const DevState &s, cudaStream_t st)
 {
-    const int first = part == 1 ? 1 : 0, nblocks = part < 0 ? 2 : 1;
-    k_scan<<<nblocks, 1024, 0, st>>>(s.reps, s.nrep, s.cell_count, s.cell_start, s.cell_cursor,
-                                     s.brick_count, s.brick_start, s.has_mesh ? s.nbrick : 0, s.rebuild, s.rb_list, first);
+    k_scan_cells<<<s.nrep < 1024 ? s.nrep : 1024, 1024, 0, st>>>(
+        s.reps, s.nrep, s.cell_count, s.cell_start, s.cell_cursor, s.rebuild, s.rb_list);
+}
+
+void launch_scan_bricks(const DevState &s, cudaStream_t st)
+{
+    if (s.has_mesh)
+        k_scan_bricks<<<s.nrep < 1024 ? s.nrep : 1024, s.max_mesh > 64 ? 512 : 64, 0, st>>>(
+            s.reps, s.nrep, s.brick_count, s.brick_start);
 }
 
 void launch_scatter(const DevState &s, cudaStream_t st)
 {
     k_scatter<<<grid_for(s.ntot, 256), 256, 0, st>>>(s.cell_key, s.cell_start, s.cell_cursor,
-                                                      s.cell_tmp, s.ntot, s.prep, s.rebuild);
+                                                      s.cell_tmp, s.ntot, s.prep, s.rebuild,
+                                                      s.rb_list);
 }
 
 template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t st)
@@ -298,10 +357,9 @@ template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t s
 template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st)
 {
     const int wpb = 8;
-    int blocks = (s.ncell + wpb - 1) / wpb;
-    k_fix_cells<<<blocks, wpb * 32, 0, st>>>(s.reps, s.nrep, s.cell_start, s.cell_tmp, s.cell_sub,
-                                             s.pos, s.cell_perm, s.cell_slot, s.pos_ref, s.ncell,
-                                             s.rebuild);
+    k_fix_cells<T><<<grid_for(s.ncell, wpb), wpb * 32, 0, st>>>(
+        s.reps, s.nrep, s.cell_start, s.cell_tmp, s.cell_sub, s.pos, s.cell_perm, s.cell_slot,
+        s.pos_ref, (typename Coord<T>::Q *)s.xq, s.rb_list);
 }
 
 template void launch_keys<float>(const DevState &, cudaStream_t);
