@@ -326,8 +326,9 @@ typedef struct {
     int32_t plane_max;    /* meshes with sides up to this (0, 32 or 64) take the fused
                              y/z plane FFT kernel, larger ones the y and z pencil passes */
     int32_t gather_mode;  /* force gather: 0 = a CTA per mesh brick and field component,
-                             1 = a CTA per brick (one tile buffer), 2 = a CTA per brick
-                             with two buffers (FP32; FP64 takes 1 for 2)              */
+                             1 = a CTA per brick (one tile buffer; few bricks: as 0),
+                             2 = a CTA per brick with two buffers (FP32; FP64 takes
+                             1 for 2). All give the same values                       */
     double skin;          /* Verlet skin for every replica (< 0: each replica's own /
                              the default); get returns the last value set              */
     double prune_buf;     /* FP32 path: 0 = the pair kernel reads the Verlet lists

@@ -141,100 +141,117 @@ k_kick_finish(const RepDev *__restrict__ reps, int nrep, const int *__restrict__
     if (threadIdx.x == 0) kin_part[b] = t;
 }
 
-// Per replica: energies, temperature and the thermostat factor; one row of
-// the energy ring; step counter advance. mode: 0 NVE, 1 thermostat, 2 force
-// only (no kinetic terms). Single block.
-__global__ void k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
-                              const double *__restrict__ kin_part, double *__restrict__ rep_out,
-                              int mode, int *__restrict__ counters, double *__restrict__ ring,
-                              int ring_cap, int recorded, int snap_interval, int snap_cap,
-                              int *rebuild, int *status, StepSums sums, int *prune,
-                              double *prune_count)
+// Energies, temperature and the thermostat factor, one block per replica; one
+// row of the energy ring; the last block to finish advances the step counters.
+// mode: 0 NVE, 1 thermostat, 2 force only (no kinetic terms). Latency-bound, on
+// the step's serial tail: the partials are summed by the block's threads (entry
+// k by thread k mod SR_THREADS, then a fixed tree -- the same order whatever the
+// batch). One block for all replicas, a warp each, took 5.4 us for 1e4 particles
+// against 4.0, 7.4 for 20 x 1e4 against 5.9, 30 for 1e6 against 8.9.
+constexpr int SR_THREADS = 512;
+
+__global__ void __launch_bounds__(SR_THREADS)
+k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
+              const double *__restrict__ kin_part, double *__restrict__ rep_out,
+              int mode, int *__restrict__ counters, double *__restrict__ ring,
+              int ring_cap, int recorded, int snap_interval, int snap_cap,
+              int *rebuild, int *status, StepSums sums, int *prune, double *prune_count)
 {
     // counters: [0] steps since the run started, [1] energy-ring position,
     // [2] step index of the run's first step (thermostat_p3m_ord6.py:15 tests
     // it <= 1999), [3] n(q,t) rows recorded, [4] snapshots taken, [5] the
-    // snapshot slot this step writes (-1: none)
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // snapshot slot this step writes (-1: none), [6] blocks finished
+    __shared__ double part[3][SR_THREADS / 32];
+    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int it = counters[2] + counters[0];
     const int step = counters[1];
-    for (int r = w; r < nrep; r += nw) {
-        const RepDev &R = reps[r];
-        if (sums.u_pp_part) {
-            // k_reduce_pp and k_reduce_pm, in their order
-            const int b0 = R.pp_blk_off, b1 = (r + 1 < nrep) ? reps[r + 1].pp_blk_off : sums.pp_nblk;
-            double t = 0.0;
-            for (int k = b0 + lane; k < b1; k += 32) t += sums.u_pp_part[k];
-            t = warp_sum(t);
-            double tm = 0.0;
-            if (R.M > 0) {
-                const int cb = R.wc_off, ce = (r + 1 < nrep) ? reps[r + 1].wc_off : sums.wc_total;
-                const int pb = sums.wc_total + R.wp_off,
-                          pe = sums.wc_total + ((r + 1 < nrep) ? reps[r + 1].wp_off : sums.wp_total);
-                for (int k = cb + lane; k < ce; k += 32) tm += sums.u_pm_part[k];
-                for (int k = pb + lane; k < pe; k += 32) tm += sums.u_pm_part[k];
-                tm = warp_sum(tm);
-            }
-            if (lane == 0) {
-                rep_out[8 * r + RO_UPP] = 0.5 * t;
-                rep_out[8 * r + RO_UPM] = 0.5 * tm;
-            }
+    const RepDev &R = reps[r];
+    const bool last = r + 1 == nrep;
+    double t = 0.0, tm = 0.0, s = 0.0;
+    if (sums.u_pp_part) {  // (k_reduce_pp and k_reduce_pm outside a step)
+        const int b0 = R.pp_blk_off, b1 = last ? sums.pp_nblk : reps[r + 1].pp_blk_off;
+        for (int k = b0 + tid; k < b1; k += SR_THREADS) t += sums.u_pp_part[k];
+        if (R.M > 0) {
+            const int c0 = R.wc_off, c1 = last ? sums.wc_total : reps[r + 1].wc_off;
+            const int p0 = sums.wc_total + R.wp_off,
+                      p1 = sums.wc_total + (last ? sums.wp_total : reps[r + 1].wp_off);
+            for (int k = c0 + tid; k < c1; k += SR_THREADS) tm += sums.u_pm_part[k];
+            for (int k = p0 + tid; k < p1; k += SR_THREADS) tm += sums.u_pm_part[k];
         }
-        const int b0 = R.blk_off, b1 = (r + 1 < nrep) ? reps[r + 1].blk_off : nblk;
-        double s = 0.0;
-        for (int k = b0 + lane; k < b1; k += 32) s += kin_part[k];
-        s = warp_sum(s);
-        if (lane == 0) {
-            double *o = rep_out + 8 * r;
-            const double u_self = -R.n * R.alpha / 1.7724538509055160273;
-            const double U = R.uf * (o[RO_UPP] + o[RO_UPM] + u_self);
-            const double K = R.kf * s;
-            const double T = K / R.kf / (double)R.n;
-            double fact = 1.0;
-            if (mode == 1) {
-                // thermostat_p3m_ord6.py:15-23
-                fact = (it <= 1999) ? sqrt(R.t_desired / T)
-                                    : sqrt((20.0 * R.t_desired / T - 1.0) / 20.0);
-            }
-            if (!isfinite(U)) raise_status(status, ST_NONFINITE);
-            o[RO_USELF] = u_self;
-            o[RO_U] = U;
-            o[RO_K] = K;
-            o[RO_T] = T;
-            o[RO_FACT] = fact;
-            if (ring && ring_cap > 0) {
-                double *row = ring + ((long long)(step % ring_cap) * nrep + r) * 4;
-                row[0] = U;
-                row[1] = K;
-                row[2] = T;
-                row[3] = fact;
-            }
-        }
+    }
+    {
+        const int b0 = R.blk_off, b1 = last ? nblk : reps[r + 1].blk_off;
+        for (int k = b0 + tid; k < b1; k += SR_THREADS) s += kin_part[k];
+    }
+    t = warp_sum(t);
+    tm = warp_sum(tm);
+    s = warp_sum(s);
+    if (lane == 0) {
+        part[0][w] = t;
+        part[1][w] = tm;
+        part[2][w] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (mode != 2) {
-            counters[0] += 1;
-            counters[1] = step + 1;
-            if (recorded) counters[3] += 1;
-            // a snapshot after step `it` when (it + 1) % interval == 0, as the
-            // reference writes its files (yukawa_MD_p3m_ord6.py:222)
-            if (snap_interval > 0 && (it + 1) % snap_interval == 0) {
-                counters[5] = counters[4] % snap_cap;
-                counters[4] += 1;
-            } else {
-                counters[5] = -1;
-            }
-        }
-    }
-    // this step's lists are built (count them); the next drift decides again
-    for (int r = threadIdx.x; r < nrep; r += blockDim.x) {
-        if (rebuild[r] && mode != 2) rep_out[8 * r + RO_REBUILDS] += 1.0;
+    if (w == 1 && lane == 0) {  // beside the first warp's sums
+        // this step's lists are built (count them); the next drift decides again
+        const bool fr = rebuild[r] != 0;
+        if (fr && mode != 2) rep_out[8 * r + RO_REBUILDS] += 1.0;
         if (prune) {  // inner lists: count the builds that came without an outer rebuild
-            if (prune[r] && !rebuild[r] && mode != 2) prune_count[r] += 1.0;
+            if (prune[r] && !fr && mode != 2) prune_count[r] += 1.0;
             prune[r] = 0;
         }
         rebuild[r] = 0;
+    }
+    if (w != 0) return;
+    constexpr int NW = SR_THREADS / 32;
+    t = warp_sum(lane < NW ? part[0][lane] : 0.0);
+    tm = warp_sum(lane < NW ? part[1][lane] : 0.0);
+    s = warp_sum(lane < NW ? part[2][lane] : 0.0);
+    if (lane != 0) return;
+    double *o = rep_out + 8 * r;
+    const double u_pp = sums.u_pp_part ? 0.5 * t : o[RO_UPP];
+    const double u_pm = sums.u_pp_part ? 0.5 * tm : o[RO_UPM];
+    const double u_self = -R.n * R.alpha / 1.7724538509055160273;
+    const double U = R.uf * (u_pp + u_pm + u_self);
+    const double K = R.kf * s;
+    const double T = K / R.kf / (double)R.n;
+    double fact = 1.0;
+    if (mode == 1) {
+        // thermostat_p3m_ord6.py:15-23
+        fact = (it <= 1999) ? sqrt(R.t_desired / T) : sqrt((20.0 * R.t_desired / T - 1.0) / 20.0);
+    }
+    if (!isfinite(U)) raise_status(status, ST_NONFINITE);
+    o[RO_UPP] = u_pp;
+    o[RO_UPM] = u_pm;
+    o[RO_USELF] = u_self;
+    o[RO_U] = U;
+    o[RO_K] = K;
+    o[RO_T] = T;
+    o[RO_FACT] = fact;
+    if (ring && ring_cap > 0) {
+        double *row = ring + ((long long)(step % ring_cap) * nrep + r) * 4;
+        row[0] = U;
+        row[1] = K;
+        row[2] = T;
+        row[3] = fact;
+    }
+    if (mode == 2) return;
+    // every block has read the counters once all have taken a ticket
+    if (nrep > 1) {
+        __threadfence();
+        if (atomicAdd(&counters[6], 1) != nrep - 1) return;
+        counters[6] = 0;
+    }
+    counters[0] = it - counters[2] + 1;
+    counters[1] = step + 1;
+    if (recorded) counters[3] += 1;
+    // a snapshot after step `it` when (it + 1) % interval == 0, as the
+    // reference writes its files (yukawa_MD_p3m_ord6.py:222)
+    if (snap_interval > 0 && (it + 1) % snap_interval == 0) {
+        counters[5] = counters[4] % snap_cap;
+        counters[4] += 1;
+    } else {
+        counters[5] = -1;
     }
 }
 
@@ -594,7 +611,7 @@ void launch_step_reduce(const DevState &s, int mode, int *counters, double *ring
                         cudaStream_t st, int recorded, int snap_interval, int snap_cap,
                         const StepSums &sums)
 {
-    k_step_reduce<<<1, 1024, 0, st>>>(s.reps, s.nrep, s.nblk, s.kin_part, s.rep_out, mode,
+    k_step_reduce<<<s.nrep, SR_THREADS, 0, st>>>(s.reps, s.nrep, s.nblk, s.kin_part, s.rep_out, mode,
                                       counters, ring, ring_cap, recorded, snap_interval, snap_cap,
                                       s.rebuild, s.status, sums,
                                       s.prune_buf > 0.0 ? s.prune : nullptr, s.prune_count);

@@ -21,7 +21,8 @@ struct DevState {
     int cell_div = CELL_DIV_MAX; // PP cells are >= (rc + skin) / cell_div wide (1 or 2)
     int plane_max = 64;          // meshes up to this side take the fused y/z plane kernel
     int gather_mode = 1;         // gather: 0 a CTA per brick and component, 1 / 2 a CTA per
-                                 // brick with one / two tile buffers (2: FP32 only)
+                                 // brick with one / two tile buffers (1: with few bricks as 0;
+                                 // 2: FP32 only)
     int pp_nblk = 0;             // blocks of the PP force kernel (replica-aligned)
     int maxnb = 0;               // list capacity per particle
     double prune_buf = 0.0;      // inner-list buffer beyond rc (FP32; 0: no inner lists)

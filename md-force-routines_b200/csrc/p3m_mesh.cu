@@ -859,6 +859,13 @@ constexpr int GTILE = TILE * TILE * GTX;
 // component: three times the work items, each staging one tile and repeating
 // the weights, so the SMs' last wave is shorter and no CTA waits for its own
 // next copy).
+// gather_mode 1 takes NC = 1 up to GATHER_SPLIT_MAX bricks (measured, us alone
+// / step with a CTA per brick against three: 8 bricks 16.5 / 51.8 - 8.3 /
+// 46.5, 64 bricks 12.4 / 66.1 - 8.3 / 62.8, FP64 18.5 / 93.1 - 12.4 / 87.5,
+// 512 bricks 28.8 / 310.0 - 26.7 / 308.3) and NC = 3 beyond (step: 1280 bricks
+// 439.1 - 441.2, 2056 747.7 - 752.3, 4096 2066 - 2089).
+constexpr int GATHER_SPLIT_MAX = 512;
+
 template <typename T, int NB, int NC>
 __global__ void __launch_bounds__(G_THREADS, sizeof(T) == 4 ? (NB == 1 ? 4 : 1) : 2)
 k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
@@ -1179,7 +1186,7 @@ template <typename T> void launch_gather(const DevState &s, cudaStream_t st)
         k_gather<T, 2, 3><<<grid_items(s.nbrick, 148 * 16), G_THREADS, 2 * GTILE * sizeof(T), st>>>(
             s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (const T *)s.efield,
             s.nmesh, (A *)s.acc_pm, s.nbrick);
-    else if (s.gather_mode == 0)
+    else if (s.gather_mode == 0 || s.nbrick <= GATHER_SPLIT_MAX)
         k_gather<T, 1, 1><<<grid_items(3 * s.nbrick, 148 * 16), G_THREADS, GTILE * sizeof(T), st>>>(
             s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (const T *)s.efield,
             s.nmesh, (A *)s.acc_pm, s.nbrick);
