@@ -270,8 +270,8 @@ static void plan_mesh_passes(p3m_ctx *ctx)
             wp += M / 2 + 1;
             if (M > maxp) maxp = M;
         } else {
-            wb += (M / 2 + 1) * (M / PENCIL);
-            wc += (M / 2 + 1) * (M / PENCIL);
+            wb += (M / 2 + 1) * (M >> pencil_log(R.logM));
+            wc += (M / 2 + 1) * (M >> pencil_log(R.logM));
         }
     }
     s.wa = wa;
@@ -386,15 +386,19 @@ template <typename T> static int alloc_bulk(p3m_ctx *ctx)
         CK(valloc(&s.ek, (size_t)3 * s.nspec * sizeof(C)));
         CK(valloc(&s.green, (size_t)s.nspec * sizeof(T)));
         CK(valloc(&s.efield, (size_t)3 * s.nmesh * sizeof(T)));
-        // twiddles exp(-2 pi i k/256), k < 128, from long double
-        std::vector<C> tw(128);
-        for (int k = 0; k < 128; ++k) {
-            long double a = -2.0L * 3.141592653589793238462643383279502884L * k / 256.0L;
-            tw[k].x = (T)cosl(a);
-            tw[k].y = (T)sinl(a);
+        // twiddles W_M^{ab} of every mesh side (see Split), from long double
+        std::vector<C> tw(TWIDDLE_N);
+        for (int logM = 5; logM <= MAX_LOGM; ++logM) {
+            const int M = 1 << logM, rb = fft_rb(logM);
+            for (int a = 0; a < fft_ra(logM); ++a)
+                for (int b = 0; b < rb; ++b) {
+                    const long double ph = -2.0L * 3.141592653589793238462643383279502884L * (a * b) / M;
+                    tw[M - 32 + a * rb + b].x = (T)cosl(ph);
+                    tw[M - 32 + a * rb + b].y = (T)sinl(ph);
+                }
         }
-        CK(valloc(&s.twiddle, 128 * sizeof(C)));
-        CK(cudaMemcpy(s.twiddle, tw.data(), 128 * sizeof(C), cudaMemcpyHostToDevice));
+        CK(valloc(&s.twiddle, TWIDDLE_N * sizeof(C)));
+        CK(cudaMemcpy(s.twiddle, tw.data(), TWIDDLE_N * sizeof(C), cudaMemcpyHostToDevice));
         configure_mesh_kernels<T>();
     }
     configure_pp_kernels<T>();
@@ -487,7 +491,7 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
             spec += (long long)(M / 2 + 1) * M * M;
             tile += (long long)R.nb * R.nb * R.nb * TILE3;
             // U_f partials: one per pencil item, more than per plane item
-            wc_cap += (M / 2 + 1) * (M / PENCIL > 1 ? M / PENCIL : 1);
+            wc_cap += (M / 2 + 1) * (M >> pencil_log(R.logM));
             if (M > maxm) maxm = M;
         } else {
             R.brick_off = brick;

@@ -21,15 +21,18 @@ constexpr int TILE3 = TILE * TILE * TILE;
 // the 512 bricks of a 128^3 mesh: drift 17.2 us with packed counters).
 constexpr int BRICK_CNT_STRIDE = 32;
 
-// Lines per pencil tile in the FFT passes (consecutive y rows or z lines).
-constexpr int PENCIL = 16;
-constexpr int LOG_PENCIL = 4;
-static_assert(PENCIL == 1 << LOG_PENCIL, "PENCIL is 2^LOG_PENCIL");
+// Lines per item of the y and z FFT passes (log2): 32, or 16 at M = 256, so
+// that each of 256 threads has a 16-point DFT in the wider of the two passes.
+__host__ __device__ constexpr int pencil_log(int logM) { return logM >= 8 ? 4 : 5; }
+// The two DFT sizes of a line of 2^logM points, M = RA RB, and the entries of
+// the twiddle table (M = 32 .. 256 at M - 32, M entries each).
+__host__ __device__ constexpr int fft_ra(int logM) { return logM >= 7 ? 16 : (logM == 6 ? 8 : 4); }
+__host__ __device__ constexpr int fft_rb(int logM) { return (1 << logM) / fft_ra(logM); }
+constexpr int TWIDDLE_N = 480;
 // Complex lines per item of the x passes (two real rows each): 32, or M/2 for
 // M = 32, so each radix pass has a group for every one of 256 threads; 16 at
 // M = 256, where the shorter items balance the last wave (FFT 0.576 against
 // 0.587 ms at 256^3; at 64^3 16 lines measured 0.144 against 0.130).
-constexpr int XL_MAX = 32;
 // PP cells are at least (rc + skin) / D wide (D, the cell divisor of a
 // context: 1 or 2), so the neighbours of a particle lie in the (2 D + 1)^3
 // cells around its own.
@@ -70,8 +73,8 @@ struct RepDev {
     long long tile_off;    // offset into assignment tiles (nb^3 TILE^3)
     // work-item offsets of the mesh passes (prefix sums over replicas)
     int wa_off;            // x-R2C / x-C2R items: M * M/(2 x_lines)
-    int wb_off;            // y-line items: (M/2+1) * M/PENCIL (multi-pass replicas)
-    int wc_off;            // z-line items: (M/2+1) * M/PENCIL (multi-pass replicas)
+    int wb_off;            // y-line items: (M/2+1) * M >> pencil_log (multi-pass replicas)
+    int wc_off;            // z-line items: the same
     int wp_off;            // plane items: M/2+1 (replicas with M <= PLANE_MAX)
     int blk_off;           // offset of this replica's particle blocks (PBLK each)
     int pp_blk_off;        // offset of this replica's blocks in the PP force kernel

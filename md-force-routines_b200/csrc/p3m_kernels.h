@@ -73,7 +73,7 @@ struct DevState {
     void *green = nullptr;       // T influence function / V, [kx][z][y]
     void *efield = nullptr;      // T 3 real field meshes [3][z][y][x]
     void *acc_pm = nullptr;      // V4<T> PM acceleration, brick-sorted order
-    void *twiddle = nullptr;     // C2<T> exp(-2 pi i k / 256), k < 128
+    void *twiddle = nullptr;     // C2<T> [TWIDDLE_N] twiddles of every mesh side
     // reductions
     double *u_pp_part = nullptr;  // [pp_nblk]
     double *u_pm_part = nullptr;  // [wc + wp]

@@ -29,145 +29,125 @@
 // Overlapping tile halos are summed in a fixed order when the first FFT pass
 // reads the mesh.
 //
-// The FFT is an in-place radix-2 decimation-in-time transform of lines held
-// in shared memory (padded strides), with up to three stages per register
-// pass, the input permuted to bit-reversed order as it is loaded. Twiddles
-// exp(-2 pi i k/256) come from an FP64-accurate table.
+// The FFTs transform lines in two passes of register DFTs (Split) with one
+// exchange through shared memory; twiddles come from an FP64-accurate table.
 #include "p3m_kernels.h"
 
 namespace p3m {
 
 constexpr int FFT_THREADS = 256;  // a multiple of the largest mesh side (256)
-constexpr int LS = PENCIL + 1;  // padded line stride of the shared tiles
-constexpr int LSX = XL_MAX + 1;  // the same for the x passes
 
 template <typename T> using cplx = typename C2<T>::t;
-
-__device__ __forceinline__ int brev(int n, int logM) { return (int)(__brev((unsigned)n) >> (32 - logM)); }
 
 // signed frequency of index n on an M-point axis
 __device__ __forceinline__ int freq(int n, int M) { return n < (M >> 1) ? n : n - M; }
 
+// ---------------------------------------------------------------------------
+// FFT lines
+// ---------------------------------------------------------------------------
+
+// A line of M = RA RB points is transformed by two passes of register DFTs with
+// one exchange through shared memory between them: with n = RB n1 + n2 and
+// k = k1 + RA k2,
+//   X[k] = sum_n2 W_RB^{n2 k2} [ W_M^{n2 k1} sum_n1 x[n] W_RA^{n1 k1} ],
+// pass 1 is an RA-point DFT per n2 (elements RB apart) and the twiddles, pass 2
+// an RB-point DFT per k1; both in natural order, no bit reversal. An inverse
+// that follows a forward transform starts from what pass 2 left in registers:
+// k = k1 + RA k2 over k2 is pass 1 of the swapped split (RB-point DFTs of
+// elements RA apart). The lanes of a warp go along the lines where the data is
+// already in shared memory (conflict-free) and along the transform where lines
+// are contiguous in global memory.
+//
+// Bound: the x passes by the latency of their tile and spectrum reads, the y
+// and z passes by L2 and, at 256^3, HBM (the inverse y pass moves 404 MB in 65
+// us, 6.2 TB/s). Radix-2 passes of three stages through shared memory in
+// bit-reversed order, which this replaced, moved each element through it eight
+// times a line (two now). All passes of a step, before / after, FP32: one 64^3
+// mesh 26 / 19 us, 20 of them 125 / 93, 128^3 85 / 54, 256^3 573 / 330; FP64
+// one 64^3 38 / 28, 128^3 169 / 95.
+template <int LOGM> struct Split {
+    static constexpr int RA = fft_ra(LOGM), RB = fft_rb(LOGM);
+};
+
+// Twiddle table: for M = 32, 64, 128, 256 the products W_M^{ab} at
+// M - 32 + a RB + b (a < RA, b < RB).
 template <typename T>
 __device__ __forceinline__ void load_twiddles(cplx<T> *tw, const cplx<T> *g)
 {
-    for (int k = threadIdx.x; k < 128; k += blockDim.x) tw[k] = g[k];
+    for (int k = threadIdx.x; k < TWIDDLE_N; k += blockDim.x) tw[k] = g[k];
 }
 
-// In-place radix-2 decimation-in-time FFT of `nlines` lines of length 2^logM
-// held in shared memory, element n of line l at buf[l * ls + n * es]; input
-// in bit-reversed order, output natural; unnormalised, the inverse uses
-// conjugate twiddles; nlines = 2^lognl. Up to three consecutive radix-2 stages are done in
-// registers on groups of 8 (4, 2) elements, so the data passes through shared
-// memory -- and the block through a barrier -- once per three stages. Thread
-// b takes line b mod nlines, so consecutive threads touch consecutive lines.
-// Ends with a barrier.
-template <typename T, int LOGR>
-__device__ __forceinline__ void fft_group_pass(cplx<T> *buf, int logM, int ls, int es, int lognl,
-                                               const cplx<T> *tw, bool inverse, int s)
+template <typename T> __device__ __forceinline__ cplx<T> cadd(cplx<T> a, cplx<T> b) { return make_c<T>(a.x + b.x, a.y + b.y); }
+template <typename T> __device__ __forceinline__ cplx<T> csub(cplx<T> a, cplx<T> b) { return make_c<T>(a.x - b.x, a.y - b.y); }
+// times -i (forward) or +i (inverse)
+template <typename T, bool INV> __device__ __forceinline__ cplx<T> crot(cplx<T> a)
 {
-    constexpr int R = 1 << LOGR;
-    const int half = 1 << s;           // distance of the first stage's pairs
-    const int ngroups = 1 << (lognl + logM - LOGR);
-    for (int b = threadIdx.x; b < ngroups; b += blockDim.x) {
-        const int l = b & ((1 << lognl) - 1), g = b >> lognl;
-        const int k = g & (half - 1), blk = g >> s;
-        const int base = (blk << (s + LOGR)) + k;
-        cplx<T> x[R];
+    return INV ? make_c<T>(-a.y, a.x) : make_c<T>(a.y, -a.x);
+}
+// times w (forward) or conj(w) (inverse)
+template <typename T, bool INV> __device__ __forceinline__ cplx<T> ctw(cplx<T> a, cplx<T> w)
+{
+    if (INV) w.y = -w.y;
+    return cmul<T>(a, w);
+}
+
+template <typename T, bool INV>
+__device__ __forceinline__ void dft4(cplx<T> &a, cplx<T> &b, cplx<T> &c, cplx<T> &d)
+{
+    const cplx<T> s = cadd<T>(a, c), t = csub<T>(a, c), u = cadd<T>(b, d),
+                  v = crot<T, INV>(csub<T>(b, d));
+    a = cadd<T>(s, u);
+    b = cadd<T>(t, v);
+    c = csub<T>(s, u);
+    d = csub<T>(t, v);
+}
+
+// R-point DFT in registers, natural order in and out, unnormalised
+template <typename T, int R, bool INV> __device__ __forceinline__ void dft(cplx<T> (&x)[R])
+{
+    if constexpr (R == 4) {
+        dft4<T, INV>(x[0], x[1], x[2], x[3]);
+    } else if constexpr (R == 8) {
+        dft4<T, INV>(x[0], x[2], x[4], x[6]);
+        dft4<T, INV>(x[1], x[3], x[5], x[7]);
+        const T h = (T)0.70710678118654752440L;  // W_8 = (1 -+ i) h
+        const cplx<T> o1 = INV ? make_c<T>(h * (x[3].x - x[3].y), h * (x[3].x + x[3].y))
+                               : make_c<T>(h * (x[3].x + x[3].y), h * (x[3].y - x[3].x));
+        const cplx<T> o2 = crot<T, INV>(x[5]);
+        const cplx<T> o3 = INV ? make_c<T>(-h * (x[7].x + x[7].y), h * (x[7].x - x[7].y))
+                               : make_c<T>(h * (x[7].y - x[7].x), -h * (x[7].x + x[7].y));
+        const cplx<T> e0 = x[0], e1 = x[2], e2 = x[4], e3 = x[6], o0 = x[1];
+        x[0] = cadd<T>(e0, o0); x[4] = csub<T>(e0, o0);
+        x[1] = cadd<T>(e1, o1); x[5] = csub<T>(e1, o1);
+        x[2] = cadd<T>(e2, o2); x[6] = csub<T>(e2, o2);
+        x[3] = cadd<T>(e3, o3); x[7] = csub<T>(e3, o3);
+    } else {
+        static_assert(R == 16, "4, 8 or 16 points");
+        // 4 x 4: DFTs of elements 4 apart, twiddles W_16^{n2 k1}, DFTs over n2
 #pragma unroll
-        for (int r = 0; r < R; ++r) x[r] = buf[l * ls + (base + r * half) * es];
+        for (int n = 0; n < 4; ++n) dft4<T, INV>(x[n], x[n + 4], x[n + 8], x[n + 12]);
+        const T c1 = (T)0.92387953251128675613L, s1 = (T)0.38268343236508977173L,
+                h = (T)0.70710678118654752440L;
+        x[5] = ctw<T, INV>(x[5], make_c<T>(c1, -s1));    // W^1
+        x[9] = ctw<T, INV>(x[9], make_c<T>(h, -h));      // W^2
+        x[13] = ctw<T, INV>(x[13], make_c<T>(s1, -c1));  // W^3
+        x[6] = ctw<T, INV>(x[6], make_c<T>(h, -h));      // W^2
+        x[10] = crot<T, INV>(x[10]);                     // W^4
+        x[14] = ctw<T, INV>(x[14], make_c<T>(-h, -h));   // W^6
+        x[7] = ctw<T, INV>(x[7], make_c<T>(s1, -c1));    // W^3
+        x[11] = ctw<T, INV>(x[11], make_c<T>(-h, -h));   // W^6
+        x[15] = ctw<T, INV>(x[15], make_c<T>(-c1, s1));  // W^9
+        // x[4 k1 + n2] now; X[k1 + 4 k2] after the DFT over n2
 #pragma unroll
-        for (int t = 0; t < LOGR; ++t) {
-            // stage s + t: pairs (r, r + 2^t); twiddle W_{2^(s+t+1)}^{k + (r mod 2^t) half}
+        for (int k = 0; k < 4; ++k) dft4<T, INV>(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (r & (1 << t)) continue;
-                const int e = k + (r & ((1 << t) - 1)) * half;
-                cplx<T> w = tw[e << (7 - (s + t))];
-                if (inverse) w.y = -w.y;
-                const cplx<T> a = x[r], c = cmul<T>(w, x[r + (1 << t)]);
-                x[r] = make_c<T>(a.x + c.x, a.y + c.y);
-                x[r + (1 << t)] = make_c<T>(a.x - c.x, a.y - c.y);
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = a + 1; b < 4; ++b) {
+                const cplx<T> t = x[4 * a + b];
+                x[4 * a + b] = x[4 * b + a];
+                x[4 * b + a] = t;
             }
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) buf[l * ls + (base + r * half) * es] = x[r];
-    }
-    __syncthreads();
-}
-
-// The first three stages (a pass of fft_group_pass with s = 0): each group is
-// an 8-point DFT of elements base + r, r < 8, whose twiddles are the eighth
-// roots of unity 1, -i and (+-1 - i)/sqrt 2 (conjugated for the inverse), so
-// no table reads and only two real products per non-trivial rotation.
-template <typename T>
-__device__ __forceinline__ void fft_first_pass8(cplx<T> *buf, int logM, int ls, int es, int lognl,
-                                                bool inverse)
-{
-    const T h = (T)0.70710678118654752440L;  // cos(pi/4), as the twiddle table holds it
-    const int ngroups = 1 << (lognl + logM - 3);
-    for (int b = threadIdx.x; b < ngroups; b += blockDim.x) {
-        const int l = b & ((1 << lognl) - 1), base = (b >> lognl) << 3;
-        cplx<T> x[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) x[r] = buf[l * ls + (base + r) * es];
-        // stage 0: pairs (r, r+1), twiddle 1
-#pragma unroll
-        for (int r = 0; r < 8; r += 2) {
-            const cplx<T> a = x[r], c = x[r + 1];
-            x[r] = make_c<T>(a.x + c.x, a.y + c.y);
-            x[r + 1] = make_c<T>(a.x - c.x, a.y - c.y);
-        }
-        // stage 1: pairs (r, r+2); twiddle 1 for even r, -i (inverse: +i) for odd r
-#pragma unroll
-        for (int r = 0; r < 8; r += (r & 1) ? 3 : 1) {
-            const cplx<T> a = x[r], v = x[r + 2];
-            cplx<T> c = v;
-            if (r & 1) c = inverse ? make_c<T>(-v.y, v.x) : make_c<T>(v.y, -v.x);
-            x[r] = make_c<T>(a.x + c.x, a.y + c.y);
-            x[r + 2] = make_c<T>(a.x - c.x, a.y - c.y);
-        }
-        // stage 2: pairs (r, r+4), twiddle W_8^r (inverse: conjugate)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const cplx<T> a = x[r], v = x[r + 4];
-            cplx<T> c;
-            if (r == 0) {
-                c = v;
-            } else if (r == 2) {
-                c = inverse ? make_c<T>(-v.y, v.x) : make_c<T>(v.y, -v.x);
-            } else if (r == 1) {  // (1 - i)/sqrt 2, inverse (1 + i)/sqrt 2
-                c = inverse ? make_c<T>(h * (v.x - v.y), h * (v.x + v.y))
-                            : make_c<T>(h * (v.x + v.y), h * (v.y - v.x));
-            } else {              // (-1 - i)/sqrt 2, inverse (-1 + i)/sqrt 2
-                c = inverse ? make_c<T>(-h * (v.x + v.y), h * (v.x - v.y))
-                            : make_c<T>(h * (v.y - v.x), -h * (v.x + v.y));
-            }
-            x[r] = make_c<T>(a.x + c.x, a.y + c.y);
-            x[r + 4] = make_c<T>(a.x - c.x, a.y - c.y);
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) buf[l * ls + (base + r) * es] = x[r];
-    }
-    __syncthreads();
-}
-
-// The passes of one line length 2^LOGM from stage S on, unrolled at compile
-// time (stage offsets, group counts and twiddle strides become constants).
-template <typename T, int LOGM, int S = 0>
-__device__ __forceinline__ void fft_lines_t(cplx<T> *buf, int ls, int es, int lognl,
-                                            const cplx<T> *tw, bool inverse)
-{
-    if constexpr (S == 0 && LOGM >= 3) {
-        fft_first_pass8<T>(buf, LOGM, ls, es, lognl, inverse);
-        fft_lines_t<T, LOGM, 3>(buf, ls, es, lognl, tw, inverse);
-    } else if constexpr (S + 3 <= LOGM) {
-        fft_group_pass<T, 3>(buf, LOGM, ls, es, lognl, tw, inverse, S);
-        fft_lines_t<T, LOGM, S + 3>(buf, ls, es, lognl, tw, inverse);
-    } else if constexpr (LOGM - S == 2) {
-        fft_group_pass<T, 2>(buf, LOGM, ls, es, lognl, tw, inverse, S);
-    } else if constexpr (LOGM - S == 1) {
-        fft_group_pass<T, 1>(buf, LOGM, ls, es, lognl, tw, inverse, S);
     }
 }
 
@@ -437,35 +417,66 @@ __device__ __forceinline__ T rho_at(const RepDev &R, const T *__restrict__ tiles
 
 // Pass A: rows of the charge mesh (reduced from the tiles) -> R2C along x,
 // written transposed into spec[kx][z][y]. Item = (replica, z, tile of
-// 2 x_lines rows); two real rows share one complex line. The item body is
-// instantiated per mesh side, so its loop bounds, masks and shifts are
-// compile-time constants.
+// 2 x_lines rows); two real rows share one complex line. Instantiated per mesh
+// side. Pass 1 takes its elements straight from the tiles, all of a thread's
+// loads independent; pass 2 leaves X[k1 + RA k2] in slot k1 RB + k2 of the
+// line, and the two real rows are split from slots k and M - k.
+template <int LOGM> __host__ __device__ constexpr int x_stride()
+{
+    // line stride of the x passes (lines are the fast index): 16 lanes of RB
+    // (r2c) or RA (c2r) consecutive transform indices and the lines they span
+    // fall on 16 different 8-byte banks
+    constexpr int NL = 1 << x_lines_log(LOGM);
+    return LOGM == 8 ? NL + 1 : NL + 2;
+}
+
 template <typename T, int LOGM>
 __device__ __forceinline__ void x_r2c_item(const RepDev &R, int w, const T *__restrict__ tiles,
                                            cplx<T> *__restrict__ spec, cplx<T> *buf,
-                                           const cplx<T> *tw)
+                                           const cplx<T> *twt)
 {
-    constexpr int M = 1 << LOGM;
-    constexpr int LNL = x_lines_log(LOGM), NROW = 2 << LNL;  // complex lines, real rows
-    constexpr int NYT = M >> (LNL + 1), NK = (M >> 1) + 1;
-    static_assert(FFT_THREADS % M == 0, "each thread keeps one x");
+    constexpr int M = 1 << LOGM, RA = Split<LOGM>::RA, RB = Split<LOGM>::RB;
+    constexpr int LNL = x_lines_log(LOGM), NL = 1 << LNL, NROW = 2 << LNL;  // complex lines, real rows
+    constexpr int NYT = M >> (LNL + 1), NK = (M >> 1) + 1, LS = x_stride<LOGM>();
+    const cplx<T> *tw = twt + M - 32;
     const int z = w / NYT, y0 = (w % NYT) * NROW;
-    const int x = threadIdx.x & (M - 1);
-    const AxisOff ax = axis_x(x, R.nb), az = axis_z(z, R.nb);
+    const AxisOff az = axis_z(z, R.nb);
     const T *t = tiles + R.tile_off;
-    T *dst = reinterpret_cast<T *>(&buf[brev(x, LOGM) * LSX]);
     __syncthreads();
-    for (int j = threadIdx.x >> LOGM; j < NROW; j += FFT_THREADS >> LOGM)
-        dst[j] = rho_sum<T>(t, ax, axis_y(y0 + j, R.nb), az);  // line j/2, part j%2
+    for (int e = threadIdx.x; e < NL * RB; e += FFT_THREADS) {
+        const int n2 = e % RB, l = e / RB;
+        const AxisOff ya = axis_y(y0 + 2 * l, R.nb), yb = axis_y(y0 + 2 * l + 1, R.nb);
+        cplx<T> x[RA];
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) {
+            const AxisOff ax = axis_x(RB * n1 + n2, R.nb);
+            x[n1].x = rho_sum<T>(t, ax, ya, az);
+            x[n1].y = rho_sum<T>(t, ax, yb, az);
+        }
+        dft<T, RA, false>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            buf[(k1 * RB + n2) * LS + l] = k1 ? cmul<T>(x[k1], tw[k1 * RB + n2]) : x[0];
+    }
     __syncthreads();
-    fft_lines_t<T, LOGM>(buf, 1, LSX, LNL, tw, false);
+    for (int e = threadIdx.x; e < NL * RA; e += FFT_THREADS) {
+        const int l = e % NL, k1 = e / NL;
+        cplx<T> x[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = buf[(k1 * RB + n2) * LS + l];
+        dft<T, RB, false>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) buf[(k1 * RB + k2) * LS + l] = x[k2];
+    }
+    __syncthreads();
     // split the two real rows: Xa = (Z[k] + conj Z[M-k])/2, Xb = (Z[k] - conj Z[M-k])/2i
     cplx<T> *out = spec + R.spec_off + (long long)z * M + y0;
+    auto slot = [](int k) { return (k % RA) * RB + k / RA; };
     for (int e = threadIdx.x; e < NROW * NK; e += FFT_THREADS) {
         const int j = e & (NROW - 1), k = e >> (LNL + 1);
         const int l = j >> 1;
-        const cplx<T> Z = buf[k * LSX + l];
-        const cplx<T> Zm = buf[((M - k) & (M - 1)) * LSX + l];
+        const cplx<T> Z = buf[slot(k) * LS + l];
+        const cplx<T> Zm = buf[slot((M - k) & (M - 1)) * LS + l];
         cplx<T> X;
         if ((j & 1) == 0) {
             X.x = (T)0.5 * (Z.x + Zm.x);
@@ -479,13 +490,13 @@ __device__ __forceinline__ void x_r2c_item(const RepDev &R, int w, const T *__re
 }
 
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
 k_fft_x_r2c(const RepDev *__restrict__ reps, int nrep, const T *__restrict__ tiles,
             cplx<T> *__restrict__ spec, const cplx<T> *__restrict__ twg, int nitems)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<T> *tw = reinterpret_cast<cplx<T> *>(smem_raw);
-    cplx<T> *buf = tw + 128;
+    cplx<T> *buf = tw + TWIDDLE_N;
     load_twiddles<T>(tw, twg);
     for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
         const int r = find_rep(item, nrep, [&](int k) { return reps[k].wa_off; });
@@ -500,40 +511,57 @@ k_fft_x_r2c(const RepDev *__restrict__ reps, int nrep, const T *__restrict__ til
     }
 }
 
-// Passes B / D: FFT along y of contiguous lines spec[kx][z][:]. Item =
-// (replica, [component,] kx, 16-line z tile). `ncomp` arrays of `stride`
-// elements are processed (1 forward, 3 inverse). The item body is
-// instantiated per mesh side.
-template <typename T, int LOGM>
-__device__ __forceinline__ void y_item(const RepDev &R, int w, cplx<T> *__restrict__ data,
-                                       long long off, cplx<T> *buf, const cplx<T> *tw,
-                                       bool inverse)
+// Passes B / D: FFT along y of contiguous lines spec[kx][z][:], in place. Item
+// = (replica, [component,] kx, tile of z lines). `ncomp` arrays of `stride`
+// elements are processed (1 forward, 3 inverse). Instantiated per mesh side.
+// Pass 1 reads and pass 2 writes global memory directly, lanes along y; the
+// strides of the exchange (k1 rows of RB + 1, lines of y_stride) keep both
+// sides of it conflict-free.
+template <int LOGM> __host__ __device__ constexpr int y_stride()
 {
-    constexpr int M = 1 << LOGM, NZT = M / PENCIL;
-    const int kx = w / NZT, z0 = (w % NZT) * PENCIL;
+    return LOGM == 8 ? 272 : (LOGM == 7 ? 152 : (LOGM == 6 ? 72 : 40));
+}
+
+template <typename T, int LOGM, bool INV>
+__device__ __forceinline__ void y_item(const RepDev &R, int w, cplx<T> *__restrict__ data,
+                                       long long off, cplx<T> *buf, const cplx<T> *twt)
+{
+    constexpr int M = 1 << LOGM, RA = Split<LOGM>::RA, RB = Split<LOGM>::RB;
+    constexpr int NL = 1 << pencil_log(LOGM), NZT = M / NL, LD = y_stride<LOGM>();
+    const cplx<T> *tw = twt + M - 32;
+    const int kx = w / NZT, z0 = (w % NZT) * NL;
     cplx<T> *base = data + off + R.spec_off + ((long long)kx * M + z0) * M;
     __syncthreads();
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int y = e & (M - 1), l = e >> LOGM;
-        buf[brev(y, LOGM) * LS + l] = base[l * M + y];
+    for (int e = threadIdx.x; e < NL * RB; e += FFT_THREADS) {
+        const int n2 = e % RB, l = e / RB;
+        cplx<T> x[RA];
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) x[n1] = base[l * M + RB * n1 + n2];
+        dft<T, RA, INV>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            buf[l * LD + k1 * (RB + 1) + n2] = k1 ? ctw<T, INV>(x[k1], tw[k1 * RB + n2]) : x[0];
     }
     __syncthreads();
-    if (inverse) fft_lines_t<T, LOGM>(buf, 1, LS, LOG_PENCIL, tw, true);
-    else fft_lines_t<T, LOGM>(buf, 1, LS, LOG_PENCIL, tw, false);
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int y = e & (M - 1), l = e >> LOGM;
-        base[l * M + y] = buf[y * LS + l];
+    for (int e = threadIdx.x; e < NL * RA; e += FFT_THREADS) {
+        const int k1 = e % RA, l = e / RA;
+        cplx<T> x[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = buf[l * LD + k1 * (RB + 1) + n2];
+        dft<T, RB, INV>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) base[l * M + k1 + RA * k2] = x[k2];
     }
 }
 
-template <typename T>
+template <typename T, bool INV>
 __global__ void __launch_bounds__(FFT_THREADS)
 k_fft_y(const RepDev *__restrict__ reps, int nrep, cplx<T> *__restrict__ data, long long stride,
-        int ncomp, const cplx<T> *__restrict__ twg, int nitems_per_comp, bool inverse)
+        int ncomp, const cplx<T> *__restrict__ twg, int nitems_per_comp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<T> *tw = reinterpret_cast<cplx<T> *>(smem_raw);
-    cplx<T> *buf = tw + 128;
+    cplx<T> *buf = tw + TWIDDLE_N;
     load_twiddles<T>(tw, twg);
     for (int item = blockIdx.x; item < nitems_per_comp * ncomp; item += gridDim.x) {
         const int comp = item / nitems_per_comp, it = item % nitems_per_comp;
@@ -542,10 +570,10 @@ k_fft_y(const RepDev *__restrict__ reps, int nrep, cplx<T> *__restrict__ data, l
         const int w = it - R.wb_off;
         const long long off = comp * stride;
         switch (R.logM) {  // block-uniform: one replica per item
-        case 5: y_item<T, 5>(R, w, data, off, buf, tw, inverse); break;
-        case 6: y_item<T, 6>(R, w, data, off, buf, tw, inverse); break;
-        case 7: y_item<T, 7>(R, w, data, off, buf, tw, inverse); break;
-        default: y_item<T, 8>(R, w, data, off, buf, tw, inverse); break;
+        case 5: y_item<T, 5, INV>(R, w, data, off, buf, tw); break;
+        case 6: y_item<T, 6, INV>(R, w, data, off, buf, tw); break;
+        case 7: y_item<T, 7, INV>(R, w, data, off, buf, tw); break;
+        default: y_item<T, 8, INV>(R, w, data, off, buf, tw); break;
         }
     }
 }
@@ -553,66 +581,93 @@ k_fft_y(const RepDev *__restrict__ reps, int nrep, cplx<T> *__restrict__ data, l
 // Pass C: forward FFT along z, U_f partial, phi = (G/V) rho_k, then the three
 // field spectra with their inverse z transforms. E_z = IFFT_z(-i kz phi);
 // E_x and E_y use psi = IFFT_z(phi) since their multipliers are constant
-// along z: E_x = -i kx psi, E_y = -i ky psi. Item = (replica, kx, 16-wide y
-// tile); the item body is instantiated per mesh side.
+// along z: E_x = -i kx psi, E_y = -i ky psi. Item = (replica, kx, tile of y);
+// instantiated per mesh side. Lanes go along y throughout. The multiplication
+// by G and by -i kz happens in registers between the forward transform's pass 2
+// and the inverse's pass 1 (split swapped): two exchanges in all.
 template <typename T, int LOGM>
 __device__ __forceinline__ void z_green_item(const RepDev &R, int w,
                                              const cplx<T> *__restrict__ spec,
                                              const T *__restrict__ green,
                                              cplx<T> *__restrict__ ek, long long nspec,
                                              double *__restrict__ u_out, cplx<T> *buf,
-                                             const cplx<T> *tw, double *red)
+                                             const cplx<T> *twt, double *red)
 {
-    constexpr int M = 1 << LOGM, NYT = M / PENCIL;
-    cplx<T> *buf2 = buf + M * LS;
-    const int kx = w / NYT, y0 = (w % NYT) * PENCIL;
+    constexpr int M = 1 << LOGM, RA = Split<LOGM>::RA, RB = Split<LOGM>::RB;
+    constexpr int NL = 1 << pencil_log(LOGM), NYT = M / NL;
+    const cplx<T> *tw = twt + M - 32;
+    cplx<T> *buf2 = buf + M * NL;
+    const int kx = w / NYT, y0 = (w % NYT) * NL;
     const long long lbase = R.spec_off + (long long)kx * M * M + y0;  // + z*M + l
     __syncthreads();
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int l = e & (PENCIL - 1), z = e >> LOG_PENCIL;
-        buf[brev(z, LOGM) * LS + l] = spec[lbase + z * M + l];
+    for (int e = threadIdx.x; e < NL * RB; e += FFT_THREADS) {
+        const int l = e % NL, n2 = e / NL;
+        cplx<T> x[RA];
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) x[n1] = spec[lbase + (RB * n1 + n2) * M + l];
+        dft<T, RA, false>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            buf[(k1 * RB + n2) * NL + l] = k1 ? cmul<T>(x[k1], tw[k1 * RB + n2]) : x[0];
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(buf, 1, LS, LOG_PENCIL, tw, false);
     const double wkx = (kx == 0 || kx == (M >> 1)) ? 1.0 : 2.0;
-    double u = 0.0;
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int l = e & (PENCIL - 1), n = e >> LOG_PENCIL;
-        const cplx<T> rk = buf[n * LS + l];
-        const T g = green[lbase + n * M + l];
-        u += wkx * (double)g * ((double)rk.x * rk.x + (double)rk.y * rk.y);
-        buf2[brev(n, LOGM) * LS + l] = make_c<T>(g * rk.x, g * rk.y);
-    }
-    __syncthreads();
     const T twopi_L = (T)(6.283185307179586477 * R.inv_L);
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int l = e & (PENCIL - 1), n = e >> LOG_PENCIL;
-        const int br = brev(n, LOGM);
-        const cplx<T> ph = buf2[br * LS + l];
-        const T kz = (n == (M >> 1)) ? (T)0 : twopi_L * (T)freq(n, M);
-        // -i kz phi = (kz phi.y, -kz phi.x)
-        buf[br * LS + l] = make_c<T>(kz * ph.y, -kz * ph.x);
+    double u = 0.0;
+    for (int e = threadIdx.x; e < NL * RA; e += FFT_THREADS) {
+        const int l = e % NL, k1 = e / NL;
+        T g[RB];
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) g[k2] = __ldg(green + lbase + (k1 + RA * k2) * M + l);
+        cplx<T> x[RB], f[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = buf[(k1 * RB + n2) * NL + l];
+        dft<T, RB, false>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) {
+            const int n = k1 + RA * k2;
+            u += wkx * (double)g[k2] * ((double)x[k2].x * x[k2].x + (double)x[k2].y * x[k2].y);
+            x[k2] = make_c<T>(g[k2] * x[k2].x, g[k2] * x[k2].y);
+            const T kz = (n == (M >> 1)) ? (T)0 : twopi_L * (T)freq(n, M);
+            f[k2] = make_c<T>(kz * x[k2].y, -kz * x[k2].x);  // -i kz phi
+        }
+        dft<T, RB, true>(x);
+        dft<T, RB, true>(f);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            const cplx<T> wj = tw[k1 * RB + j];
+            buf[(k1 * RB + j) * NL + l] = ctw<T, true>(f[j], wj);
+            buf2[(k1 * RB + j) * NL + l] = ctw<T, true>(x[j], wj);
+        }
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(buf, 1, LS, LOG_PENCIL, tw, true);   // E_z
-    fft_lines_t<T, LOGM>(buf2, 1, LS, LOG_PENCIL, tw, true);  // psi
     const T kxv = (kx == (M >> 1)) ? (T)0 : twopi_L * (T)kx;
-    for (int e = threadIdx.x; e < PENCIL * M; e += FFT_THREADS) {
-        const int l = e & (PENCIL - 1), z = e >> LOG_PENCIL;
+    for (int e = threadIdx.x; e < NL * RB; e += FFT_THREADS) {
+        const int l = e % NL, j = e / NL;
         const int yy = y0 + l;
         const T kyv = (yy == (M >> 1)) ? (T)0 : twopi_L * (T)freq(yy, M);
-        const cplx<T> ps = buf2[z * LS + l];
-        const long long o = lbase + z * M + l;
-        ek[o] = make_c<T>(kxv * ps.y, -kxv * ps.x);
-        ek[nspec + o] = make_c<T>(kyv * ps.y, -kyv * ps.x);
-        ek[2 * nspec + o] = buf[z * LS + l];
+        cplx<T> x[RA];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = buf[(k1 * RB + j) * NL + l];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) ek[2 * nspec + lbase + (j + RB * i) * M + l] = x[i];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = buf2[(k1 * RB + j) * NL + l];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) {
+            const long long o = lbase + (j + RB * i) * M + l;
+            ek[o] = make_c<T>(kxv * x[i].y, -kxv * x[i].x);
+            ek[nspec + o] = make_c<T>(kyv * x[i].y, -kyv * x[i].x);
+        }
     }
     const double ut = block_sum(u, red);
     if (threadIdx.x == 0) *u_out = ut;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS)
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 2 : 1)
 k_fft_z_green(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restrict__ spec,
               const T *__restrict__ green, cplx<T> *__restrict__ ek, long long nspec,
               double *__restrict__ u_part, const cplx<T> *__restrict__ twg, int nitems)
@@ -625,7 +680,7 @@ k_fft_z_green(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restri
         const int r = find_rep(item, nrep, [&](int k) { return reps[k].wc_off; });
         const RepDev &R = reps[r];
         const int w = item - R.wc_off;
-        cplx<T> *buf = tw + 128;
+        cplx<T> *buf = tw + TWIDDLE_N;
         double *u_out = u_part + item;
         switch (R.logM) {  // block-uniform: one replica per item
         case 5: z_green_item<T, 5>(R, w, spec, green, ek, nspec, u_out, buf, tw, red); break;
@@ -637,96 +692,188 @@ k_fft_z_green(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restri
 }
 
 // Passes B-D fused for meshes whose kx planes fit in shared memory
-// (M <= PLANE_MAX): one CTA per (replica, kx) loads the plane rho_k(kx,z,y),
-// transforms it along y and z, forms the U_f partial and phi = (G/V) rho_k,
-// and transforms back: E_z = IFFT_y IFFT_z(-i kz phi), E_y = IFFT_y(-i ky
-// IFFT_z(phi)), E_x = -i kx IFFT_y IFFT_z(phi) -- seven line-FFT sweeps in
-// shared memory, one plane read and three plane writes. The plane is stored
-// [z][y] with a padded row (M+1); radix-2 DIT needs bit-reversed input, so the
-// load and the multiplies write bit-reversed positions.
+// (M <= PLANE_MAX): one CTA per (replica, kx) transforms the plane rho_k(kx,z,y)
+// along y and z, forms the U_f partial and phi = (G/V) rho_k, and transforms
+// back: E_z = IFFT_y IFFT_z(-i kz phi), E_y = IFFT_y(-i ky IFFT_z(phi)), E_x =
+// -i kx IFFT_y IFFT_z(phi). One plane read and three plane writes; in between
+// the plane goes through shared memory nine times, in eight phases, every pass
+// in place (a thread writes the slots it read): after the forward y transform
+// column s holds ky = s / RB + RA (s mod RB), which the inverse y transform,
+// with the split swapped, takes as it is. The multiplications happen in
+// registers between passes. Rows are M + 1 apart: lanes along z or along a row
+// fall on different banks; where lanes go along y to meet global memory, the
+// rows of a half warp are plane_row()'s, spaced to do the same.
 constexpr int PLANE_MAX = 64;
 
-template <typename T, int LOGM>
+__device__ __forceinline__ int plane_row(int g) { return ((g & 1) << 3) | ((g >> 1) & 7) | (g & ~15); }
+
+template <typename T, int LOGM, int NT>
 __device__ __forceinline__ void plane_item(const RepDev &R, int kx, const cplx<T> *__restrict__ spec,
                                            const T *__restrict__ green, cplx<T> *__restrict__ ek,
                                            long long nspec, double *__restrict__ u_out,
-                                           cplx<T> *A, cplx<T> *B, const cplx<T> *tw,
+                                           cplx<T> *A, cplx<T> *B, const cplx<T> *twt,
                                            double *red)
 {
-    constexpr int M = 1 << LOGM, LD = M + 1, MM = M * M;
+    constexpr int M = 1 << LOGM, RA = Split<LOGM>::RA, RB = Split<LOGM>::RB, LD = M + 1;
+    const cplx<T> *tw = twt + M - 32;
     const long long lbase = R.spec_off + (long long)kx * M * M;
     __syncthreads();
-    for (int e = threadIdx.x; e < MM; e += FFT_THREADS) {
-        const int z = e >> LOGM, y = e & (M - 1);
-        A[brev(z, LOGM) * LD + brev(y, LOGM)] = spec[lbase + e];
-    }
-    // this thread's influence-function values, in flight during the sweeps
-    constexpr int GPT = (MM + FFT_THREADS - 1) / FFT_THREADS;
-    T gr[GPT];
+    // y, pass 1
+    for (int e = threadIdx.x; e < M * RB; e += NT) {
+        const int n2 = e % RB, z = plane_row(e / RB);
+        cplx<T> x[RA];
 #pragma unroll
-    for (int i = 0; i < GPT; ++i) {
-        const int e = threadIdx.x + i * FFT_THREADS;
-        gr[i] = e < MM ? __ldg(green + lbase + e) : (T)0;
+        for (int n1 = 0; n1 < RA; ++n1) x[n1] = spec[lbase + z * M + RB * n1 + n2];
+        dft<T, RA, false>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            A[z * LD + k1 * RB + n2] = k1 ? cmul<T>(x[k1], tw[k1 * RB + n2]) : x[0];
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(A, LD, 1, LOGM, tw, false);  // along y
-    fft_lines_t<T, LOGM>(A, 1, LD, LOGM, tw, false);  // along z
+    // y, pass 2: column k1 RB + k2 = ky k1 + RA k2
+    for (int e = threadIdx.x; e < M * RA; e += NT) {
+        const int z = e % M, k1 = e / M;
+        cplx<T> x[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = A[z * LD + k1 * RB + n2];
+        dft<T, RB, false>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) A[z * LD + k1 * RB + k2] = x[k2];
+    }
+    __syncthreads();
+    // z, pass 1
+    for (int e = threadIdx.x; e < M * RB; e += NT) {
+        const int s = e % M, n2 = e / M;
+        cplx<T> x[RA];
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) x[n1] = A[(RB * n1 + n2) * LD + s];
+        dft<T, RA, false>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            A[(RB * k1 + n2) * LD + s] = k1 ? cmul<T>(x[k1], tw[k1 * RB + n2]) : x[0];
+    }
+    __syncthreads();
+    // z, pass 2; U_f, phi, -i kz phi; their inverse z transforms, pass 1
     const double wkx = (kx == 0 || kx == (M >> 1)) ? 1.0 : 2.0;
-    double u = 0.0;
-#pragma unroll
-    for (int i = 0; i < GPT; ++i) {
-        const int e = threadIdx.x + i * FFT_THREADS;
-        if (e >= MM) break;
-        const int z = e >> LOGM, y = e & (M - 1);
-        const cplx<T> rk = A[z * LD + y];
-        const T g = gr[i];
-        u += wkx * (double)g * ((double)rk.x * rk.x + (double)rk.y * rk.y);
-        B[brev(z, LOGM) * LD + brev(y, LOGM)] = make_c<T>(g * rk.x, g * rk.y);
-    }
-    __syncthreads();
     const T twopi_L = (T)(6.283185307179586477 * R.inv_L);
-    for (int e = threadIdx.x; e < MM; e += FFT_THREADS) {
-        const int zb = e >> LOGM, yb = e & (M - 1);
-        const int z = brev(zb, LOGM);
-        const T kz = (z == (M >> 1)) ? (T)0 : twopi_L * (T)freq(z, M);
-        const cplx<T> ph = B[zb * LD + yb];
-        A[zb * LD + yb] = make_c<T>(kz * ph.y, -kz * ph.x);  // -i kz phi
+    double u = 0.0;
+    for (int e = threadIdx.x; e < M * RA; e += NT) {
+        const int s = e % M, k1 = e / M, y = s / RB + RA * (s % RB);
+        T g[RB];
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) g[k2] = __ldg(green + lbase + (k1 + RA * k2) * M + y);
+        cplx<T> x[RB], f[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = A[(k1 * RB + n2) * LD + s];
+        dft<T, RB, false>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) {
+            const int n = k1 + RA * k2;
+            u += wkx * (double)g[k2] * ((double)x[k2].x * x[k2].x + (double)x[k2].y * x[k2].y);
+            x[k2] = make_c<T>(g[k2] * x[k2].x, g[k2] * x[k2].y);
+            const T kz = (n == (M >> 1)) ? (T)0 : twopi_L * (T)freq(n, M);
+            f[k2] = make_c<T>(kz * x[k2].y, -kz * x[k2].x);  // -i kz phi
+        }
+        dft<T, RB, true>(x);
+        dft<T, RB, true>(f);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            const cplx<T> wj = tw[k1 * RB + j];
+            A[(k1 * RB + j) * LD + s] = ctw<T, true>(f[j], wj);
+            B[(k1 * RB + j) * LD + s] = ctw<T, true>(x[j], wj);
+        }
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(A, 1, LD, LOGM, tw, true);  // z, of -i kz phi
-    fft_lines_t<T, LOGM>(B, 1, LD, LOGM, tw, true);  // z, of phi: psi
-    fft_lines_t<T, LOGM>(A, LD, 1, LOGM, tw, true);  // y: E_z
-    cplx<T> *Ez = ek + 2 * nspec + lbase;
-    for (int e = threadIdx.x; e < MM; e += FFT_THREADS) {
-        const int z = e >> LOGM, y = e & (M - 1);
-        Ez[e] = A[z * LD + y];
+    // inverse z, pass 2: rows in natural z
+    for (int e = threadIdx.x; e < M * RB; e += NT) {
+        const int s = e % M, j = e / M;
+        cplx<T> x[RA];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = A[(k1 * RB + j) * LD + s];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) A[(i * RB + j) * LD + s] = x[i];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = B[(k1 * RB + j) * LD + s];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) B[(i * RB + j) * LD + s] = x[i];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < MM; e += FFT_THREADS) {
-        const int z = e >> LOGM, yb = e & (M - 1);
-        const int y = brev(yb, LOGM);
-        const T ky = (y == (M >> 1)) ? (T)0 : twopi_L * (T)freq(y, M);
-        const cplx<T> ps = B[z * LD + yb];
-        A[z * LD + yb] = make_c<T>(ky * ps.y, -ky * ps.x);  // -i ky psi
+    // inverse y, pass 1, of E_z (A) and psi (B); that of -i ky psi waits in
+    // registers for A
+    constexpr int TPT = (M * RA + NT - 1) / NT;
+    cplx<T> h[TPT][RB];
+#pragma unroll
+    for (int q = 0; q < TPT; ++q) {
+        const int e = threadIdx.x + q * NT;
+        if (TPT * NT != M * RA && e >= M * RA) break;
+        const int z = e % M, k1 = e / M;
+        cplx<T> x[RB];
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) x[k2] = A[z * LD + k1 * RB + k2];
+        dft<T, RB, true>(x);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) A[z * LD + k1 * RB + j] = ctw<T, true>(x[j], tw[k1 * RB + j]);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) {
+            const int y = k1 + RA * k2;
+            x[k2] = B[z * LD + k1 * RB + k2];
+            const T ky = (y == (M >> 1)) ? (T)0 : twopi_L * (T)freq(y, M);
+            h[q][k2] = make_c<T>(ky * x[k2].y, -ky * x[k2].x);  // -i ky psi
+        }
+        dft<T, RB, true>(x);
+        dft<T, RB, true>(h[q]);
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            const cplx<T> wj = tw[k1 * RB + j];
+            B[z * LD + k1 * RB + j] = ctw<T, true>(x[j], wj);
+            h[q][j] = ctw<T, true>(h[q][j], wj);
+        }
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(A, LD, 1, LOGM, tw, true);  // y: E_y
-    fft_lines_t<T, LOGM>(B, LD, 1, LOGM, tw, true);  // y: IFFT(psi)
+    // inverse y, pass 2, to global memory: E_z and E_x, then E_y
     const T kxv = (kx == (M >> 1)) ? (T)0 : twopi_L * (T)kx;
-    cplx<T> *Ey = ek + nspec + lbase;
-    cplx<T> *Ex = ek + lbase;
-    for (int e = threadIdx.x; e < MM; e += FFT_THREADS) {
-        const int z = e >> LOGM, y = e & (M - 1);
-        Ey[e] = A[z * LD + y];
-        const cplx<T> ps = B[z * LD + y];
-        Ex[e] = make_c<T>(kxv * ps.y, -kxv * ps.x);
+    for (int e = threadIdx.x; e < M * RB; e += NT) {
+        const int j = e % RB, z = plane_row(e / RB);
+        cplx<T> x[RA];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = A[z * LD + k1 * RB + j];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) ek[2 * nspec + lbase + z * M + j + RB * i] = x[i];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = B[z * LD + k1 * RB + j];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i)
+            ek[lbase + z * M + j + RB * i] = make_c<T>(kxv * x[i].y, -kxv * x[i].x);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < TPT; ++q) {
+        const int e = threadIdx.x + q * NT;
+        if (TPT * NT != M * RA && e >= M * RA) break;
+        const int z = e % M, k1 = e / M;
+#pragma unroll
+        for (int j = 0; j < RB; ++j) A[z * LD + k1 * RB + j] = h[q][j];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < M * RB; e += NT) {
+        const int j = e % RB, z = plane_row(e / RB);
+        cplx<T> x[RA];
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1) x[k1] = A[z * LD + k1 * RB + j];
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int i = 0; i < RA; ++i) ek[nspec + lbase + z * M + j + RB * i] = x[i];
     }
     const double ut = block_sum(u, red);
     if (threadIdx.x == 0) *u_out = ut;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS)
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 3 : 1)
 k_fft_plane(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restrict__ spec,
             const T *__restrict__ green, cplx<T> *__restrict__ ek, long long nspec,
             double *__restrict__ u_part, const cplx<T> *__restrict__ twg, int nitems)
@@ -739,27 +886,12 @@ k_fft_plane(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restrict
         const int r = find_rep(item, nrep, [&](int k) { return reps[k].wp_off; });
         const RepDev &R = reps[r];
         const int kx = item - R.wp_off;
-        cplx<T> *A = tw + 128;
+        cplx<T> *A = tw + TWIDDLE_N;
         cplx<T> *B = A + R.M * (R.M + 1);
         if (R.logM == 5)
-            plane_item<T, 5>(R, kx, spec, green, ek, nspec, u_part + item, A, B, tw, red);
+            plane_item<T, 5, NT>(R, kx, spec, green, ek, nspec, u_part + item, A, B, tw, red);
         else
-            plane_item<T, 6>(R, kx, spec, green, ek, nspec, u_part + item, A, B, tw, red);
-    }
-}
-
-// Two adjacent spectrum rows a, b of line l, wavenumber k, packed into the
-// complex line of an inverse transform whose real and imaginary parts come
-// out as the two real rows (k and M - k from Hermitian symmetry).
-template <typename T, int LOGM>
-__device__ __forceinline__ void c2r_split(cplx<T> *buf, int k, int l, cplx<T> a, cplx<T> b)
-{
-    constexpr int M = 1 << LOGM;
-    if (k == 0 || k == (M >> 1)) {
-        buf[brev(k, LOGM) * LSX + l] = make_c<T>(a.x, b.x);
-    } else {
-        buf[brev(k, LOGM) * LSX + l] = make_c<T>(a.x - b.y, a.y + b.x);
-        buf[brev(M - k, LOGM) * LSX + l] = make_c<T>(a.x + b.y, b.x - a.y);
+            plane_item<T, 6, NT>(R, kx, spec, green, ek, nspec, u_part + item, A, B, tw, red);
     }
 }
 
@@ -767,54 +899,74 @@ __device__ __forceinline__ void c2r_split(cplx<T> *buf, int k, int l, cplx<T> a,
 // efield[c][z][y][x]. Item = (replica, component, z, tile of 2 x_lines rows); rows
 // 2l and 2l+1 share complex line l: Z[k] = Xa[k] + i Xb[k] over the
 // Hermitian extension, with the imaginary parts at k = 0 and M/2 dropped.
-// Instantiated per mesh side like pass A.
+// Instantiated per mesh side like pass A. Pass 1 takes its elements straight
+// from the spectra (k and M - k from the same one: its second read hits L1),
+// pass 2 writes the meshes.
 template <typename T, int LOGM>
 __device__ __forceinline__ void x_c2r_item(const RepDev &R, int comp, int w,
                                            const cplx<T> *__restrict__ ek, long long nspec,
                                            T *__restrict__ efield, long long nmesh, cplx<T> *buf,
-                                           const cplx<T> *tw)
+                                           const cplx<T> *twt)
 {
-    constexpr int M = 1 << LOGM;
-    constexpr int LNL = x_lines_log(LOGM), NROW = 2 << LNL;  // complex lines, real rows
-    constexpr int NYT = M >> (LNL + 1), NK = (M >> 1) + 1;
+    constexpr int M = 1 << LOGM, RA = Split<LOGM>::RA, RB = Split<LOGM>::RB;
+    constexpr int LNL = x_lines_log(LOGM), NL = 1 << LNL, NROW = 2 << LNL;  // complex lines, real rows
+    constexpr int NYT = M >> (LNL + 1);
+    // 16 lanes: RA values of k1 on 16 / RA lines
+    constexpr int LS = NL + 16 / RA;
+    const cplx<T> *tw = twt + M - 32;
     const int z = w / NYT, y0 = (w % NYT) * NROW;
     const cplx<T> *src = ek + comp * nspec + R.spec_off + (long long)z * M + y0;
     __syncthreads();
-    if constexpr (sizeof(T) == 4) {
-        for (int e = threadIdx.x; e < (NK << LNL); e += FFT_THREADS) {
-            const int l = e & ((1 << LNL) - 1), k = e >> LNL;
-            const long long o = (long long)k * M * M + 2 * l;
-            // o is even: one 16-byte load
-            const float4 ab = __ldg(reinterpret_cast<const float4 *>(src + o));
-            const cplx<T> a = make_c<T>(ab.x, ab.y), b = make_c<T>(ab.z, ab.w);
-            c2r_split<T, LOGM>(buf, k, l, a, b);
+    for (int e = threadIdx.x; e < NL * RB; e += FFT_THREADS) {
+        const int l = e % NL, n2 = e / NL;
+        cplx<T> x[RA];
+#pragma unroll
+        for (int n1 = 0; n1 < RA; ++n1) {
+            const int k = RB * n1 + n2, kk = k <= (M >> 1) ? k : M - k;
+            const long long o = (long long)kk * M * M + 2 * l;
+            cplx<T> a, b;
+            if constexpr (sizeof(T) == 4) {  // o is even: one 16-byte load
+                const float4 ab = *reinterpret_cast<const float4 *>(src + o);
+                a = make_c<T>(ab.x, ab.y);
+                b = make_c<T>(ab.z, ab.w);
+            } else {
+                a = src[o];
+                b = src[o + 1];
+            }
+            if (k == 0 || k == (M >> 1)) x[n1] = make_c<T>(a.x, b.x);
+            else if (k < (M >> 1)) x[n1] = make_c<T>(a.x - b.y, a.y + b.x);
+            else x[n1] = make_c<T>(a.x + b.y, b.x - a.y);
         }
-    } else {
-        for (int e = threadIdx.x; e < (NK << LNL); e += FFT_THREADS) {
-            const int l = e & ((1 << LNL) - 1), k = e >> LNL;
-            const long long o = (long long)k * M * M + 2 * l;
-            c2r_split<T, LOGM>(buf, k, l, src[o], src[o + 1]);
-        }
+        dft<T, RA, true>(x);
+#pragma unroll
+        for (int k1 = 0; k1 < RA; ++k1)
+            buf[(n2 * RA + k1) * LS + l] = k1 ? ctw<T, true>(x[k1], tw[k1 * RB + n2]) : x[0];
     }
     __syncthreads();
-    fft_lines_t<T, LOGM>(buf, 1, LSX, LNL, tw, true);
     T *dst = efield + comp * nmesh + R.mesh_off + ((long long)z * M + y0) * M;
-    for (int e = threadIdx.x; e < NROW * M; e += FFT_THREADS) {
-        const int x = e & (M - 1), j = e >> LOGM;
-        const cplx<T> v = buf[x * LSX + (j >> 1)];
-        dst[j * M + x] = (j & 1) ? v.y : v.x;
+    for (int e = threadIdx.x; e < NL * RA; e += FFT_THREADS) {
+        const int k1 = e % RA, l = e / RA;
+        cplx<T> x[RB];
+#pragma unroll
+        for (int n2 = 0; n2 < RB; ++n2) x[n2] = buf[(n2 * RA + k1) * LS + l];
+        dft<T, RB, true>(x);
+#pragma unroll
+        for (int k2 = 0; k2 < RB; ++k2) {
+            dst[2 * l * M + k1 + RA * k2] = x[k2].x;
+            dst[(2 * l + 1) * M + k1 + RA * k2] = x[k2].y;
+        }
     }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS)
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 4 : 2)
 k_fft_x_c2r(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restrict__ ek,
             long long nspec, T *__restrict__ efield, long long nmesh,
             const cplx<T> *__restrict__ twg, int nitems_per_comp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cplx<T> *tw = reinterpret_cast<cplx<T> *>(smem_raw);
-    cplx<T> *buf = tw + 128;
+    cplx<T> *buf = tw + TWIDDLE_N;
     load_twiddles<T>(tw, twg);
     for (int item = blockIdx.x; item < nitems_per_comp * 3; item += gridDim.x) {
         const int comp = item / nitems_per_comp, it = item % nitems_per_comp;
@@ -1085,20 +1237,31 @@ __global__ void k_efield_from_mesh(const RepDev *__restrict__ reps, int rep,
 // launchers
 // ---------------------------------------------------------------------------
 
-template <typename T> static size_t fft_smem(int maxM, int nbuf)
+// shared memory of the passes for meshes up to maxM: the twiddles and the
+// largest exchange buffer of the sides up to maxM
+template <typename T> static size_t y_smem(int maxM)
 {
-    return (128 + (size_t)nbuf * maxM * LS) * sizeof(cplx<T>);
+    const int n = maxM >= 128 ? (32 * y_stride<7>() > 16 * y_stride<8>() ? 32 * y_stride<7>() : 16 * y_stride<8>())
+                              : 32 * y_stride<6>();
+    return (size_t)(TWIDDLE_N + n) * sizeof(cplx<T>);
 }
+
+template <typename T> static size_t z_smem(int maxM)
+{
+    return (size_t)(TWIDDLE_N + 2 * (maxM >= 128 ? 256 << pencil_log(8) : 64 << pencil_log(6))) * sizeof(cplx<T>);
+}
+static_assert((128 << pencil_log(7)) <= (256 << pencil_log(8)), "z exchange at 128");
 
 template <typename T> static size_t plane_smem(int M)
 {
-    return (128 + 2 * (size_t)M * (M + 1)) * sizeof(cplx<T>);
+    return (TWIDDLE_N + 2 * (size_t)M * (M + 1)) * sizeof(cplx<T>);
 }
 
 template <typename T> static size_t x_smem(int maxM)
 {
-    return (128 + (size_t)maxM * LSX) * sizeof(cplx<T>);
+    return (size_t)(TWIDDLE_N + (maxM >= 128 ? 256 * x_stride<8>() : 64 * x_stride<6>())) * sizeof(cplx<T>);
 }
+static_assert(128 * x_stride<7>() <= 256 * x_stride<8>(), "x exchange at 128");
 
 template <typename K> static void set_smem(K kernel, size_t bytes)
 {
@@ -1112,13 +1275,15 @@ template <typename T> void configure_mesh_kernels()
     set_smem(k_assign<T, false>, assign_smem(1));
     set_smem(k_assign<T, true>, assign_smem(1));
     set_smem(k_fft_x_r2c<T>, x_smem<T>(256));
-    set_smem(k_fft_y<T>, fft_smem<T>(256, 1));
-    set_smem(k_fft_z_green<T>, fft_smem<T>(256, 2));
+    set_smem(k_fft_y<T, false>, y_smem<T>(256));
+    set_smem(k_fft_y<T, true>, y_smem<T>(256));
+    set_smem(k_fft_z_green<T>, z_smem<T>(256));
     set_smem(k_fft_x_c2r<T>, x_smem<T>(256));
     set_smem(k_gather<T, 1, 3>, GTILE * sizeof(T));
     set_smem(k_gather<T, 1, 1>, GTILE * sizeof(T));
     if constexpr (sizeof(T) == 4) set_smem(k_gather<T, 2, 3>, 2 * GTILE * sizeof(T));
-    set_smem(k_fft_plane<T>, plane_smem<T>(PLANE_MAX));
+    if constexpr (sizeof(T) == 4) set_smem(k_fft_plane<T, 256>, plane_smem<T>(PLANE_MAX));
+    set_smem(k_fft_plane<T, 512>, plane_smem<T>(PLANE_MAX));
 }
 
 // CTAs per brick of the assignment: two for up to 32 bricks (FP32, one
@@ -1147,20 +1312,31 @@ template <typename T> void launch_fft_forward(const DevState &s, cudaStream_t st
 {
     using C = cplx<T>;
     const int maxM = s.max_mesh;
-    const size_t sm1 = fft_smem<T>(maxM, 1), sm2 = fft_smem<T>(maxM, 2);
     k_fft_x_r2c<T><<<grid_items(s.wa), FFT_THREADS, x_smem<T>(maxM), st>>>(s.reps, s.nrep, (const T *)s.tiles,
                                                                 (C *)s.spec, (const C *)s.twiddle, s.wa);
     if (s.wb > 0) {
-        k_fft_y<T><<<grid_items(s.wb), FFT_THREADS, sm1, st>>>(s.reps, s.nrep, (C *)s.spec, s.nspec,
-                                                                1, (const C *)s.twiddle, s.wb, false);
-        k_fft_z_green<T><<<grid_items(s.wc), FFT_THREADS, sm2, st>>>(
+        k_fft_y<T, false><<<grid_items(s.wb), FFT_THREADS, y_smem<T>(maxM), st>>>(
+            s.reps, s.nrep, (C *)s.spec, s.nspec, 1, (const C *)s.twiddle, s.wb);
+        k_fft_z_green<T><<<grid_items(s.wc), FFT_THREADS, z_smem<T>(maxM), st>>>(
             s.reps, s.nrep, (const C *)s.spec, (const T *)s.green, (C *)s.ek, s.nspec, s.u_pm_part,
             (const C *)s.twiddle, s.wc);
     }
     if (s.wp > 0) {
-        k_fft_plane<T><<<grid_items(s.wp), FFT_THREADS, plane_smem<T>(s.max_plane), st>>>(
-            s.reps, s.nrep, (const C *)s.spec, (const T *)s.green, (C *)s.ek, s.nspec,
-            s.u_pm_part + s.wc, (const C *)s.twiddle, s.wp);
+        // 512 threads a plane where every plane has an SM (FP32 64^3, 512 / 256
+        // threads: 33 planes 8.9 / 9.9 us, 132 planes 9.4 / 10.5), and in FP64,
+        // whose two planes take an SM's shared memory; 256 where planes share
+        // SMs, three CTAs each (264 planes 18.0 / 15.4 us, 660 45.2 / 32.9)
+        auto go = [&](auto kern, int nt) {
+            kern<<<grid_items(s.wp), nt, plane_smem<T>(s.max_plane), st>>>(
+                s.reps, s.nrep, (const C *)s.spec, (const T *)s.green, (C *)s.ek, s.nspec,
+                s.u_pm_part + s.wc, (const C *)s.twiddle, s.wp);
+        };
+        if constexpr (sizeof(T) == 4) {
+            if (s.wp > 148) go(k_fft_plane<T, 256>, 256);
+            else go(k_fft_plane<T, 512>, 512);
+        } else {
+            go(k_fft_plane<T, 512>, 512);
+        }
     }
 }
 
@@ -1170,10 +1346,9 @@ int plane_max_mesh() { return PLANE_MAX; }  // the largest side the plane kernel
 template <typename T> void launch_fft_inverse(const DevState &s, cudaStream_t st)
 {
     using C = cplx<T>;
-    const size_t sm1 = fft_smem<T>(s.max_mesh, 1);
     if (s.wb > 0)
-        k_fft_y<T><<<grid_items(3 * s.wb), FFT_THREADS, sm1, st>>>(s.reps, s.nrep, (C *)s.ek, s.nspec,
-                                                                    3, (const C *)s.twiddle, s.wb, true);
+        k_fft_y<T, true><<<grid_items(3 * s.wb), FFT_THREADS, y_smem<T>(s.max_mesh), st>>>(
+            s.reps, s.nrep, (C *)s.ek, s.nspec, 3, (const C *)s.twiddle, s.wb);
     k_fft_x_c2r<T><<<grid_items(3 * s.wa), FFT_THREADS, x_smem<T>(s.max_mesh), st>>>(
         s.reps, s.nrep, (const C *)s.ek, s.nspec, (T *)s.efield, s.nmesh, (const C *)s.twiddle,
         s.wa);
