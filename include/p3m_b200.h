@@ -104,7 +104,7 @@ int p3m_gf_opt(int device, double kappa, double alpha, int p, int m_alias, int M
  * passes device pointers for the outputs -- G_k_dev (M*M*M doubles,
  * fftshifted layout) and A_pm_dev (one double) -- and the stream to launch
  * on; the call returns without waiting. The only scratch (one FP64 partial
- * per 256-point block) lives in a fixed file-scope device array of 8192
+ * per block) lives in a fixed file-scope device array of 8192
  * doubles (64 KiB, held on every GPU that loads the library until exit), so
  * M is limited to 128; larger M is rejected with P3M_EARG. The call
  * allocates nothing. Every call made outside stream capture looks up that

@@ -1,15 +1,15 @@
 // p3m_gf_opt_static: the FP64 optimal influence function for callers that
 // cannot allocate device memory.
 //
-// p3m_gf_opt allocates its output and its per-block partial sums with
-// cudaMalloc on every call. Some callers cannot do that: code that owns a
+// p3m_gf_opt allocates its output and its per-block partial sums from the
+// device's memory pool on every call. Some callers cannot do that: code that owns a
 // fixed device-memory budget and hands out every byte itself through its own
 // pool or arena (an allocation behind its back can push a full GPU over the
 // edge), or long-running services that must not allocate after start-up
 // (cudaMalloc can block on the device and fragments memory over time). This
 // entry point takes
 // the output buffers from the caller and keeps its only scratch -- one FP64
-// partial sum per 256-point block -- in the file-scope array below, which
+// partial sum per block -- in the file-scope array below, which
 // every GPU that loads the library holds until the process exits
 // (kMaxBlocks doubles, 64 KiB).
 //
@@ -26,7 +26,7 @@
 namespace {
 
 constexpr int kMaxMesh = 128;                                         // M <= 128
-constexpr int kMaxBlocks = kMaxMesh * kMaxMesh * kMaxMesh / 256;      // 8192 partials
+constexpr int kMaxBlocks = kMaxMesh * kMaxMesh * kMaxMesh / 256;      // 8192 partials (1498 used at 128^3)
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) double g_gf_scratch[kMaxBlocks];
