@@ -56,6 +56,8 @@ struct p3m_ctx {
     // kGraphSteps steps per graph (launched for whole groups of steps)
     cudaGraphExec_t graphK[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     long long graph_kernels[2][2] = {{0, 0}, {0, 0}};  // kernels per step of the captured graphs
+    cudaGraphExec_t graph_force = nullptr;             // one force evaluation (p3m_force)
+    long long graph_force_kernels = 0;
     int ncell_cap = 0;            // cells allocated (grid with skin 0)
     long long nlist_cap = 0;      // list entries allocated
     long long nlist_in_cap = 0;   // inner-list entries allocated
@@ -76,6 +78,7 @@ static int graph_steps(const p3m_ctx *ctx) { return ctx->prec == P3M_FP32 ? kGra
 // Drop the captured step graphs (all, or only those recording n(q,t)).
 static void drop_graphs(p3m_ctx *ctx, bool rec_only = false)
 {
+    if (!rec_only && ctx->graph_force) { cudaGraphExecDestroy(ctx->graph_force); ctx->graph_force = nullptr; }
     for (int a = 0; a < 2; ++a)
         for (int b = rec_only ? 1 : 0; b < 2; ++b) {
             if (ctx->graph[a][b]) { cudaGraphExecDestroy(ctx->graph[a][b]); ctx->graph[a][b] = nullptr; }
@@ -736,17 +739,63 @@ template <typename T> static int ensure_green(p3m_ctx *ctx)
     return P3M_OK;
 }
 
-// One full force evaluation of the current device positions: sort (with or
-// without the key pass), PP, PM. Leaves acc_pp / acc_pm and U parts.
-template <typename T> static int seq_force(p3m_ctx *ctx, bool keys)
+// One full force evaluation of the current device positions: keys, then the
+// particle branch (cell sort, lists, PP) and beside it on a second stream the
+// mesh branch (brick sort, PM), as in a step. Leaves acc_pp / acc_pm and U parts.
+// The influence functions exist (ensure_green).
+template <typename T> static int seq_force(p3m_ctx *ctx)
 {
-    if (ctx->s.has_mesh) {
-        int rc = ensure_green<T>(ctx);
-        if (rc != P3M_OK) return rc;
+    DevState &s = ctx->s;
+    cudaStream_t st = ctx->st, st2 = ctx->st2;
+    launch_set_flags(s.rebuild, s.nrep, 1, st);
+    launch_keys<T>(s, st);
+    ctx->launches += 2;
+    cudaError_t e = cudaSuccess;
+    if (s.has_mesh) {
+        e = cudaEventRecord(ctx->ev_fork, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
+        if (e == cudaSuccess) {
+            launch_scan_bricks(s, st2);
+            launch_place_bricks<T>(s, st2);
+            ctx->launches += 2;
+            seq_pm<T>(ctx, true, st2);
+            e = cudaEventRecord(ctx->ev_join, st2);
+        }
     }
-    seq_sort<T>(ctx, keys);
-    seq_pp<T>(ctx);
-    if (ctx->s.has_mesh) seq_pm<T>(ctx);
+    launch_scan_cells(s, st);
+    launch_scatter(s, st);
+    launch_fix_cells<T>(s, st);
+    launch_build_lists<T>(s, st);
+    ctx->launches += 4;
+    seq_pp<T>(ctx, true, st);
+    if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
+    if (e != cudaSuccess) return fail(ctx, P3M_ECUDA, "force fork/join", cudaGetErrorString(e));
+    launch_kick_finish<T>(s, 0, nullptr, st);
+    launch_step_reduce(s, 2, ctx->counters, nullptr, 0, st);
+    ctx->launches += 2;
+    return P3M_OK;
+}
+
+// Capture what `seq` enqueues on the context's stream into *out; *kernels
+// receives the number of kernels.
+template <typename F>
+static int capture_graph(p3m_ctx *ctx, cudaGraphExec_t *out, long long *kernels, F seq)
+{
+    cudaGraph_t g;
+    const long long before = ctx->launches;
+    CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
+    const int rc = seq();
+    cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
+    *kernels = ctx->launches - before;
+    ctx->launches = before;
+    if (rc != P3M_OK) {
+        if (e == cudaSuccess) cudaGraphDestroy(g);
+        return rc;
+    }
+    if (e != cudaSuccess) return fail(ctx, P3M_ECUDA, "cudaStreamEndCapture", cudaGetErrorString(e));
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) return fail(ctx, P3M_ECUDA, "cudaGraphInstantiate", cudaGetErrorString(e));
     return P3M_OK;
 }
 
@@ -1088,12 +1137,13 @@ static int do_force(p3m_ctx *ctx, const double *pos, const double *Z, double *ac
                     double *parts)
 {
     DevState &s = ctx->s;
+    if (s.has_mesh) RET(ensure_green<T>(ctx));
+    if (!ctx->graph_force)  // one launch per call instead of twenty
+        RET(capture_graph(ctx, &ctx->graph_force, &ctx->graph_force_kernels, [&] { return seq_force<T>(ctx); }));
     RET(h2d(ctx, s.pos, pos, sizeof(double) * 3 * s.ntot));
     RET(upload_charge(ctx, Z));
-    RET(seq_force<T>(ctx, true));
-    launch_kick_finish<T>(s, 0, nullptr, ctx->st);
-    launch_step_reduce(s, 2, ctx->counters, nullptr, 0, ctx->st);
-    ctx->launches += 2;
+    CK(cudaGraphLaunch(ctx->graph_force, ctx->st));
+    ctx->launches += ctx->graph_force_kernels;
     RET(d2h(ctx, acc, s.acc, sizeof(double) * 3 * s.ntot));
     double ro[8];
     RET(d2h(ctx, ro, s.rep_out, sizeof ro));
@@ -1121,14 +1171,18 @@ static int do_update(p3m_ctx *ctx, int mode, int it, double *pos, double *vel, d
 {
     DevState &s = ctx->s;
     const size_t b = sizeof(double) * 3 * s.ntot;
+    if (s.has_mesh) RET(ensure_green<T>(ctx));
+    if (!ctx->graph[mode][0])
+        RET(capture_graph(ctx, &ctx->graph[mode][0], &ctx->graph_kernels[mode][0],
+                          [&] { return seq_step<T>(ctx, mode, 0); }));
     RET(h2d(ctx, s.pos, pos, b));
     RET(h2d(ctx, s.vel, vel, b));
     RET(h2d(ctx, s.acc, acc, b));
-    if (s.has_mesh) RET(ensure_green<T>(ctx));
     launch_set_counters(ctx->counters, 0, -1, it, ctx->st);
     launch_set_flags(s.rebuild, s.nrep, 1, ctx->st);  // the caller's arrays may hold any state
     ctx->launches += 2;
-    RET(seq_step<T>(ctx, mode, 0));
+    CK(cudaGraphLaunch(ctx->graph[mode][0], ctx->st));  // the graph of one p3m_run step
+    ctx->launches += ctx->graph_kernels[mode][0];
     RET(d2h(ctx, pos, s.pos, b));
     RET(d2h(ctx, vel, s.vel, b));
     RET(d2h(ctx, acc, s.acc, b));
@@ -1298,10 +1352,8 @@ extern "C" int p3m_get_step_async(p3m_ctx *ctx, double *pos, double *vel, double
 
 template <typename T> static int do_init_forces(p3m_ctx *ctx)
 {
-    RET(seq_force<T>(ctx, true));
-    launch_kick_finish<T>(ctx->s, 0, nullptr, ctx->st);
-    launch_step_reduce(ctx->s, 2, ctx->counters, nullptr, 0, ctx->st);
-    ctx->launches += 2;
+    if (ctx->s.has_mesh) RET(ensure_green<T>(ctx));
+    RET(seq_force<T>(ctx));
     return finish(ctx);
 }
 
@@ -1351,23 +1403,13 @@ template <typename T> static int do_run(p3m_ctx *ctx, int n_steps, int mode, int
     const int gi = (mode == P3M_MODE_THERMOSTAT) ? 1 : 0, gr = rec ? 1 : 0;
     // capture `steps` steps into `*out` (the kernels of one step are counted)
     auto capture = [&](int steps, cudaGraphExec_t *out) -> int {
-        cudaGraph_t g;
-        const long long before = ctx->launches;
-        CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
-        int step_rc = P3M_OK;
-        for (int k = 0; k < steps && step_rc == P3M_OK; ++k) step_rc = seq_step<T>(ctx, mode, rec);
-        cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
-        ctx->graph_kernels[gi][gr] = (ctx->launches - before) / steps;  // kernels per step
-        ctx->launches = before;
-        if (step_rc != P3M_OK) {
-            if (e == cudaSuccess) cudaGraphDestroy(g);
+        const int rc = capture_graph(ctx, out, &ctx->graph_kernels[gi][gr], [&] {
+            int step_rc = P3M_OK;
+            for (int k = 0; k < steps && step_rc == P3M_OK; ++k) step_rc = seq_step<T>(ctx, mode, rec);
             return step_rc;
-        }
-        if (e != cudaSuccess) return fail(ctx, P3M_ECUDA, "cudaStreamEndCapture", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(out, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(ctx, P3M_ECUDA, "cudaGraphInstantiate", cudaGetErrorString(e));
-        return P3M_OK;
+        });
+        ctx->graph_kernels[gi][gr] /= steps;
+        return rc;
     };
     // both graphs on first use, so that a warm-up of any length has captured
     // them before the runs it prepares
