@@ -61,30 +61,40 @@ __device__ __forceinline__ typename Coord<T>::I qdiff(typename Coord<T>::U a, ty
 // ---------------------------------------------------------------------------
 // list build (rebuild steps only)
 // ---------------------------------------------------------------------------
-constexpr int LB_THREADS = 256;
-constexpr int LB_TPI = 16;                    // lanes per particle
-constexpr int LB_PPB = LB_THREADS / LB_TPI;   // particles per pass
+constexpr int LB_WARPS = 8;
+constexpr int LB_THREADS = 32 * LB_WARPS;
+constexpr int LB_P = 2;                       // home particles per warp and pass
+constexpr int LB_PPB = LB_WARPS * LB_P;       // home particles per pass
 constexpr int LB_HC = 256;                    // home particles per chunk
-constexpr int LB_SCAP = 1024;                 // candidates staged per window (16 KB)
-static_assert(cell_stencil(CELL_DIV_MAX) <= LB_THREADS, "one thread per stencil cell");
-static_assert(LB_TPI >= PP_LIST_PAD, "one pad entry per lane at most");
+constexpr int LB_SCAP = 1280;                 // candidates staged per window (20 KB)
+static_assert(LB_SCAP >= LB_THREADS && LB_SCAP % 32 == 0, "a round of candidates fits the window");
+static_assert(PP_LIST_PAD <= 32, "one pad entry per lane at most");
 
 // One CTA per cell of the replicas rebuilding this step (the list k_scan_cells
 // wrote); cells are (rc + skin)/D wide (about 10 particles at D = 2 and unit
 // density 3/(4 pi), 80 at D = 1). The (2D+1)^3 neighbour cells'
-// coordinates are staged in shared memory in the fixed stencil order (x
-// fastest, offsets -D .. D), a window of LB_SCAP candidates at a time, as
+// coordinates are taken in the fixed stencil order (x
+// fastest, offsets -D .. D) as
 // FP32 offsets from the home cell's centre: the wrap-around integer
 // difference, exact, then one rounding. A home particle lies within half a
 // cell of the centre and a candidate in range within rc + skin <= D cells of
 // it, so both offsets are minimum images (at most (D + 1/2) L / nc <= L/2,
-// nc >= 3 D) and their difference is the pair's separation; a test is three
-// subtractions and the squared length, against a cutoff with a 1e-5
-// relative margin over the rounding, so the list holds every pair within
-// rc + skin. The LB_TPI lanes of a particle test LB_TPI consecutive candidates per round,
-// and a warp ballot gives each candidate in range its place: the list holds
-// the in-range candidates in stencil order, as a scan by one thread would,
-// then the particle's own index up to a whole block of PP_LIST_PAD entries.
+// nc >= 3 D) and their difference is the pair's separation. Candidates farther
+// than rc + skin from the home cell's box are dropped there and then (nearly
+// half of the stencil's volume), the others staged in order in shared memory, a
+// window of LB_SCAP at a time. The 32 lanes of a warp test 32 consecutive
+// staged candidates against the warp's home particles -- three subtractions and
+// the squared length, against a cutoff with a 1e-5 relative margin over the
+// rounding, so the list holds every pair within rc + skin -- and a ballot per
+// particle gives each candidate in range its place: the list holds the in-range
+// candidates in stencil order, as a scan by one thread would, then the
+// particle's own index up to a whole block of PP_LIST_PAD entries.
+//
+// Bound: instruction issue, about evenly in staging and tests; hence the
+// search over the 25 rows of cells instead of 125 cells, and the box test.
+// Full rebuild before (16 lanes per particle, every stencil candidate tested) /
+// now: 2e3 particles 18.8 / 15.8 us, 1e4 39 / 30, 20 x 1e4 597 / 490, 1e5 278 /
+// 254, 1e6 2734 / 2650; D = 1: 20 x 1e4 750 / 560, 1e6 2414 / 2240.
 template <typename T, int D, int LT>
 __global__ void __launch_bounds__(LB_THREADS)
 k_build_lists(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ cell_start,
@@ -95,19 +105,21 @@ k_build_lists(const RepDev *__restrict__ reps, int nrep, const int *__restrict__
     constexpr int lt = LT;  // the list layout of the pair kernel's TPI = 2^LT
     using Q = typename Coord<T>::Q;
     using U = typename Coord<T>::U;
-    constexpr int SCAP = LB_SCAP;
     constexpr int CELL_SPAN = 2 * D + 1;
-    constexpr int CELL_STENCIL = cell_stencil(D);
+    constexpr int NROW = CELL_SPAN * CELL_SPAN;
+    constexpr int NSEARCH = NROW > 16 ? 5 : 4;
+    static_assert((1 << NSEARCH) > NROW, "binary search depth");
     extern __shared__ __align__(16) unsigned char lb_smem[];
     float4 *stage = reinterpret_cast<float4 *>(lb_smem);  // offsets from the centre, .w = index bits
-    __shared__ int pre[CELL_STENCIL + 1];  // candidates before stencil cell k
-    __shared__ int nstart[CELL_STENCIL];   // first sorted index of stencil cell k
-    __shared__ int wsum[LB_THREADS / 32];
+    // stencil row k (the cells of one (dy, dz), consecutive in the sorted order
+    // but for the periodic wrap): candidates before it, its first sorted index
+    // and, from offset rsplit on, what its offsets are relative to
+    __shared__ int pre[(1 << NSEARCH) + 1];
+    __shared__ int rstart[NROW], rsplit[NROW], rwrap[NROW];
+    __shared__ int wsum[2][LB_WARPS];
     __shared__ int cnt_sm[LB_HC];          // list length so far of each particle of the chunk
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int sub = tid % LB_TPI;
-    const int gshift = lane & ~(LB_TPI - 1);            // first lane of this particle's group
-    const unsigned below = (1u << (lane & (LB_TPI - 1))) - 1u;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
     const int nrb = rb_list[0];
     const int *rb_cells = rb_list + nrep_all + 1;
     for (int item = blockIdx.x; item < rb_cells[nrb]; item += gridDim.x) {
@@ -121,106 +133,144 @@ k_build_lists(const RepDev *__restrict__ reps, int nrep, const int *__restrict__
         const int cx = local % nc, cy = (local / nc) % nc, cz = local / (nc * nc);
         const float sc = (float)(R.L / Coord<T>::scale);
         const float rl2 = (float)(R.rcl * R.rcl * (1.0 + 1e-5));
+        const float hw = (float)(0.5 * R.cellw * (1.0 + 1e-5));  // half the home cell, over its rounding
         // the home cell's centre in the integer coordinates
         const U ox = Coord<T>::q(((double)cx + 0.5) / nc), oy = Coord<T>::q(((double)cy + 0.5) / nc),
                 oz = Coord<T>::q(((double)cz + 0.5) / nc);
         __syncthreads();  // the previous cell is done with pre, nstart and stage
-        // stencil cell tid: its start and count; pre = exclusive prefix sum
-        int cntc = 0;
-        if (tid < CELL_STENCIL) {
-            const int dx = tid % CELL_SPAN - D, dy = (tid / CELL_SPAN) % CELL_SPAN - D,
-                      dz = tid / (CELL_SPAN * CELL_SPAN) - D;
-            const int nx = (cx + dx + nc) % nc, ny = (cy + dy + nc) % nc, nz = (cz + dz + nc) % nc;
-            const int nb = R.cell_off + nx + nc * (ny + nc * nz);
-            nstart[tid] = cell_start[nb];
-            cntc = cell_start[nb + 1] - cell_start[nb];
-        }
-        int v = cntc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += t;
-        }
-        if (lane == 31) wsum[tid >> 5] = v;
-        __syncthreads();
-        for (int w = 0; w < (tid >> 5); ++w) v += wsum[w];
-        if (tid < CELL_STENCIL) pre[tid + 1] = v;
-        if (tid == 0) pre[0] = 0;
-        __syncthreads();
-        const int total = pre[CELL_STENCIL];
-        // home particles in chunks of LB_HC: each window of candidates is
-        // staged once per chunk, and every particle's count so far is kept
-        // in shared memory between windows
-        for (int c0 = 0; c0 < nhome; c0 += LB_HC) {
-            const int nch = min(LB_HC, nhome - c0);
-            for (int w0 = 0; w0 < total; w0 += SCAP) {
-                const int wlen = min(SCAP, total - w0);
-                __syncthreads();  // the previous window's tests (and counts) are done
-                if (w0 == 0)
-                    for (int i = tid; i < nch; i += LB_THREADS) cnt_sm[i] = 0;
-                // candidate g of the window: the stencil cell holding it by
-                // binary search over pre
-                for (int g = tid; g < wlen; g += LB_THREADS) {
-                    const int gg = w0 + g;
-                    int lo = 0, hi = CELL_STENCIL - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (pre[mid] <= gg) lo = mid; else hi = mid - 1;
-                    }
-                    const int j = nstart[lo] + gg - pre[lo];
-                    const Q q = xq[j];
-                    // the staged copy carries the sorted index
-                    stage[g] = make_float4((float)qdiff<T>(q.x, ox) * sc, (float)qdiff<T>(q.y, oy) * sc,
-                                           (float)qdiff<T>(q.z, oz) * sc, __int_as_float(j));
+        // pre = exclusive prefix sum over the rows (one warp holds them all)
+        if (tid < 32) {
+            int n = 0;
+            if (tid < NROW) {
+                const int ny = (cy + tid % CELL_SPAN - D + nc) % nc, nz = (cz + tid / CELL_SPAN - D + nc) % nc;
+                const int row = R.cell_off + nc * (ny + nc * nz);
+                const int x0 = cx - D, x1 = cx + D;  // cells x0 .. x1, nc >= 3 D: at most one wraps
+                const int lo = x0 < 0 ? x0 + nc : x0;                    // first cell
+                const int hi = x0 < 0 ? nc - 1 : min(x1, nc - 1);        // last before the wrap
+                const int a0 = cell_start[row + lo], a1 = cell_start[row + hi + 1];
+                int b0 = 0, b1 = 0;
+                if (x0 < 0 || x1 >= nc) {
+                    b0 = cell_start[row];
+                    b1 = cell_start[row + (x0 < 0 ? x1 : x1 - nc) + 1];
                 }
-                // the window's last round filled with candidates out of range
-                const int wpad = (wlen + LB_TPI - 1) & ~(LB_TPI - 1);
-                for (int g = wlen + tid; g < wpad; g += LB_THREADS)
-                    stage[g] = make_float4(1e30f, 1e30f, 1e30f, __int_as_float(-1));
-                __syncthreads();
-                for (int i0 = 0; i0 < nch; i0 += LB_PPB) {
-                    const int i = i0 + tid / LB_TPI;
-                    const bool have = i < nch;
-                    const int s = hstart + c0 + i;
-                    float xr = 0.f, yr = 0.f, zr = 0.f;  // this particle's offset from the centre
-                    if (have) {
-                        const Q xi = xq[s];
-                        xr = (float)qdiff<T>(xi.x, ox) * sc;
-                        yr = (float)qdiff<T>(xi.y, oy) * sc;
-                        zr = (float)qdiff<T>(xi.z, oz) * sc;
-                    }
-                    int cnt = have ? cnt_sm[i] : 0;
-                    int *lrow = nlist + list_row(have ? s : hstart, maxnb, lt);
-                    for (int kb = 0; kb < wpad; kb += LB_TPI) {  // uniform over the block
-                        const float4 q = stage[kb + sub];
-                        const float dx = xr - q.x, dy = yr - q.y, dz = zr - q.z;
-                        const int j = __float_as_int(q.w);
-                        const bool in = have && (dx * dx + dy * dy + dz * dz < rl2) && j != s;
-                        const unsigned grp = (__ballot_sync(0xffffffffu, in) >> gshift) &
-                                             ((1u << LB_TPI) - 1u);
-                        if (in) {
-                            const int pos = cnt + __popc(grp & below);
-                            if (pos < maxnb) lrow[list_col(pos, lt)] = j;
-                        }
-                        cnt += __popc(grp);
-                    }
-                    if (have && sub == 0) cnt_sm[i] = cnt;
-                }
+                rstart[tid] = a0;
+                rsplit[tid] = a1 - a0;
+                rwrap[tid] = b0 - (a1 - a0);
+                n = a1 - a0 + b1 - b0;
             }
-            __syncthreads();  // the chunk's counts are complete
-            for (int i = tid / LB_TPI; i < nch; i += LB_PPB) {
-                const int s = hstart + c0 + i;
-                const int cnt = cnt_sm[i], nn = min(cnt, maxnb);
-                if (sub == 0) {
-                    if (cnt > maxnb) raise_status(status, ST_NBOVF);
-                    nnb[s] = nn;
+            int v = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += t;
+            }
+            if (tid < (1 << NSEARCH)) pre[tid + 1] = v;  // (rows past the last: the total)
+            if (tid == 0) pre[0] = 0;
+        }
+        __syncthreads();
+        const int total = pre[NROW];
+        // Home particles in chunks of LB_HC, the stencil in windows (staged once
+        // per chunk; for all chunks where it fits one), LB_PPB particles a pass.
+        // A particle stays with its warp; its count is kept between windows.
+        int nst = 0;          // candidates staged
+        bool whole = false;   // the window holds the whole stencil
+        for (int h0 = 0; h0 < nhome; h0 += LB_HC) {
+            const int nch = min(LB_HC, nhome - h0);
+            for (int next = whole ? total : 0, first = 1; first || next < total; first = 0) {
+                if (!whole) {
+                    __syncthreads();  // the previous window's tests are done
+                    nst = 0;
+                    for (int q2 = 0; next < total && nst + LB_THREADS <= LB_SCAP; next += LB_THREADS, q2 ^= 1) {
+                        // candidate gg: the row holding it by binary search over pre
+                        const int gg = next + tid;
+                        bool keep = false;
+                        float4 q4;
+                        if (gg < total) {
+                            int lo = 0;
+#pragma unroll
+                            for (int b = 1 << (NSEARCH - 1); b > 0; b >>= 1)
+                                if (pre[lo + b] <= gg) lo += b;
+                            const int off = gg - pre[lo];
+                            const int j = off + (off < rsplit[lo] ? rstart[lo] : rwrap[lo]);
+                            const Q q = xq[j];
+                            // the staged copy carries the sorted index
+                            q4 = make_float4((float)qdiff<T>(q.x, ox) * sc, (float)qdiff<T>(q.y, oy) * sc,
+                                             (float)qdiff<T>(q.z, oz) * sc, __int_as_float(j));
+                            const float bx = fmaxf(fabsf(q4.x) - hw, 0.f), by = fmaxf(fabsf(q4.y) - hw, 0.f),
+                                        bz = fmaxf(fabsf(q4.z) - hw, 0.f);
+                            keep = bx * bx + by * by + bz * bz < rl2;
+                        }
+                        const unsigned m = __ballot_sync(0xffffffffu, keep);
+                        if (lane == 0) wsum[q2][warp] = __popc(m);
+                        __syncthreads();  // (the other half of wsum is free for the next round)
+                        int at = nst, all = 0;
+#pragma unroll
+                        for (int w = 0; w < LB_WARPS; ++w) {
+                            if (w < warp) at += wsum[q2][w];
+                            all += wsum[q2][w];
+                        }
+                        if (keep) stage[at + __popc(m & below)] = q4;
+                        nst += all;
+                    }
+                    // the window's last round is filled up out of range
+                    if (tid < 32 && nst + tid < ((nst + 31) & ~31))
+                        stage[nst + tid] = make_float4(1e30f, 1e30f, 1e30f, __int_as_float(-1));
+                    whole = first && next >= total;
+                    __syncthreads();
                 }
-                // pad to a whole block of PP_LIST_PAD entries with the
-                // particle itself (r = 0: no contribution); maxnb is a
-                // multiple of PP_LIST_PAD, so the pad stays in the list
-                const int pe = nn + sub;
-                if (pe < ((nn + PP_LIST_PAD - 1) & ~(PP_LIST_PAD - 1)))
-                    nlist[list_index(s, pe, maxnb, lt)] = s;
+                const bool last = next >= total;
+                for (int c0 = warp; c0 < nch; c0 += LB_PPB) {
+                    const int np = min(LB_P, (nch - c0 + LB_WARPS - 1) / LB_WARPS);  // this warp's
+                    float xr[LB_P], yr[LB_P], zr[LB_P];  // offsets from the centre
+                    int sp[LB_P], cnt[LB_P];
+                    int *lrow[LB_P];
+#pragma unroll
+                    for (int p = 0; p < LB_P; ++p) {
+                        const int i = p < np ? c0 + p * LB_WARPS : 0;
+                        sp[p] = hstart + h0 + i;
+                        cnt[p] = first ? 0 : cnt_sm[i];
+                        const Q xi = xq[sp[p]];
+                        xr[p] = (float)qdiff<T>(xi.x, ox) * sc;
+                        yr[p] = (float)qdiff<T>(xi.y, oy) * sc;
+                        zr[p] = (float)qdiff<T>(xi.z, oz) * sc;
+                        lrow[p] = nlist + list_row(sp[p], maxnb, lt);
+                    }
+                    for (int kb = 0; kb < nst; kb += 32) {
+                        const float4 q = stage[kb + lane];
+                        const int j = __float_as_int(q.w);
+#pragma unroll
+                        for (int p = 0; p < LB_P; ++p) {
+                            if (p >= np) break;
+                            const float dx = xr[p] - q.x, dy = yr[p] - q.y, dz = zr[p] - q.z;
+                            const bool in = (dx * dx + dy * dy + dz * dz < rl2) && j != sp[p];
+                            const unsigned m = __ballot_sync(0xffffffffu, in);
+                            if (m != 0u) {  // warp-uniform
+                                const int pos = cnt[p] + __popc(m & below);
+                                cnt[p] += __popc(m);
+                                if (in && pos < maxnb) lrow[p][list_col(pos, lt)] = j;
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int p = 0; p < LB_P; ++p) {
+                        if (p >= np) break;
+                        if (!last) {
+                            if (lane == 0) cnt_sm[c0 + p * LB_WARPS] = cnt[p];
+                            continue;
+                        }
+                        const int nn = min(cnt[p], maxnb);
+                        if (lane == 0) {
+                            if (cnt[p] > maxnb) raise_status(status, ST_NBOVF);
+                            nnb[sp[p]] = nn;
+                        }
+                        // pad to a whole block of PP_LIST_PAD entries with the
+                        // particle itself (r = 0: no contribution); maxnb is a
+                        // multiple of PP_LIST_PAD, so the pad stays in the list
+                        const int pe = nn + lane;
+                        if (pe < ((nn + PP_LIST_PAD - 1) & ~(PP_LIST_PAD - 1)))
+                            nlist[list_index(sp[p], pe, maxnb, lt)] = sp[p];
+                    }
+                }
             }
         }
     }
@@ -775,12 +825,6 @@ int pp_particles_per_block(int tpi) { return PPL_THREADS / tpi; }
 template <typename T> void configure_pp_kernels()
 {
     using Q = typename Coord<T>::Q;
-    const int lbs = (int)(LB_SCAP * sizeof(float4));
-    auto setl = [&](auto k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lbs); };
-    setl(k_build_lists<T, 1, 0>); setl(k_build_lists<T, 1, 1>);
-    setl(k_build_lists<T, 1, 2>); setl(k_build_lists<T, 1, 3>);
-    setl(k_build_lists<T, 2, 0>); setl(k_build_lists<T, 2, 1>);
-    setl(k_build_lists<T, 2, 2>); setl(k_build_lists<T, 2, 3>);
     if constexpr (sizeof(T) == 4) {
         const int tab = (int)(PP_TABLE_N * PP_TABLE_COPIES * sizeof(float4));
         auto set = [&](auto k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tab); };
