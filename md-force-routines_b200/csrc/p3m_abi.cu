@@ -25,6 +25,7 @@ struct p3m_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t st3 = nullptr;   // the n(q,t) branch of a step
     cudaEvent_t ev_join3 = nullptr;
+    cudaEvent_t ev_fin = nullptr, ev_red = nullptr;  // the step reduction beside the next drift
     int *counters = nullptr;      // [0] run step, [1] ring position, [2] it0, [3] n(q,t) rows,
                                   // [4] snapshots taken, [5] this step's snapshot slot
     int snap_interval = 0, snap_cap = 0;
@@ -68,12 +69,12 @@ struct p3m_ctx {
 
 static thread_local std::string g_err;
 
-// Steps captured in one multi-step graph on the FP32 path: fewer graph
-// launches, and no gap between them, for small systems whose steps last tens
-// of microseconds (cfg1: 0.0781 against 0.0810 ms per step). The FP64 path's
-// steps measured 3.5 % slower as groups, so it launches them one at a time.
+// Steps captured in one multi-step graph: fewer graph launches, no gap between
+// the steps of small systems, which last tens of microseconds, and an energy
+// reduction that runs beside the next step's drift (FP32, 1e4 particles: 54.2
+// -> 51.2 us a step; FP64, one at a time / in groups: 2e3 particles 70.0 /
+// 64.6, 1e4 78.2 / 73.5, 4e4 235.5 / 230.3).
 static const int kGraphSteps = 8;
-static int graph_steps(const p3m_ctx *ctx) { return ctx->prec == P3M_FP32 ? kGraphSteps : 1; }
 
 // Drop the captured step graphs (all, or only those recording n(q,t)).
 static void drop_graphs(p3m_ctx *ctx, bool rec_only = false)
@@ -396,6 +397,8 @@ extern "C" int p3m_destroy(p3m_ctx *ctx)
         cudaStreamDestroy(ctx->st3);
     }
     if (ctx->ev_join3) cudaEventDestroy(ctx->ev_join3);
+    if (ctx->ev_fin) cudaEventDestroy(ctx->ev_fin);
+    if (ctx->ev_red) cudaEventDestroy(ctx->ev_red);
     if (ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
     return P3M_OK;
@@ -581,6 +584,8 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
     CKC(cudaStreamCreateWithFlags(&ctx->st3, cudaStreamNonBlocking));
     CKC(cudaEventCreateWithFlags(&ctx->ev_join3, cudaEventDisableTiming));
+    CKC(cudaEventCreateWithFlags(&ctx->ev_fin, cudaEventDisableTiming));
+    CKC(cudaEventCreateWithFlags(&ctx->ev_red, cudaEventDisableTiming));
     CKC(dalloc(&s.reps, n_reps));
     CKC(cudaMemcpy(s.reps, ctx->rh.data(), sizeof(RepDev) * n_reps, cudaMemcpyHostToDevice));
     {
@@ -807,7 +812,14 @@ static int capture_graph(p3m_ctx *ctx, cudaGraphExec_t *out, long long *kernels,
 // no arrays -- and they join before the forces are combined, so the
 // latency-bound kernels of each branch fill the SMs the others leave idle
 // (one graph holds all branches).
-template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt)
+//
+// The energy reduction ends a step, but an NVE step that follows in the same
+// sequence (`more`) needs nothing of it to drift: it runs on the third stream
+// beside that drift, and the next step (`after`) waits for it before its
+// branches, which overwrite the partial sums. A thermostat's rescale and a
+// snapshot come after it, and keep it in line.
+template <typename T>
+static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, bool more = false)
 {
     DevState &s = ctx->s;
     cudaStream_t st = ctx->st, st2 = ctx->st2;
@@ -815,8 +827,10 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
     ctx->launches++;
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
     const bool fork = s.has_mesh || rec;
+    const bool beside = mode == P3M_MODE_NVE && ctx->snap_interval == 0;
     cudaError_t e = cudaSuccess;
-    if (fork) {
+    if (after && beside) e = cudaStreamWaitEvent(st, ctx->ev_red, 0);  // the previous step's sums
+    if (e == cudaSuccess && fork) {
         e = cudaEventRecord(ctx->ev_fork, st);
         if (e == cudaSuccess && s.has_mesh) {
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
@@ -856,9 +870,16 @@ template <typename T> static int seq_step(p3m_ctx *ctx, int mode, int record_nqt
     sums.u_pm_part = s.u_pm_part;
     sums.wc_total = s.wc;
     sums.wp_total = s.wp;
-    launch_step_reduce(s, mode, ctx->counters, ctx->ring, ctx->ring_cap, st, rec,
+    cudaStream_t st_red = st;
+    if (more && beside && e == cudaSuccess) {
+        e = cudaEventRecord(ctx->ev_fin, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->st3, ctx->ev_fin, 0);
+        st_red = ctx->st3;
+    }
+    launch_step_reduce(s, mode, ctx->counters, ctx->ring, ctx->ring_cap, st_red, rec,
                        ctx->snap_interval, ctx->snap_cap, sums);
     ctx->launches++;
+    if (st_red != st && e == cudaSuccess) e = cudaEventRecord(ctx->ev_red, st_red);
     if (mode == P3M_MODE_THERMOSTAT) {
         launch_scale_vel(s, st);
         ctx->launches++;
@@ -1405,7 +1426,8 @@ template <typename T> static int do_run(p3m_ctx *ctx, int n_steps, int mode, int
     auto capture = [&](int steps, cudaGraphExec_t *out) -> int {
         const int rc = capture_graph(ctx, out, &ctx->graph_kernels[gi][gr], [&] {
             int step_rc = P3M_OK;
-            for (int k = 0; k < steps && step_rc == P3M_OK; ++k) step_rc = seq_step<T>(ctx, mode, rec);
+            for (int k = 0; k < steps && step_rc == P3M_OK; ++k)
+                step_rc = seq_step<T>(ctx, mode, rec, k > 0, k + 1 < steps);
             return step_rc;
         });
         ctx->graph_kernels[gi][gr] /= steps;
@@ -1413,10 +1435,10 @@ template <typename T> static int do_run(p3m_ctx *ctx, int n_steps, int mode, int
     };
     // both graphs on first use, so that a warm-up of any length has captured
     // them before the runs it prepares
-    const int gsteps = graph_steps(ctx);
-    const int groups = (use_graph && gsteps > 1) ? n_steps / gsteps : 0;
+    const int gsteps = kGraphSteps;
+    const int groups = use_graph ? n_steps / gsteps : 0;
     if (use_graph && !ctx->graph[gi][gr]) RET(capture(1, &ctx->graph[gi][gr]));
-    if (use_graph && gsteps > 1 && !ctx->graphK[gi][gr]) RET(capture(gsteps, &ctx->graphK[gi][gr]));
+    if (use_graph && !ctx->graphK[gi][gr]) RET(capture(gsteps, &ctx->graphK[gi][gr]));
     for (int k = 0; k < groups; ++k) {
         CK(cudaGraphLaunch(ctx->graphK[gi][gr], ctx->st));
         ctx->launches += (long long)gsteps * ctx->graph_kernels[gi][gr];

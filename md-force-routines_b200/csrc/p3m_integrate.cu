@@ -93,17 +93,32 @@ __device__ __forceinline__ int block_replica(const RepDev *reps, int nrep, int b
 }
 
 // acc = af (a_pp + Z E) for every particle; with do_kick the second half kick
-// and the per-block FP64 sum of v^2.
+// and the per-block FP64 sum of v^2. The lists of this step are built and used:
+// block 0 counts the builds (steps only) and clears the flags, which the next
+// drift may raise again.
 template <typename T>
 __global__ void __launch_bounds__(PBLK)
 k_kick_finish(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ cell_slot,
               const int *__restrict__ brick_slot, const typename V4<T>::t *__restrict__ acc_pp,
               const typename V4<T>::t *__restrict__ acc_pm, int has_mesh,
               double *__restrict__ acc, double *__restrict__ vel, double *__restrict__ kin_part,
-              int do_kick, double *__restrict__ ep_out, int *status)
+              int do_kick, double *__restrict__ ep_out, int *status, int *__restrict__ rebuild,
+              int *__restrict__ prune, double *__restrict__ prune_count,
+              double *__restrict__ rep_out)
 {
     __shared__ double red[32];
     const int b = blockIdx.x;
+    if (b == 0) {
+        for (int k = threadIdx.x; k < nrep; k += PBLK) {
+            const bool fr = rebuild[k] != 0;
+            if (fr && do_kick) rep_out[8 * k + RO_REBUILDS] += 1.0;
+            if (prune) {  // inner lists: count the builds that came without an outer rebuild
+                if (prune[k] && !fr && do_kick) prune_count[k] += 1.0;
+                prune[k] = 0;
+            }
+            rebuild[k] = 0;
+        }
+    }
     const int r = block_replica(reps, nrep, b);
     const RepDev &R = reps[r];
     const int i = R.p_off + (b - R.blk_off) * PBLK + threadIdx.x;
@@ -154,8 +169,8 @@ __global__ void __launch_bounds__(SR_THREADS)
 k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
               const double *__restrict__ kin_part, double *__restrict__ rep_out,
               int mode, int *__restrict__ counters, double *__restrict__ ring,
-              int ring_cap, int recorded, int snap_interval, int snap_cap,
-              int *rebuild, int *status, StepSums sums, int *prune, double *prune_count)
+              int ring_cap, int recorded, int snap_interval, int snap_cap, int *status,
+              StepSums sums)
 {
     // counters: [0] steps since the run started, [1] energy-ring position,
     // [2] step index of the run's first step (thermostat_p3m_ord6.py:15 tests
@@ -192,16 +207,6 @@ k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
         part[2][w] = s;
     }
     __syncthreads();
-    if (w == 1 && lane == 0) {  // beside the first warp's sums
-        // this step's lists are built (count them); the next drift decides again
-        const bool fr = rebuild[r] != 0;
-        if (fr && mode != 2) rep_out[8 * r + RO_REBUILDS] += 1.0;
-        if (prune) {  // inner lists: count the builds that came without an outer rebuild
-            if (prune[r] && !fr && mode != 2) prune_count[r] += 1.0;
-            prune[r] = 0;
-        }
-        rebuild[r] = 0;
-    }
     if (w != 0) return;
     constexpr int NW = SR_THREADS / 32;
     t = warp_sum(lane < NW ? part[0][lane] : 0.0);
@@ -660,7 +665,9 @@ void launch_kick_finish(const DevState &s, int do_kick, double *ep_out, cudaStre
     k_kick_finish<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, s.cell_slot, s.brick_slot,
                                               (const T4 *)s.acc_pp, (const T4 *)s.acc_pm,
                                               s.has_mesh, s.acc, s.vel, s.kin_part, do_kick,
-                                              ep_out, s.status);
+                                              ep_out, s.status, s.rebuild,
+                                              s.prune_buf > 0.0 ? s.prune : nullptr,
+                                              s.prune_count, s.rep_out);
 }
 
 void launch_step_reduce(const DevState &s, int mode, int *counters, double *ring, int ring_cap,
@@ -669,8 +676,7 @@ void launch_step_reduce(const DevState &s, int mode, int *counters, double *ring
 {
     k_step_reduce<<<s.nrep, SR_THREADS, 0, st>>>(s.reps, s.nrep, s.nblk, s.kin_part, s.rep_out, mode,
                                       counters, ring, ring_cap, recorded, snap_interval, snap_cap,
-                                      s.rebuild, s.status, sums,
-                                      s.prune_buf > 0.0 ? s.prune : nullptr, s.prune_count);
+                                      s.status, sums);
 }
 
 void launch_snapshot(const DevState &s, const int *counters, double *snap, int *steps,
