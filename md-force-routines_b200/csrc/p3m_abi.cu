@@ -377,7 +377,7 @@ extern "C" int p3m_destroy(p3m_ctx *ctx)
                     s.nlist, s.rebuild, s.rb_list, s.pos_ref, s.pp_tables, s.pp_tables64,
                     s.nnb_in, s.nlist_in, s.prune, s.pos_pref, s.prune_count,
                     s.acc_pp, s.brick_key, s.brick_rank, s.brick_count, s.brick_start,
-                    s.brick_slot, s.slot_pt, s.slot_q, s.tiles, s.spec, s.ek, s.green, s.efield,
+                    s.brick_slot, s.place_done, s.slot_pt, s.slot_q, s.tiles, s.spec, s.ek, s.green, s.efield,
                     s.acc_pm, s.twiddle, s.u_pp_part, s.u_pm_part, s.kin_part, s.rep_out,
                     s.status, ctx->counters, ctx->ring, ctx->qmult, ctx->nqt_part, ctx->snap,
                     ctx->snap_steps,
@@ -638,6 +638,7 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(dalloc(&s.brick_count, (size_t)brick * BRICK_CNT_STRIDE));
     CKC(dalloc(&s.brick_start, (size_t)brick + 1));
     CKC(dalloc(&s.brick_slot, (size_t)p));
+    CKC(dalloc(&s.place_done, (size_t)n_reps));
     if (with_mesh)
         CKC(valloc(&s.tiles, (size_t)tile * (precision == P3M_FP32 ? sizeof(float) : sizeof(double))));
     {
@@ -694,9 +695,7 @@ template <typename T> static void seq_sort(p3m_ctx *ctx, bool keys)
     launch_build_lists<T>(s, ctx->st);  // rebuild steps
     ctx->launches += 4;
     if (s.has_mesh) {
-        launch_scan_bricks(s, ctx->st);
-        launch_place_bricks<T>(s, ctx->st);
-        ctx->launches += 2;
+        ctx->launches += launch_place_bricks<T>(s, ctx->st);
     }
 }
 
@@ -760,9 +759,7 @@ template <typename T> static int seq_force(p3m_ctx *ctx)
         e = cudaEventRecord(ctx->ev_fork, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
         if (e == cudaSuccess) {
-            launch_scan_bricks(s, st2);
-            launch_place_bricks<T>(s, st2);
-            ctx->launches += 2;
+            ctx->launches += launch_place_bricks<T>(s, st2);
             seq_pm<T>(ctx, true, st2);
             e = cudaEventRecord(ctx->ev_join, st2);
         }
@@ -817,17 +814,19 @@ static int capture_graph(p3m_ctx *ctx, cudaGraphExec_t *out, long long *kernels,
 // sequence (`more`) needs nothing of it to drift: it runs on the third stream
 // beside that drift, and the next step (`after`) waits for it before its
 // branches, which overwrite the partial sums. A thermostat's rescale and a
-// snapshot come after it, and keep it in line.
+// snapshot come after it, and keep it in line; the rescale of a step with a
+// successor is left to that step's drift.
 template <typename T>
 static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, bool more = false)
 {
     DevState &s = ctx->s;
     cudaStream_t st = ctx->st, st2 = ctx->st2;
-    launch_kick_drift<T>(s, st);
+    const bool thermo = mode == P3M_MODE_THERMOSTAT, plain = ctx->snap_interval == 0;
+    launch_kick_drift<T>(s, after && thermo && plain, st);
     ctx->launches++;
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
     const bool fork = s.has_mesh || rec;
-    const bool beside = mode == P3M_MODE_NVE && ctx->snap_interval == 0;
+    const bool beside = !thermo && plain;
     cudaError_t e = cudaSuccess;
     if (after && beside) e = cudaStreamWaitEvent(st, ctx->ev_red, 0);  // the previous step's sums
     if (e == cudaSuccess && fork) {
@@ -835,9 +834,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
         if (e == cudaSuccess && s.has_mesh) {
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
-                launch_scan_bricks(s, st2);
-                launch_place_bricks<T>(s, st2);
-                ctx->launches += 2;
+                ctx->launches += launch_place_bricks<T>(s, st2);
                 seq_pm<T>(ctx, false, st2);
                 e = cudaEventRecord(ctx->ev_join, st2);
             }
@@ -880,7 +877,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
                        ctx->snap_interval, ctx->snap_cap, sums);
     ctx->launches++;
     if (st_red != st && e == cudaSuccess) e = cudaEventRecord(ctx->ev_red, st_red);
-    if (mode == P3M_MODE_THERMOSTAT) {
+    if (thermo && !(more && plain)) {
         launch_scale_vel(s, st);
         ctx->launches++;
     }
@@ -1790,7 +1787,7 @@ template <typename T> static void enqueue_stage(p3m_ctx *ctx, int k)
     DevState &s = ctx->s;
     switch (k) {
     case 0:
-        launch_kick_drift<T>(s, ctx->st);
+        launch_kick_drift<T>(s, false, ctx->st);
         seq_sort<T>(ctx, false);
         break;
     case 1: seq_sort<T>(ctx, true); break;

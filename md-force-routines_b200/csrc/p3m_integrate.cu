@@ -36,7 +36,7 @@ __device__ __forceinline__ double wrap_once(double x, double L)
 // (a replica that rebuilds this step has them rewritten at its new slots by
 // k_fix_cells): a pass of its own read the positions again at random (1e6
 // particles: 40 us).
-template <typename T>
+template <typename T, bool RESCALE>
 __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                              double *__restrict__ pos, double *__restrict__ vel,
                              const double *__restrict__ acc, const double *__restrict__ pos_ref,
@@ -44,7 +44,8 @@ __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restr
                              int *__restrict__ brick_count, int has_mesh, int *rebuild, int *status,
                              const double *__restrict__ pos_pref, int *prune,
                              const int *__restrict__ cell_slot,
-                             typename Coord<T>::Q *__restrict__ xq)
+                             typename Coord<T>::Q *__restrict__ xq,
+                             const double *__restrict__ rep_out)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int r = prep[i];
@@ -54,7 +55,10 @@ __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restr
         bool vfin = true;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            double v = kick(vel[3 * i + d], acc[3 * i + d], R.dt);
+            // (the previous step's thermostat rescale, when it was left to this pass)
+            double v = vel[3 * i + d];
+            if (RESCALE) v *= rep_out[8 * r + RO_FACT];
+            v = kick(v, acc[3 * i + d], R.dt);
             vfin = vfin && isfinite(v);
             vel[3 * i + d] = v;
             x[d] = wrap_once(__dadd_rn(pos[3 * i + d], __dmul_rn(v, R.dt)), R.L);
@@ -644,13 +648,15 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
 // ---------------------------------------------------------------------------
 static int pgrid(int n) { int g = (n + 255) / 256; return g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g); }
 
-template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st)
+template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st)
 {
     const bool inner = s.prune_buf > 0.0;
-    k_kick_drift<T><<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
+    auto kern = rescale ? k_kick_drift<T, true> : k_kick_drift<T, false>;
+    kern<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
                                                 s.ntot, s.brick_key, s.brick_rank, s.brick_count, s.has_mesh,
                                                 s.rebuild, s.status, inner ? s.pos_pref : nullptr,
-                                                s.prune, s.cell_slot, (typename Coord<T>::Q *)s.xq);
+                                                s.prune, s.cell_slot, (typename Coord<T>::Q *)s.xq,
+                                                s.rep_out);
 }
 
 void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
@@ -738,7 +744,7 @@ void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double
 int gf_opt_blocks(int M) { return (int)((gf_triples(M) + GF_TRIPLES - 1) / GF_TRIPLES); }
 
 #define P3M_INST(T)                                                                             \
-    template void launch_kick_drift<T>(const DevState &, cudaStream_t);                          \
+    template void launch_kick_drift<T>(const DevState &, bool, cudaStream_t);                    \
     template void launch_kick_finish<T>(const DevState &, int, double *, cudaStream_t);          \
     template void launch_nqt<T>(const DevState &, const double *, const double *, int, int,      \
                                 double *, double *, const int *, int, cudaStream_t);            \

@@ -62,6 +62,7 @@ struct DevState {
     int *brick_key = nullptr, *brick_rank = nullptr;  // per particle: brick, arrival rank in it
     int *brick_count = nullptr;  // [nbrick * BRICK_CNT_STRIDE], zero between sorts
     int *brick_start = nullptr, *brick_slot = nullptr;
+    int *place_done = nullptr;   // [nrep] blocks of the placing pass that have read the counts
     // the particles in brick order: V4<T> (stencil offsets x, y, z, packed
     // base in the brick) and T charge per slot
     void *slot_pt = nullptr, *slot_q = nullptr;
@@ -91,10 +92,9 @@ template <typename T> void configure_mesh_kernels();
 template <typename T> void launch_keys(const DevState &s, cudaStream_t st);
 void launch_cell_keys(const DevState &s, cudaStream_t st);
 void launch_scan_cells(const DevState &s, cudaStream_t st);
-void launch_scan_bricks(const DevState &s, cudaStream_t st);
 void launch_scatter(const DevState &s, cudaStream_t st);
 template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st);
-template <typename T> void launch_place_bricks(const DevState &s, cudaStream_t st);
+template <typename T> int launch_place_bricks(const DevState &s, cudaStream_t st);  // kernels launched
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st);
 template <typename T> void launch_pp(const DevState &s, cudaStream_t st);
 int pp_particles_per_block(int tpi);
@@ -120,7 +120,8 @@ template <typename T> void launch_efield_from_mesh(const DevState &s, int rep,
 void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double L,
                    double *G_k, double *a_part, cudaStream_t st);
 
-template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st);
+// rescale: the velocities still lack the last step's thermostat factor
+template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st);
 template <typename T> void launch_kick_finish(const DevState &s, int do_kick, double *ep_out,
                                               cudaStream_t st);
 // Sums that k_step_reduce can take over from k_reduce_pp, k_reduce_pm and

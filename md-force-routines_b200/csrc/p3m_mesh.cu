@@ -159,23 +159,28 @@ template <typename T, int R, bool INV> __device__ __forceinline__ void dft(cplx<
 // and odd parts that mirrored nodes share: w[5 - c](x) = w[c](-x), and the
 // outermost are (1 -+ 2x)^5 / 3840. Coefficients are divided by 3840 and 1920
 // beforehand (the six divisions per axis were a third of the instructions of
-// an FP64 stencil).
+// an FP64 stencil). Multiplications and fused multiply-adds are written out, so
+// that every kernel that inlines this rounds alike: a brick's integer sums must
+// not depend on which instantiation made them.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 template <typename T>
 __device__ __forceinline__ void weights6(T x, T *w)
 {
-    const T x2 = x * x;
-    const T a = (T)1 - (T)2 * x, b = (T)1 + (T)2 * x;
-    const T a2 = a * a, b2 = b * b;
-    w[0] = a2 * a2 * (a * (T)(1.0 / 3840));
-    w[5] = b2 * b2 * (b * (T)(1.0 / 3840));
-    const T e1 = (T)(237.0 / 3840) + x2 * ((T)(840.0 / 3840) + x2 * (T)(-240.0 / 3840));
-    const T o1 = x * ((T)(750.0 / 3840) + x2 * ((T)(240.0 / 3840) + x2 * (T)(-160.0 / 3840)));
-    w[1] = e1 - o1;
-    w[4] = e1 + o1;
-    const T e2 = (T)(841.0 / 1920) + x2 * ((T)(-440.0 / 1920) + x2 * (T)(80.0 / 1920));
-    const T o2 = x * ((T)(770.0 / 1920) + x2 * ((T)(-560.0 / 1920) + x2 * (T)(160.0 / 1920)));
-    w[2] = e2 - o2;
-    w[3] = e2 + o2;
+    const T x2 = mul_rn(x, x);
+    const T a = fma((T)-2, x, (T)1), b = fma((T)2, x, (T)1);
+    const T a2 = mul_rn(a, a), b2 = mul_rn(b, b);
+    w[0] = mul_rn(mul_rn(a2, a2), mul_rn(a, (T)(1.0 / 3840)));
+    w[5] = mul_rn(mul_rn(b2, b2), mul_rn(b, (T)(1.0 / 3840)));
+    const T e1 = fma(x2, fma(x2, (T)(-240.0 / 3840), (T)(840.0 / 3840)), (T)(237.0 / 3840));
+    const T o1 = fma(x2, fma(x2, (T)(-160.0 / 3840), (T)(240.0 / 3840)), (T)(750.0 / 3840));
+    w[1] = fma(-x, o1, e1);
+    w[4] = fma(x, o1, e1);
+    const T e2 = fma(x2, fma(x2, (T)(80.0 / 1920), (T)(-440.0 / 1920)), (T)(841.0 / 1920));
+    const T o2 = fma(x2, fma(x2, (T)(160.0 / 1920), (T)(-560.0 / 1920)), (T)(770.0 / 1920));
+    w[2] = fma(-x, o2, e2);
+    w[3] = fma(x, o2, e2);
 }
 
 // One CTA of 256 threads per brick, a thread per particle, the 216
@@ -326,7 +331,7 @@ k_assign(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
                     const int row = base + (g * TILE + a) * TILE;
 #pragma unroll
                     for (int cx = 0; cx < 6; ++cx) {
-                        const T t = qzy * wx[cx];
+                        const T t = mul_rn(qzy, wx[cx]);
                         if constexpr (sizeof(T) == 4) {
                             const float hb = (t - 0.5f) + kRound;    // floor(t), as a float
                             const int hi = __float_as_int(hb) - kRoundBits;
@@ -1298,14 +1303,12 @@ template <typename T> void launch_assign(const DevState &s, cudaStream_t st)
     using A = typename V4<T>::t;
     const int parts = s.assign_parts;
     const int grid = grid_items(s.nbrick * parts, 148 * 16);
-    if (parts > 1)
-        k_assign<T, true><<<grid, A_THREADS, assign_smem(parts), st>>>(
-            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (T *)s.tiles,
-            s.nbrick, parts);
-    else
-        k_assign<T, false><<<grid, A_THREADS, assign_smem(1), st>>>(
-            s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt, (const T *)s.slot_q, (T *)s.tiles,
-            s.nbrick, parts);
+    auto go = [&](auto kern) {
+        kern<<<grid, A_THREADS, assign_smem(parts), st>>>(s.reps, s.nrep, s.brick_start, (const A *)s.slot_pt,
+                                                   (const T *)s.slot_q, (T *)s.tiles, s.nbrick, parts);
+    };
+    if (parts > 1) go(k_assign<T, true>);
+    else go(k_assign<T, false>);
 }
 
 template <typename T> void launch_fft_forward(const DevState &s, cudaStream_t st)
