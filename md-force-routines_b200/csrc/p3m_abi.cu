@@ -25,6 +25,7 @@ struct p3m_ctx {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t st3 = nullptr;   // the n(q,t) branch of a step
     cudaEvent_t ev_join3 = nullptr;
+    cudaEvent_t ev_asg = nullptr;                   // the charges are assigned
     cudaEvent_t ev_fin = nullptr, ev_red = nullptr;  // the step reduction beside the next drift
     int *counters = nullptr;      // [0] run step, [1] ring position, [2] it0, [3] n(q,t) rows,
                                   // [4] snapshots taken, [5] this step's snapshot slot
@@ -399,6 +400,7 @@ extern "C" int p3m_destroy(p3m_ctx *ctx)
     if (ctx->ev_join3) cudaEventDestroy(ctx->ev_join3);
     if (ctx->ev_fin) cudaEventDestroy(ctx->ev_fin);
     if (ctx->ev_red) cudaEventDestroy(ctx->ev_red);
+    if (ctx->ev_asg) cudaEventDestroy(ctx->ev_asg);
     if (ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
     return P3M_OK;
@@ -586,6 +588,7 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(cudaEventCreateWithFlags(&ctx->ev_join3, cudaEventDisableTiming));
     CKC(cudaEventCreateWithFlags(&ctx->ev_fin, cudaEventDisableTiming));
     CKC(cudaEventCreateWithFlags(&ctx->ev_red, cudaEventDisableTiming));
+    CKC(cudaEventCreateWithFlags(&ctx->ev_asg, cudaEventDisableTiming));
     CKC(dalloc(&s.reps, n_reps));
     CKC(cudaMemcpy(s.reps, ctx->rh.data(), sizeof(RepDev) * n_reps, cudaMemcpyHostToDevice));
     {
@@ -711,11 +714,13 @@ template <typename T> static void seq_pp(p3m_ctx *ctx, bool reduce = true, cudaS
     }
 }
 
-template <typename T> static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr)
+template <typename T>
+static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr, cudaEvent_t assigned = nullptr)
 {
     if (!st) st = ctx->st;
     DevState &s = ctx->s;
     launch_assign<T>(s, st);
+    if (assigned) cudaEventRecord(assigned, st);
     launch_fft_forward<T>(s, st);
     if (reduce) {
         launch_reduce_pm(s, st);
@@ -827,6 +832,13 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
     const bool fork = s.has_mesh || rec;
     const bool beside = !thermo && plain;
+    // FP32: the pair loop starts after the assignment. The two share the load
+    // path, and the mesh branch is the longer one: side by side the assignment
+    // lost more than the pair loop won (us a step, beside / after: 2e3 particles
+    // 44.6 / 44.1, 1e4 50.9 / 50.2, 1e5 273.9 / 271.9, 1e6 1824 / 1776; 20 x 1e4
+    // 403.4 / 404.8). FP64: the pair loop is bound by the double-precision pipe
+    // and hides behind the mesh branch only if it starts with it (75.6 / 76.7).
+    const bool pairs_wait = sizeof(T) == 4 && s.has_mesh;
     cudaError_t e = cudaSuccess;
     if (after && beside) e = cudaStreamWaitEvent(st, ctx->ev_red, 0);  // the previous step's sums
     if (e == cudaSuccess && fork) {
@@ -835,7 +847,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
                 ctx->launches += launch_place_bricks<T>(s, st2);
-                seq_pm<T>(ctx, false, st2);
+                seq_pm<T>(ctx, false, st2, pairs_wait ? ctx->ev_asg : nullptr);
                 e = cudaEventRecord(ctx->ev_join, st2);
             }
         }
@@ -856,6 +868,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
     launch_fix_cells<T>(s, st);
     launch_build_lists<T>(s, st);  // rebuild steps
     ctx->launches += 5;
+    if (e == cudaSuccess && pairs_wait) e = cudaStreamWaitEvent(st, ctx->ev_asg, 0);
     seq_pp<T>(ctx, false, st);
     if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
     if (e == cudaSuccess && rec) e = cudaStreamWaitEvent(st, ctx->ev_join3, 0);
