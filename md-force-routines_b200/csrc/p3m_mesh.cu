@@ -996,8 +996,12 @@ k_fft_x_c2r(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restrict
 // brick-sorted order so the caller forms acc = Z E (:308-310). One CTA per
 // brick: each field component's TILE^3 neighbourhood of the brick is staged
 // in shared memory (coalesced rows), and every particle of the brick reads
-// its 216 nodes from there; each thread keeps the weights of up to GPT
-// particles across the three components.
+// its 216 nodes from there.
+//
+// Bound: shared-memory reads, 648 words a particle at about two cycles per
+// warp's read: a brick's bank counts scatter about their mean, so however the
+// particles are dealt, most warps hold two of some bank (1e6 particles on
+// 256^3: 144 us of reads in a 200 us kernel).
 constexpr int G_THREADS = 256;
 
 // Gather tiles keep rows of GTX nodes (TILE padded up) so each row is filled
@@ -1009,8 +1013,12 @@ constexpr int GTILE = TILE * TILE * GTX;
 
 // NB field-tile buffers per CTA: with two, the copy of component c+1 is in
 // flight while component c is summed; with one, the CTA is half the size and,
-// held to 64 registers, four of them share an SM (FP32: 57 against 63 us on
-// the 20 x 64^3 ensemble). The choice is the context's gather_mode.
+// held to 48 registers, five of them share an SM (FP32: 57 against 63 us on
+// the 20 x 64^3 ensemble, with four). The choice is the context's gather_mode.
+// The first copies start before the particles are ranked, and a tile stays for
+// all chunks of its brick (us a step: FP64 1e4 particles 75.5 -> 73.9, 2e3
+// 42.5 -> 42.1; with the fifth CTA 20 x 1e4 404.7 -> 403.3, the mixed batch of
+// twelve 636 -> 633).
 //
 // NC field components per CTA: 3 (a CTA per brick), or 1 (a CTA per brick and
 // component: three times the work items, each staging one tile and repeating
@@ -1024,7 +1032,7 @@ constexpr int GTILE = TILE * TILE * GTX;
 constexpr int GATHER_SPLIT_MAX = 512;
 
 template <typename T, int NB, int NC>
-__global__ void __launch_bounds__(G_THREADS, sizeof(T) == 4 ? (NB == 1 ? 4 : 1) : 2)
+__global__ void __launch_bounds__(G_THREADS, sizeof(T) == 4 ? (NB == 1 ? 5 : 1) : 2)
 k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ brick_start,
          const typename V4<T>::t *__restrict__ slot_pt, const T *__restrict__ slot_q,
          const T *__restrict__ efield, long long nmesh,
@@ -1045,84 +1053,90 @@ k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
         const int bx = (local % nb) * BRICK, by = ((local / nb) % nb) * BRICK,
                   bz = (local / (nb * nb)) * BRICK;
         const int p0 = brick_start[b], p1 = brick_start[b + 1];
-        for (int c0 = p0; c0 < p1; c0 += G_THREADS) {
-            // Lanes of a warp read their particles' stencils at the same
-            // offsets from different bases, so two lanes whose bases share a
-            // shared-memory bank conflict on every read. The chunk's particles
-            // are ranked by bank (base mod 32) and dealt round-robin to the
-            // warps: each warp gets bases spread over the banks. Which thread
-            // handles a particle does not change its sums.
-            const int nch = min(G_THREADS, p1 - c0);
-            int bank = 0, rank = 0;
-            if (threadIdx.x < nch) {
-                const int pb = max(0, unpack_base(slot_pt[c0 + threadIdx.x].w));
-                bank = (((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15)) & 31;
+        if (p0 == p1) continue;
+        // component tiles through the NB buffers
+        auto issue = [&](int comp) {
+            constexpr int EPC = 16 / sizeof(T);   // elements per 16-byte chunk
+            constexpr int CPR = GTX / EPC;        // chunks per tile row
+            constexpr int RP = G_THREADS / CPR;   // tile rows per pass
+            static_assert(RP % TILE == 0, "a thread keeps its row's y");
+            if (threadIdx.x < RP * CPR) {
+                // thread: chunk ch of rows r0, r0 + RP, ... -- fixed x and
+                // y, z advancing by RP / TILE
+                const int ch = threadIdx.x % CPR, r0 = threadIdx.x / CPR;
+                const int gx = (bx + ch * EPC) & (M - 1), gy = (by + r0 % TILE) & (M - 1);
+                const T *exy = efield + comp * nmesh + R.mesh_off + (long long)gy * M + gx;
+                T *d = tile + (comp % NB) * GTILE + r0 * GTX + ch * EPC;
+                for (int tz = r0 / TILE; tz < TILE; tz += RP / TILE, d += RP * GTX)
+                    cp_async16(d, exy + (long long)((bz + tz) & (M - 1)) * M * M);
             }
-            __syncthreads();  // the previous chunk / brick is done with g_* and the buffers
-            g_src[threadIdx.x] = -1;
-            if (threadIdx.x < 32) g_cnt[threadIdx.x] = 0;
-            __syncthreads();
-            if (threadIdx.x < nch) rank = atomicAdd(&g_cnt[bank], 1);
-            __syncthreads();
-            if (threadIdx.x < 32) {  // exclusive scan of the bank counts
-                const int v = g_cnt[lane];
-                int x = v;
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        __syncthreads();  // the previous brick is done with the buffers
+        issue(cfirst);
+        if (NB == 2 && cfirst + 1 < cend) issue(cfirst + 1);
+        // Up to G_THREADS particles keep slot, base and weights over the
+        // components; more are taken in chunks from each staged tile.
+        const bool one = p1 - p0 <= G_THREADS;
+        T wx[6], wy[6], wz[6];
+        int p = -1, base = -1;
+        for (int comp = cfirst; comp < cend; ++comp) {
+            for (int c0 = p0; c0 < p1; c0 += G_THREADS) {
+                if (comp == cfirst || !one) {
+                    // Lanes of a warp read their particles' stencils at the same
+                    // offsets from different bases, so two lanes whose bases share a
+                    // shared-memory bank conflict on every read. The chunk's particles
+                    // are ranked by bank (base mod 32) and dealt round-robin to the
+                    // warps: each warp gets bases spread over the banks. Which thread
+                    // handles a particle does not change its sums.
+                    const int nch = min(G_THREADS, p1 - c0);
+                    int bank = 0, rank = 0;
+                    if (threadIdx.x < nch) {
+                        const int pb = max(0, unpack_base(slot_pt[c0 + threadIdx.x].w));
+                        bank = (((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15)) & 31;
+                    }
+                    __syncthreads();  // the previous chunk / brick is done with g_*
+                    g_src[threadIdx.x] = -1;
+                    if (threadIdx.x < 32) g_cnt[threadIdx.x] = 0;
+                    __syncthreads();
+                    if (threadIdx.x < nch) rank = atomicAdd(&g_cnt[bank], 1);
+                    __syncthreads();
+                    if (threadIdx.x < 32) {  // exclusive scan of the bank counts
+                        const int v = g_cnt[lane];
+                        int x = v;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += t;
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int t = __shfl_up_sync(0xffffffffu, x, o);
+                            if (lane >= o) x += t;
+                        }
+                        g_cnt[lane] = x - v;
+                    }
+                    __syncthreads();
+                    if (threadIdx.x < nch) {
+                        const int q = g_cnt[bank] + rank, nw = (nch + 31) >> 5;
+                        g_src[(q % nw) * 32 + q / nw] = c0 + threadIdx.x;
+                    }
+                    __syncthreads();
+                    p = g_src[threadIdx.x];
+                    base = -1;
+                    if (p >= 0) {
+                        const typename V4<T>::t v = slot_pt[p];
+                        const int pb = unpack_base(v.w);  // -1: flagged by the key pass
+                        if (pb >= 0) base = ((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15);
+                        weights6<T>(v.x, wx);
+                        weights6<T>(v.y, wy);
+                        weights6<T>(v.z, wz);
+                    }
                 }
-                g_cnt[lane] = x - v;
-            }
-            __syncthreads();
-            if (threadIdx.x < nch) {
-                const int q = g_cnt[bank] + rank, nw = (nch + 31) >> 5;
-                g_src[(q % nw) * 32 + q / nw] = c0 + threadIdx.x;
-            }
-            __syncthreads();
-            const int p = g_src[threadIdx.x];
-            T wx[6], wy[6], wz[6];
-            int base = -1;
-            T e[3] = {(T)0, (T)0, (T)0};
-            if (p >= 0) {
-                const typename V4<T>::t v = slot_pt[p];
-                const int pb = unpack_base(v.w);  // -1: flagged by the key pass
-                if (pb >= 0) base = ((pb >> 8) * TILE + ((pb >> 4) & 15)) * GTX + (pb & 15);
-                weights6<T>(v.x, wx);
-                weights6<T>(v.y, wy);
-                weights6<T>(v.z, wz);
-            }
-            // component tiles through the NB buffers
-            auto issue = [&](int comp) {
-                constexpr int EPC = 16 / sizeof(T);   // elements per 16-byte chunk
-                constexpr int CPR = GTX / EPC;        // chunks per tile row
-                constexpr int RP = G_THREADS / CPR;   // tile rows per pass
-                static_assert(RP % TILE == 0, "a thread keeps its row's y");
-                if (threadIdx.x < RP * CPR) {
-                    // thread: chunk ch of rows r0, r0 + RP, ... -- fixed x and
-                    // y, z advancing by RP / TILE
-                    const int ch = threadIdx.x % CPR, r0 = threadIdx.x / CPR;
-                    const int gx = (bx + ch * EPC) & (M - 1), gy = (by + r0 % TILE) & (M - 1);
-                    const T *exy = efield + comp * nmesh + R.mesh_off + (long long)gy * M + gx;
-                    T *d = tile + (comp % NB) * GTILE + r0 * GTX + ch * EPC;
-                    for (int tz = r0 / TILE; tz < TILE; tz += RP / TILE, d += RP * GTX)
-                        cp_async16(d, exy + (long long)((bz + tz) & (M - 1)) * M * M);
+                if (c0 == p0) {
+                    if (NB == 2 && comp + 1 < cend) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+                    __syncthreads();
                 }
-                asm volatile("cp.async.commit_group;\n" ::: "memory");
-            };
-            issue(cfirst);
-            for (int comp = cfirst; comp < cend; ++comp) {
-                if (NB == 2 && comp + 1 < cend) {
-                    issue(comp + 1);
-                    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-                } else {
-                    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                }
-                __syncthreads();
                 const T *tl = tile + (comp % NB) * GTILE;
+                T acc = 0;
                 if (base >= 0) {
                     // separable contraction: sum_g wz sum_a wy sum_c wx E
-                    T acc = 0;
 #pragma unroll
                     for (int g = 0; g < 6; ++g) {
                         T sg = 0;
@@ -1136,28 +1150,16 @@ k_gather(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
                         }
                         acc += wz[g] * sg;
                     }
-                    e[comp] = acc;
                 }
-                if (NB == 1 && comp + 1 < cend) {
-                    __syncthreads();
-                    issue(comp + 1);
-                } else if (comp + 2 < cend) {
-                    __syncthreads();  // buffer (comp % 2) is refilled next
+                if (p >= 0) {
+                    T *o = reinterpret_cast<T *>(acc_pm + p);  // (Ex, Ey, Ez, Z)
+                    o[comp] = acc;
+                    if (comp == 0) o[3] = slot_q[p];
                 }
             }
-            if (p >= 0) {
-                if constexpr (NC == 3) {
-                    typename V4<T>::t out;
-                    out.x = e[0];
-                    out.y = e[1];
-                    out.z = e[2];
-                    out.w = slot_q[p];
-                    acc_pm[p] = out;
-                } else {
-                    T *o = reinterpret_cast<T *>(acc_pm + p);  // (Ex, Ey, Ez, Z)
-                    o[cfirst] = e[cfirst];
-                    if (cfirst == 0) o[3] = slot_q[p];
-                }
+            if (comp + NB < cend) {
+                __syncthreads();  // buffer comp % NB is refilled
+                issue(comp + NB);
             }
         }
     }
