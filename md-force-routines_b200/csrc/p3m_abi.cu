@@ -57,7 +57,8 @@ struct p3m_ctx {
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     // kGraphSteps steps per graph (launched for whole groups of steps)
     cudaGraphExec_t graphK[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    long long graph_kernels[2][2] = {{0, 0}, {0, 0}};  // kernels per step of the captured graphs
+    long long graph_kernels[2][2] = {{0, 0}, {0, 0}};   // kernels of the captured graphs
+    long long graphK_kernels[2][2] = {{0, 0}, {0, 0}};
     cudaGraphExec_t graph_force = nullptr;             // one force evaluation (p3m_force)
     long long graph_force_kernels = 0;
     int ncell_cap = 0;            // cells allocated (grid with skin 0)
@@ -71,10 +72,11 @@ struct p3m_ctx {
 static thread_local std::string g_err;
 
 // Steps captured in one multi-step graph: fewer graph launches, no gap between
-// the steps of small systems, which last tens of microseconds, and an energy
-// reduction that runs beside the next step's drift (FP32, 1e4 particles: 54.2
-// -> 51.2 us a step; FP64, one at a time / in groups: 2e3 particles 70.0 /
-// 64.6, 1e4 78.2 / 73.5, 4e4 235.5 / 230.3).
+// the steps of small systems, which last tens of microseconds, one pass for a
+// step's end and the next one's drift, and an energy reduction off the serial
+// chain (reduction alone, FP32, 1e4 particles: 54.2 -> 51.2 us a step; FP64, one
+// at a time / in groups: 2e3 particles 70.0 / 64.6, 1e4 78.2 / 73.5, 4e4 235.5 /
+// 230.3; the pass: see k_finish_drift).
 static const int kGraphSteps = 8;
 
 // Drop the captured step graphs (all, or only those recording n(q,t)).
@@ -626,10 +628,10 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(dalloc(&s.cell_sub, (size_t)p));
     ctx->nlist_cap = (long long)((p + 31) / 32) * 32 * s.maxnb;
     CKC(dalloc(&s.nlist, (size_t)ctx->nlist_cap));
-    CKC(dalloc(&s.rebuild, (size_t)n_reps));
+    CKC(dalloc(&s.rebuild, (size_t)2 * n_reps));  // of a step, and of its successor (seq_step)
     CKC(dalloc(&s.rb_list, (size_t)2 * n_reps + 2));
     CKC(dalloc(&s.pos_ref, (size_t)3 * p));
-    CKC(dalloc(&s.prune, (size_t)n_reps));
+    CKC(dalloc(&s.prune, (size_t)2 * n_reps));
     CKC(dalloc(&s.nnb_in, (size_t)p));
     CKC(dalloc(&s.pos_pref, (size_t)3 * p));
     CKC(dalloc(&s.prune_count, (size_t)n_reps));
@@ -715,12 +717,14 @@ template <typename T> static void seq_pp(p3m_ctx *ctx, bool reduce = true, cudaS
 }
 
 template <typename T>
-static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr, cudaEvent_t assigned = nullptr)
+static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr, cudaEvent_t assigned = nullptr,
+                   cudaEvent_t sums_free = nullptr)
 {
     if (!st) st = ctx->st;
     DevState &s = ctx->s;
     launch_assign<T>(s, st);
     if (assigned) cudaEventRecord(assigned, st);
+    if (sums_free) cudaStreamWaitEvent(st, sums_free, 0);
     launch_fft_forward<T>(s, st);
     if (reduce) {
         launch_reduce_pm(s, st);
@@ -815,23 +819,33 @@ static int capture_graph(p3m_ctx *ctx, cudaGraphExec_t *out, long long *kernels,
 // latency-bound kernels of each branch fill the SMs the others leave idle
 // (one graph holds all branches).
 //
-// The energy reduction ends a step, but an NVE step that follows in the same
-// sequence (`more`) needs nothing of it to drift: it runs on the third stream
-// beside that drift, and the next step (`after`) waits for it before its
-// branches, which overwrite the partial sums. A thermostat's rescale and a
-// snapshot come after it, and keep it in line; the rescale of a step with a
-// successor is left to that step's drift.
+// Step k of a captured sequence of NVE steps without snapshots ends, when another
+// follows (`more`), in the pass that also drifts that one (k_finish_drift); its
+// energy reduction then runs on the third stream, and the next step waits for it
+// where it overwrites the partial sums (y/z transforms, pair loop). The flags of
+// consecutive steps are two arrays, the first of which is the one that calls
+// between sequences set; both are clear after a sequence. A thermostat's rescale
+// and a snapshot need the reduction and keep it in line; the rescale of a step
+// with a successor is left to that step's drift.
 template <typename T>
-static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, bool more = false)
+static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more = false)
 {
-    DevState &s = ctx->s;
     cudaStream_t st = ctx->st, st2 = ctx->st2;
-    const bool thermo = mode == P3M_MODE_THERMOSTAT, plain = ctx->snap_interval == 0;
-    launch_kick_drift<T>(s, after && thermo && plain, st);
-    ctx->launches++;
+    const bool thermo = mode == P3M_MODE_THERMOSTAT, plain = ctx->snap_interval == 0, after = k > 0;
+    const bool beside = !thermo && plain;
+    // the flags of this step and of the next
+    DevState s = ctx->s, next = ctx->s;
+    if (beside) {
+        DevState &odd = (k & 1) ? s : next;
+        odd.rebuild += s.nrep;
+        odd.prune += s.nrep;
+    }
+    if (!(after && beside)) {
+        launch_kick_drift<T>(s, after && thermo && plain, st);
+        ctx->launches++;
+    }
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
     const bool fork = s.has_mesh || rec;
-    const bool beside = !thermo && plain;
     // FP32: the pair loop starts after the assignment. The two share the load
     // path, and the mesh branch is the longer one: side by side the assignment
     // lost more than the pair loop won (us a step, beside / after: 2e3 particles
@@ -840,14 +854,15 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
     // and hides behind the mesh branch only if it starts with it (75.6 / 76.7).
     const bool pairs_wait = sizeof(T) == 4 && s.has_mesh;
     cudaError_t e = cudaSuccess;
-    if (after && beside) e = cudaStreamWaitEvent(st, ctx->ev_red, 0);  // the previous step's sums
+    // (the previous step's sums are taken before its partials are overwritten)
+    cudaEvent_t sums_free = after && beside ? ctx->ev_red : nullptr;
     if (e == cudaSuccess && fork) {
         e = cudaEventRecord(ctx->ev_fork, st);
         if (e == cudaSuccess && s.has_mesh) {
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
                 ctx->launches += launch_place_bricks<T>(s, st2);
-                seq_pm<T>(ctx, false, st2, pairs_wait ? ctx->ev_asg : nullptr);
+                seq_pm<T>(ctx, false, st2, pairs_wait ? ctx->ev_asg : nullptr, sums_free);
                 e = cudaEventRecord(ctx->ev_join, st2);
             }
         }
@@ -869,10 +884,13 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, bool after = false, 
     launch_build_lists<T>(s, st);  // rebuild steps
     ctx->launches += 5;
     if (e == cudaSuccess && pairs_wait) e = cudaStreamWaitEvent(st, ctx->ev_asg, 0);
-    seq_pp<T>(ctx, false, st);
+    if (e == cudaSuccess && sums_free) e = cudaStreamWaitEvent(st, sums_free, 0);
+    launch_pp<T>(s, st);
+    ctx->launches++;
     if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
     if (e == cudaSuccess && rec) e = cudaStreamWaitEvent(st, ctx->ev_join3, 0);
-    launch_kick_finish<T>(s, 1, nullptr, st);
+    if (more && beside) launch_finish_drift<T>(s, next, st);
+    else launch_kick_finish<T>(s, 1, nullptr, st);
     ctx->launches++;
     StepSums sums;  // the energy sums, in the reduction (the n(q,t) row is summed on its branch)
     sums.u_pp_part = s.u_pp_part;
@@ -1432,26 +1450,25 @@ template <typename T> static int do_run(p3m_ctx *ctx, int n_steps, int mode, int
     launch_set_counters(ctx->counters, 0, -1, it0, ctx->st);
     ctx->launches++;
     const int gi = (mode == P3M_MODE_THERMOSTAT) ? 1 : 0, gr = rec ? 1 : 0;
-    // capture `steps` steps into `*out` (the kernels of one step are counted)
-    auto capture = [&](int steps, cudaGraphExec_t *out) -> int {
-        const int rc = capture_graph(ctx, out, &ctx->graph_kernels[gi][gr], [&] {
+    // capture `steps` steps into `*out`, counting their kernels
+    auto capture = [&](int steps, cudaGraphExec_t *out, long long *kernels) -> int {
+        return capture_graph(ctx, out, kernels, [&] {
             int step_rc = P3M_OK;
             for (int k = 0; k < steps && step_rc == P3M_OK; ++k)
-                step_rc = seq_step<T>(ctx, mode, rec, k > 0, k + 1 < steps);
+                step_rc = seq_step<T>(ctx, mode, rec, k, k + 1 < steps);
             return step_rc;
         });
-        ctx->graph_kernels[gi][gr] /= steps;
-        return rc;
     };
     // both graphs on first use, so that a warm-up of any length has captured
     // them before the runs it prepares
     const int gsteps = kGraphSteps;
     const int groups = use_graph ? n_steps / gsteps : 0;
-    if (use_graph && !ctx->graph[gi][gr]) RET(capture(1, &ctx->graph[gi][gr]));
-    if (use_graph && !ctx->graphK[gi][gr]) RET(capture(gsteps, &ctx->graphK[gi][gr]));
+    if (use_graph && !ctx->graph[gi][gr]) RET(capture(1, &ctx->graph[gi][gr], &ctx->graph_kernels[gi][gr]));
+    if (use_graph && !ctx->graphK[gi][gr])
+        RET(capture(gsteps, &ctx->graphK[gi][gr], &ctx->graphK_kernels[gi][gr]));
     for (int k = 0; k < groups; ++k) {
         CK(cudaGraphLaunch(ctx->graphK[gi][gr], ctx->st));
-        ctx->launches += (long long)gsteps * ctx->graph_kernels[gi][gr];
+        ctx->launches += ctx->graphK_kernels[gi][gr];
     }
     for (int k = groups * gsteps; k < n_steps; ++k) {
         if (use_graph) {

@@ -7,6 +7,7 @@
 //   ... sort, PP, PM ...
 //   k_kick_finish  a = af (a_pp + Z E) (yukawa_p3m_ord6.py:21); v += 0.5 a dt
 //                  (:24); per-block sums of v^2 in FP64
+//   k_finish_drift both in one pass, where a captured sequence allows it
 //   k_step_reduce  per replica K = kf sum v^2, T = K/kf/N, U = uf (U_pp + U_pm
 //                  + U_self) (yukawa_p3m_ord6.py:23-24) and, in thermostat
 //                  mode, the factor of thermostat_p3m_ord6.py:9-23
@@ -32,60 +33,95 @@ __device__ __forceinline__ double wrap_once(double x, double L)
     return x;
 }
 
-// Also the coordinates of the pair stage, at the slots of the last cell sort
-// (a replica that rebuilds this step has them rewritten at its new slots by
-// k_fix_cells): a pass of its own read the positions again at random (1e6
-// particles: 40 us).
+// A particle's drift from its kicked velocity v: new position, rebuild and prune
+// flags, brick key and arrival rank. Also the coordinates of the pair stage, at
+// the slots of the last cell sort (a replica that rebuilds this step has them
+// rewritten at its new slots by k_fix_cells): a pass of its own read the
+// positions again at random (1e6 particles: 40 us).
+struct DriftArgs {
+    double *pos = nullptr;
+    const double *pos_ref = nullptr, *pos_pref = nullptr;  // pos_pref: inner lists only
+    int *brick_key = nullptr, *brick_rank = nullptr, *brick_count = nullptr;
+    int has_mesh = 0;
+    int *rebuild = nullptr, *prune = nullptr, *status = nullptr;
+    const int *cell_slot = nullptr;
+    void *xq = nullptr;
+};
+
+// What the drift reads, loaded before the pass's first store (the compiler keeps
+// loads behind stores that could alias them).
+struct DriftIn {
+    double x[3], ref[3], pref[3];
+    int slot;
+    __device__ __forceinline__ DriftIn(const DriftArgs &A, int i) : slot(A.cell_slot[i])
+    {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            x[d] = A.pos[3 * i + d];
+            ref[d] = A.pos_ref[3 * i + d];
+            pref[d] = A.pos_pref ? A.pos_pref[3 * i + d] : 0.0;
+        }
+    }
+};
+
+template <typename T>
+__device__ __forceinline__ void drift(const DriftArgs &A, const RepDev &R, int r, int i, const DriftIn &in,
+                                      const double *v)
+{
+    double x[3];
+    double d2 = 0.0, d2p = 0.0;
+    bool vfin = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        vfin = vfin && isfinite(v[d]);
+        x[d] = wrap_once(__dadd_rn(in.x[d], __dmul_rn(v[d], R.dt)), R.L);
+        A.pos[3 * i + d] = x[d];
+        // displacement since the last list rebuild, minimum image
+        double dd = x[d] - in.ref[d];
+        dd = fma(-R.L, rint(dd * R.inv_L), dd);
+        d2 = fma(dd, dd, d2);
+        if (A.pos_pref) {  // and since the last inner-list build
+            double dp = x[d] - in.pref[d];
+            dp = fma(-R.L, rint(dp * R.inv_L), dp);
+            d2p = fma(dp, dp, d2p);
+        }
+    }
+    // a non-finite velocity (or acceleration) is reported as such; the
+    // position it makes is also flagged by particle_keys below
+    if (!vfin) raise_status(A.status, ST_NONFINITE);
+    if (d2 > 0.25 * R.skin * R.skin && !A.rebuild[r]) atomicOr(A.rebuild + r, 1);
+    if (A.pos_pref && d2p > 0.25 * R.pbuf * R.pbuf && !A.prune[r]) atomicOr(A.prune + r, 1);
+    int b, rank = 0;
+    particle_keys(R, x[0], x[1], x[2], A.has_mesh, nullptr, &b, A.status);
+    if (b >= 0) rank = atomicAdd(&A.brick_count[b * BRICK_CNT_STRIDE], 1);
+    // while the atomic returns
+    ((typename Coord<T>::Q *)A.xq)[in.slot] = quantize<T>(x[0], x[1], x[2], R.inv_L, r);
+    if (b >= 0) {
+        A.brick_key[i] = b;
+        A.brick_rank[i] = rank;
+    }
+}
+
 template <typename T, bool RESCALE>
 __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restrict__ prep,
-                             double *__restrict__ pos, double *__restrict__ vel,
-                             const double *__restrict__ acc, const double *__restrict__ pos_ref,
-                             int ntot, int *__restrict__ brick_key, int *__restrict__ brick_rank,
-                             int *__restrict__ brick_count, int has_mesh, int *rebuild, int *status,
-                             const double *__restrict__ pos_pref, int *prune,
-                             const int *__restrict__ cell_slot,
-                             typename Coord<T>::Q *__restrict__ xq,
-                             const double *__restrict__ rep_out)
+                             double *__restrict__ vel, const double *__restrict__ acc, int ntot,
+                             const double *__restrict__ rep_out, DriftArgs A)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int r = prep[i];
         const RepDev &R = reps[r];
-        double x[3];
-        double d2 = 0.0, d2p = 0.0;
-        bool vfin = true;
+        const DriftIn in(A, i);
+        double v[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             // (the previous step's thermostat rescale, when it was left to this pass)
-            double v = vel[3 * i + d];
-            if (RESCALE) v *= rep_out[8 * r + RO_FACT];
-            v = kick(v, acc[3 * i + d], R.dt);
-            vfin = vfin && isfinite(v);
-            vel[3 * i + d] = v;
-            x[d] = wrap_once(__dadd_rn(pos[3 * i + d], __dmul_rn(v, R.dt)), R.L);
-            pos[3 * i + d] = x[d];
-            // displacement since the last list rebuild, minimum image
-            double dd = x[d] - pos_ref[3 * i + d];
-            dd -= R.L * rint(dd * R.inv_L);
-            d2 += dd * dd;
-            if (pos_pref) {  // and since the last inner-list build
-                double dp = x[d] - pos_pref[3 * i + d];
-                dp -= R.L * rint(dp * R.inv_L);
-                d2p += dp * dp;
-            }
+            v[d] = vel[3 * i + d];
+            if (RESCALE) v[d] *= rep_out[8 * r + RO_FACT];
+            v[d] = kick(v[d], acc[3 * i + d], R.dt);
         }
-        // a non-finite velocity (or acceleration) is reported as such; the
-        // position it makes is also flagged by particle_keys below
-        if (!vfin) raise_status(status, ST_NONFINITE);
-        if (d2 > 0.25 * R.skin * R.skin && !rebuild[r]) atomicOr(rebuild + r, 1);
-        if (pos_pref && d2p > 0.25 * R.pbuf * R.pbuf && !prune[r]) atomicOr(prune + r, 1);
-        int b, rank = 0;
-        particle_keys(R, x[0], x[1], x[2], has_mesh, nullptr, &b, status);
-        if (b >= 0) rank = atomicAdd(&brick_count[b * BRICK_CNT_STRIDE], 1);
-        xq[cell_slot[i]] = quantize<T>(x[0], x[1], x[2], R.inv_L, r);  // while the atomic returns
-        if (b >= 0) {
-            brick_key[i] = b;
-            brick_rank[i] = rank;
-        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) vel[3 * i + d] = v[d];
+        drift<T>(A, R, r, i, in, v);
     }
 }
 
@@ -96,68 +132,132 @@ __device__ __forceinline__ int block_replica(const RepDev *reps, int nrep, int b
     return find_rep(b, nrep, [&](int k) { return reps[k].blk_off; });
 }
 
+struct FinishArgs {
+    const int *cell_slot = nullptr, *brick_slot = nullptr;
+    const void *acc_pp = nullptr, *acc_pm = nullptr;
+    int has_mesh = 0;
+    double *vel = nullptr, *kin_part = nullptr;
+    int *status = nullptr;
+    int *rebuild = nullptr, *prune = nullptr;  // the finished step's flags; prune: inner lists only
+    double *prune_count = nullptr, *rep_out = nullptr;
+};
+
+// a = af (a_pp + Z E) of a particle
+template <typename T>
+__device__ __forceinline__ void combine(const FinishArgs &A, const RepDev &R, int i, double *a,
+                                        double *ep_out)
+{
+    using T4 = typename V4<T>::t;
+    const T4 ap = ((const T4 *)A.acc_pp)[A.cell_slot[i]];
+    a[0] = (double)ap.x;
+    a[1] = (double)ap.y;
+    a[2] = (double)ap.z;
+    if (A.has_mesh) {
+        const T4 e = ((const T4 *)A.acc_pm)[A.brick_slot[i]];
+        const double q = (double)e.w;
+        const double E[3] = {(double)e.x, (double)e.y, (double)e.z};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) a[d] = fma(q, E[d], a[d]);
+        if (ep_out) {
+            ep_out[3 * i + 0] = E[0];
+            ep_out[3 * i + 1] = E[1];
+            ep_out[3 * i + 2] = E[2];
+        }
+    }
+    bool finite = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        a[d] = R.af * a[d];
+        finite = finite && isfinite(a[d]);
+    }
+    if (!finite) raise_status(A.status, ST_NONFINITE);
+}
+
+// The lists of a step are built and used: count the builds (steps only) and
+// clear the flags. One block.
+__device__ __forceinline__ void settle_flags(const FinishArgs &A, int nrep, int do_kick)
+{
+    for (int k = threadIdx.x; k < nrep; k += PBLK) {
+        const bool fr = A.rebuild[k] != 0;
+        if (fr && do_kick) A.rep_out[8 * k + RO_REBUILDS] += 1.0;
+        if (A.prune) {  // inner lists: count the builds that came without an outer rebuild
+            if (A.prune[k] && !fr && do_kick) A.prune_count[k] += 1.0;
+            A.prune[k] = 0;
+        }
+        A.rebuild[k] = 0;
+    }
+}
+
 // acc = af (a_pp + Z E) for every particle; with do_kick the second half kick
-// and the per-block FP64 sum of v^2. The lists of this step are built and used:
-// block 0 counts the builds (steps only) and clears the flags, which the next
+// and the per-block FP64 sum of v^2. Block 0 settles the flags, which the next
 // drift may raise again.
 template <typename T>
 __global__ void __launch_bounds__(PBLK)
-k_kick_finish(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ cell_slot,
-              const int *__restrict__ brick_slot, const typename V4<T>::t *__restrict__ acc_pp,
-              const typename V4<T>::t *__restrict__ acc_pm, int has_mesh,
-              double *__restrict__ acc, double *__restrict__ vel, double *__restrict__ kin_part,
-              int do_kick, double *__restrict__ ep_out, int *status, int *__restrict__ rebuild,
-              int *__restrict__ prune, double *__restrict__ prune_count,
-              double *__restrict__ rep_out)
+k_kick_finish(const RepDev *__restrict__ reps, int nrep, FinishArgs A, double *__restrict__ acc,
+              int do_kick, double *__restrict__ ep_out)
 {
     __shared__ double red[32];
     const int b = blockIdx.x;
-    if (b == 0) {
-        for (int k = threadIdx.x; k < nrep; k += PBLK) {
-            const bool fr = rebuild[k] != 0;
-            if (fr && do_kick) rep_out[8 * k + RO_REBUILDS] += 1.0;
-            if (prune) {  // inner lists: count the builds that came without an outer rebuild
-                if (prune[k] && !fr && do_kick) prune_count[k] += 1.0;
-                prune[k] = 0;
-            }
-            rebuild[k] = 0;
-        }
-    }
+    if (b == 0) settle_flags(A, nrep, do_kick);
     const int r = block_replica(reps, nrep, b);
     const RepDev &R = reps[r];
     const int i = R.p_off + (b - R.blk_off) * PBLK + threadIdx.x;
     double kin = 0.0;
     if (i < R.p_off + R.n) {
-        const typename V4<T>::t ap = acc_pp[cell_slot[i]];
-        double a[3] = {(double)ap.x, (double)ap.y, (double)ap.z};
-        if (has_mesh) {
-            const typename V4<T>::t e = acc_pm[brick_slot[i]];
-            const double q = (double)e.w;
-            const double E[3] = {(double)e.x, (double)e.y, (double)e.z};
+        double a[3], v[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) a[d] = a[d] + q * E[d];
-            if (ep_out) {
-                ep_out[3 * i + 0] = E[0];
-                ep_out[3 * i + 1] = E[1];
-                ep_out[3 * i + 2] = E[2];
-            }
-        }
-        bool finite = true;
+        for (int d = 0; d < 3; ++d) v[d] = do_kick ? A.vel[3 * i + d] : 0.0;
+        combine<T>(A, R, i, a, ep_out);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const double ad = R.af * a[d];
-            finite = finite && isfinite(ad);
-            acc[3 * i + d] = ad;
+            acc[3 * i + d] = a[d];
             if (do_kick) {
-                const double v = kick(vel[3 * i + d], ad, R.dt);
-                vel[3 * i + d] = v;
-                kin += v * v;
+                v[d] = kick(v[d], a[d], R.dt);
+                A.vel[3 * i + d] = v[d];
+                kin = fma(v[d], v[d], kin);
             }
         }
-        if (!finite) raise_status(status, ST_NONFINITE);
     }
     const double t = block_sum(kin, red);
-    if (threadIdx.x == 0) kin_part[b] = t;
+    if (threadIdx.x == 0) A.kin_part[b] = t;
+}
+
+// A step's end and the next one's beginning in one pass, for steps of one
+// captured sequence with nothing between them that needs all particles (NVE, no
+// snapshots): second half kick, sum of v^2, first half kick, drift. The
+// acceleration stays in registers. The two steps' flags are different arrays (F's
+// are settled, D's raised). Bound: latency in small systems -- a kernel and its
+// edge less on the serial chain -- and memory in large ones (us a step, two passes
+// / one: 1e4 particles 50.0 / 47.4, FP64 74.0 / 71.3, 20 x 1e4 403 / 400, 1e5
+// 271.1 / 269.6, 1e6 1775 / 1746).
+template <typename T>
+__global__ void __launch_bounds__(PBLK)
+k_finish_drift(const RepDev *__restrict__ reps, int nrep, FinishArgs F, DriftArgs D)
+{
+    __shared__ double red[32];
+    const int b = blockIdx.x;
+    if (b == 0) settle_flags(F, nrep, 1);
+    const int r = block_replica(reps, nrep, b);
+    const RepDev &R = reps[r];
+    const int i = R.p_off + (b - R.blk_off) * PBLK + threadIdx.x;
+    double kin = 0.0;
+    if (i < R.p_off + R.n) {
+        const DriftIn in(D, i);
+        double a[3], v[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[d] = F.vel[3 * i + d];
+        combine<T>(F, R, i, a, nullptr);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            v[d] = kick(v[d], a[d], R.dt);
+            kin = fma(v[d], v[d], kin);
+            v[d] = kick(v[d], a[d], R.dt);
+            F.vel[3 * i + d] = v[d];
+        }
+        drift<T>(D, R, r, i, in, v);
+    }
+    const double t = block_sum(kin, red);
+    if (threadIdx.x == 0) F.kin_part[b] = t;
 }
 
 // Energies, temperature and the thermostat factor, one block per replica; one
@@ -648,15 +748,46 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
 // ---------------------------------------------------------------------------
 static int pgrid(int n) { int g = (n + 255) / 256; return g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g); }
 
+static DriftArgs drift_args(const DevState &s)
+{
+    DriftArgs A;
+    A.pos = s.pos;
+    A.pos_ref = s.pos_ref;
+    A.pos_pref = s.prune_buf > 0.0 ? s.pos_pref : nullptr;
+    A.brick_key = s.brick_key;
+    A.brick_rank = s.brick_rank;
+    A.brick_count = s.brick_count;
+    A.has_mesh = s.has_mesh;
+    A.rebuild = s.rebuild;
+    A.prune = s.prune;
+    A.status = s.status;
+    A.cell_slot = s.cell_slot;
+    A.xq = s.xq;
+    return A;
+}
+
+static FinishArgs finish_args(const DevState &s)
+{
+    FinishArgs A;
+    A.cell_slot = s.cell_slot;
+    A.brick_slot = s.brick_slot;
+    A.acc_pp = s.acc_pp;
+    A.acc_pm = s.acc_pm;
+    A.has_mesh = s.has_mesh;
+    A.vel = s.vel;
+    A.kin_part = s.kin_part;
+    A.status = s.status;
+    A.rebuild = s.rebuild;
+    A.prune = s.prune_buf > 0.0 ? s.prune : nullptr;
+    A.prune_count = s.prune_count;
+    A.rep_out = s.rep_out;
+    return A;
+}
+
 template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st)
 {
-    const bool inner = s.prune_buf > 0.0;
     auto kern = rescale ? k_kick_drift<T, true> : k_kick_drift<T, false>;
-    kern<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.pos, s.vel, s.acc, s.pos_ref,
-                                                s.ntot, s.brick_key, s.brick_rank, s.brick_count, s.has_mesh,
-                                                s.rebuild, s.status, inner ? s.pos_pref : nullptr,
-                                                s.prune, s.cell_slot, (typename Coord<T>::Q *)s.xq,
-                                                s.rep_out);
+    kern<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.vel, s.acc, s.ntot, s.rep_out, drift_args(s));
 }
 
 void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
@@ -667,13 +798,12 @@ void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
 template <typename T>
 void launch_kick_finish(const DevState &s, int do_kick, double *ep_out, cudaStream_t st)
 {
-    using T4 = typename V4<T>::t;
-    k_kick_finish<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, s.cell_slot, s.brick_slot,
-                                              (const T4 *)s.acc_pp, (const T4 *)s.acc_pm,
-                                              s.has_mesh, s.acc, s.vel, s.kin_part, do_kick,
-                                              ep_out, s.status, s.rebuild,
-                                              s.prune_buf > 0.0 ? s.prune : nullptr,
-                                              s.prune_count, s.rep_out);
+    k_kick_finish<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, finish_args(s), s.acc, do_kick, ep_out);
+}
+
+template <typename T> void launch_finish_drift(const DevState &s, const DevState &next, cudaStream_t st)
+{
+    k_finish_drift<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, finish_args(s), drift_args(next));
 }
 
 void launch_step_reduce(const DevState &s, int mode, int *counters, double *ring, int ring_cap,
@@ -746,6 +876,7 @@ int gf_opt_blocks(int M) { return (int)((gf_triples(M) + GF_TRIPLES - 1) / GF_TR
 #define P3M_INST(T)                                                                             \
     template void launch_kick_drift<T>(const DevState &, bool, cudaStream_t);                    \
     template void launch_kick_finish<T>(const DevState &, int, double *, cudaStream_t);          \
+    template void launch_finish_drift<T>(const DevState &, const DevState &, cudaStream_t);      \
     template void launch_nqt<T>(const DevState &, const double *, const double *, int, int,      \
                                 double *, double *, const int *, int, cudaStream_t);            \
     template void configure_integrate_kernels<T>(int);                                          \

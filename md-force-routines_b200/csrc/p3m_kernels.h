@@ -124,6 +124,8 @@ void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double
 template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st);
 template <typename T> void launch_kick_finish(const DevState &s, int do_kick, double *ep_out,
                                               cudaStream_t st);
+// The end of a step and the drift of the next, whose flags are next's.
+template <typename T> void launch_finish_drift(const DevState &s, const DevState &next, cudaStream_t st);
 // Sums that k_step_reduce can take over from k_reduce_pp, k_reduce_pm and
 // k_nqt_reduce inside a step (NULL pointers: not this time).
 struct StepSums {
