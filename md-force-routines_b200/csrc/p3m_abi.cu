@@ -820,28 +820,30 @@ static int capture_graph(p3m_ctx *ctx, cudaGraphExec_t *out, long long *kernels,
 // (one graph holds all branches).
 //
 // Step k of a captured sequence of NVE steps without snapshots ends, when another
-// follows (`more`), in the pass that also drifts that one (k_finish_drift); its
-// energy reduction then runs on the third stream, and the next step waits for it
-// where it overwrites the partial sums (y/z transforms, pair loop). The flags of
-// consecutive steps are two arrays, the first of which is the one that calls
-// between sequences set; both are clear after a sequence. A thermostat's rescale
-// and a snapshot need the reduction and keep it in line; the rescale of a step
-// with a successor is left to that step's drift.
+// follows (`more`), in the pass that also drifts that one (k_finish_drift). The
+// flags of consecutive steps are then two arrays, the first of which is the one
+// that calls between sequences set; both are clear after a sequence. A thermostat
+// step with a successor leaves its rescale to that step's drift
+// (k_rescale_drift). Either way the energy reduction runs on the third stream,
+// and the next step waits for it where it overwrites the partial sums (y/z
+// transforms, pair loop). A snapshot needs the reduction and keeps it in line.
 template <typename T>
 static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more = false)
 {
     cudaStream_t st = ctx->st, st2 = ctx->st2;
     const bool thermo = mode == P3M_MODE_THERMOSTAT, plain = ctx->snap_interval == 0, after = k > 0;
-    const bool beside = !thermo && plain;
+    // one pass for a step's end and the next one's drift
+    const bool fuse = !thermo && plain;
     // the flags of this step and of the next
     DevState s = ctx->s, next = ctx->s;
-    if (beside) {
+    if (fuse) {
         DevState &odd = (k & 1) ? s : next;
         odd.rebuild += s.nrep;
         odd.prune += s.nrep;
     }
-    if (!(after && beside)) {
-        launch_kick_drift<T>(s, after && thermo && plain, st);
+    if (!(after && fuse)) {
+        if (after && plain) launch_rescale_drift<T>(s, ctx->counters, st);
+        else launch_kick_drift<T>(s, st);
         ctx->launches++;
     }
     const int rec = (record_nqt && ctx->nq > 0) ? 1 : 0;
@@ -855,7 +857,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more
     const bool pairs_wait = sizeof(T) == 4 && s.has_mesh;
     cudaError_t e = cudaSuccess;
     // (the previous step's sums are taken before its partials are overwritten)
-    cudaEvent_t sums_free = after && beside ? ctx->ev_red : nullptr;
+    cudaEvent_t sums_free = after && plain ? ctx->ev_red : nullptr;
     if (e == cudaSuccess && fork) {
         e = cudaEventRecord(ctx->ev_fork, st);
         if (e == cudaSuccess && s.has_mesh) {
@@ -889,8 +891,8 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more
     ctx->launches++;
     if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
     if (e == cudaSuccess && rec) e = cudaStreamWaitEvent(st, ctx->ev_join3, 0);
-    if (more && beside) launch_finish_drift<T>(s, next, st);
-    else launch_kick_finish<T>(s, 1, nullptr, st);
+    if (more && fuse) launch_finish_drift<T>(s, next, st);
+    else launch_kick_finish<T>(s, 1, nullptr, st, more && plain ? ctx->counters : nullptr);
     ctx->launches++;
     StepSums sums;  // the energy sums, in the reduction (the n(q,t) row is summed on its branch)
     sums.u_pp_part = s.u_pp_part;
@@ -899,7 +901,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more
     sums.wc_total = s.wc;
     sums.wp_total = s.wp;
     cudaStream_t st_red = st;
-    if (more && beside && e == cudaSuccess) {
+    if (more && plain && e == cudaSuccess) {
         e = cudaEventRecord(ctx->ev_fin, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->st3, ctx->ev_fin, 0);
         st_red = ctx->st3;
@@ -1817,7 +1819,7 @@ template <typename T> static void enqueue_stage(p3m_ctx *ctx, int k)
     DevState &s = ctx->s;
     switch (k) {
     case 0:
-        launch_kick_drift<T>(s, false, ctx->st);
+        launch_kick_drift<T>(s, ctx->st);
         seq_sort<T>(ctx, false);
         break;
     case 1: seq_sort<T>(ctx, true); break;

@@ -102,10 +102,10 @@ __device__ __forceinline__ void drift(const DriftArgs &A, const RepDev &R, int r
     }
 }
 
-template <typename T, bool RESCALE>
+template <typename T>
 __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restrict__ prep,
                              double *__restrict__ vel, const double *__restrict__ acc, int ntot,
-                             const double *__restrict__ rep_out, DriftArgs A)
+                             DriftArgs A)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntot; i += gridDim.x * blockDim.x) {
         const int r = prep[i];
@@ -114,10 +114,7 @@ __global__ void k_kick_drift(const RepDev *__restrict__ reps, const int *__restr
         double v[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            // (the previous step's thermostat rescale, when it was left to this pass)
-            v[d] = vel[3 * i + d];
-            if (RESCALE) v[d] *= rep_out[8 * r + RO_FACT];
-            v[d] = kick(v[d], acc[3 * i + d], R.dt);
+            v[d] = kick(vel[3 * i + d], acc[3 * i + d], R.dt);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) vel[3 * i + d] = v[d];
@@ -132,6 +129,62 @@ __device__ __forceinline__ int block_replica(const RepDev *reps, int nrep, int b
     return find_rep(b, nrep, [&](int k) { return reps[k].blk_off; });
 }
 
+constexpr int SR_THREADS = 512;
+
+// Sum of a replica's kinetic partials [b0, b1), in every thread of the block:
+// entry k by thread k mod SR_THREADS, then a fixed tree, whatever the block size.
+// red: SR_THREADS / 32 doubles.
+template <int NT>
+__device__ __forceinline__ double kin_sum(const double *__restrict__ kin_part, int b0, int b1, double *red)
+{
+    static_assert(SR_THREADS % NT == 0, "whole shares");
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+#pragma unroll
+    for (int h = 0; h < SR_THREADS / NT; ++h) {
+        double s = 0.0;
+        for (int k = b0 + tid + h * NT; k < b1; k += SR_THREADS) s += kin_part[k];
+        s = warp_sum(s);
+        if (lane == 0) red[w + h * (NT / 32)] = s;
+    }
+    __syncthreads();
+    return warp_sum(lane < SR_THREADS / 32 ? red[lane] : 0.0);
+}
+
+// The thermostat's factor after step `it`, from the sum of v^2
+// (thermostat_p3m_ord6.py:15-23)
+__device__ __forceinline__ double thermostat_factor(const RepDev &R, double s, int it)
+{
+    const double T = R.kf * s / R.kf / (double)R.n;
+    return (it <= 1999) ? sqrt(R.t_desired / T) : sqrt((20.0 * R.t_desired / T - 1.0) / 20.0);
+}
+
+// k_kick_drift after a thermostat step of the same captured sequence: every
+// block takes its replica's factor from the kinetic partials itself, so that the
+// energy reduction, which does the same sum, runs beside this pass and not
+// before it (2e3 particles 41.2 -> 39.3 us a step, twelve uneven replicas 631.2 ->
+// 630.2). it: the finished step's index.
+template <typename T>
+__global__ void __launch_bounds__(PBLK)
+k_rescale_drift(const RepDev *__restrict__ reps, int nrep, int nblk, double *__restrict__ vel,
+                const double *__restrict__ acc, const double *__restrict__ kin_part,
+                const int *__restrict__ it, DriftArgs A)
+{
+    __shared__ double red[SR_THREADS / 32];
+    const int b = blockIdx.x, r = block_replica(reps, nrep, b);
+    const RepDev &R = reps[r];
+    const int i = R.p_off + (b - R.blk_off) * PBLK + threadIdx.x;
+    const double s = kin_sum<PBLK>(kin_part, R.blk_off, r + 1 < nrep ? reps[r + 1].blk_off : nblk, red);
+    if (i >= R.p_off + R.n) return;
+    const DriftIn in(A, i);
+    const double fact = thermostat_factor(R, s, *it);
+    double v[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[d] = kick(__dmul_rn(vel[3 * i + d], fact), acc[3 * i + d], R.dt);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) vel[3 * i + d] = v[d];
+    drift<T>(A, R, r, i, in, v);
+}
+
 struct FinishArgs {
     const int *cell_slot = nullptr, *brick_slot = nullptr;
     const void *acc_pp = nullptr, *acc_pm = nullptr;
@@ -140,6 +193,7 @@ struct FinishArgs {
     int *status = nullptr;
     int *rebuild = nullptr, *prune = nullptr;  // the finished step's flags; prune: inner lists only
     double *prune_count = nullptr, *rep_out = nullptr;
+    int *counters = nullptr;  // set: [7] receives the step's index, for k_rescale_drift
 };
 
 // a = af (a_pp + Z E) of a particle
@@ -198,7 +252,10 @@ k_kick_finish(const RepDev *__restrict__ reps, int nrep, FinishArgs A, double *_
 {
     __shared__ double red[32];
     const int b = blockIdx.x;
-    if (b == 0) settle_flags(A, nrep, do_kick);
+    if (b == 0) {
+        settle_flags(A, nrep, do_kick);
+        if (A.counters && threadIdx.x == 0) A.counters[7] = A.counters[2] + A.counters[0];
+    }
     const int r = block_replica(reps, nrep, b);
     const RepDev &R = reps[r];
     const int i = R.p_off + (b - R.blk_off) * PBLK + threadIdx.x;
@@ -267,8 +324,6 @@ k_finish_drift(const RepDev *__restrict__ reps, int nrep, FinishArgs F, DriftArg
 // k by thread k mod SR_THREADS, then a fixed tree -- the same order whatever the
 // batch). One block for all replicas, a warp each, took 5.4 us for 1e4 particles
 // against 4.0, 7.4 for 20 x 1e4 against 5.9, 30 for 1e6 against 8.9.
-constexpr int SR_THREADS = 512;
-
 __global__ void __launch_bounds__(SR_THREADS)
 k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
               const double *__restrict__ kin_part, double *__restrict__ rep_out,
@@ -279,14 +334,15 @@ k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
     // counters: [0] steps since the run started, [1] energy-ring position,
     // [2] step index of the run's first step (thermostat_p3m_ord6.py:15 tests
     // it <= 1999), [3] n(q,t) rows recorded, [4] snapshots taken, [5] the
-    // snapshot slot this step writes (-1: none), [6] blocks finished
+    // snapshot slot this step writes (-1: none), [6] blocks finished, [7] see
+    // k_kick_finish
     __shared__ double part[3][SR_THREADS / 32];
     const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int it = counters[2] + counters[0];
     const int step = counters[1];
     const RepDev &R = reps[r];
     const bool last = r + 1 == nrep;
-    double t = 0.0, tm = 0.0, s = 0.0;
+    double t = 0.0, tm = 0.0;
     if (sums.u_pp_part) {  // (k_reduce_pp and k_reduce_pm outside a step)
         const int b0 = R.pp_blk_off, b1 = last ? sums.pp_nblk : reps[r + 1].pp_blk_off;
         for (int k = b0 + tid; k < b1; k += SR_THREADS) t += sums.u_pp_part[k];
@@ -298,24 +354,17 @@ k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
             for (int k = p0 + tid; k < p1; k += SR_THREADS) tm += sums.u_pm_part[k];
         }
     }
-    {
-        const int b0 = R.blk_off, b1 = last ? nblk : reps[r + 1].blk_off;
-        for (int k = b0 + tid; k < b1; k += SR_THREADS) s += kin_part[k];
-    }
     t = warp_sum(t);
     tm = warp_sum(tm);
-    s = warp_sum(s);
     if (lane == 0) {
         part[0][w] = t;
         part[1][w] = tm;
-        part[2][w] = s;
     }
-    __syncthreads();
+    const double s = kin_sum<SR_THREADS>(kin_part, R.blk_off, last ? nblk : reps[r + 1].blk_off, part[2]);
     if (w != 0) return;
     constexpr int NW = SR_THREADS / 32;
     t = warp_sum(lane < NW ? part[0][lane] : 0.0);
     tm = warp_sum(lane < NW ? part[1][lane] : 0.0);
-    s = warp_sum(lane < NW ? part[2][lane] : 0.0);
     if (lane != 0) return;
     double *o = rep_out + 8 * r;
     const double u_pp = sums.u_pp_part ? 0.5 * t : o[RO_UPP];
@@ -324,11 +373,7 @@ k_step_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
     const double U = R.uf * (u_pp + u_pm + u_self);
     const double K = R.kf * s;
     const double T = K / R.kf / (double)R.n;
-    double fact = 1.0;
-    if (mode == 1) {
-        // thermostat_p3m_ord6.py:15-23
-        fact = (it <= 1999) ? sqrt(R.t_desired / T) : sqrt((20.0 * R.t_desired / T - 1.0) / 20.0);
-    }
+    const double fact = mode == 1 ? thermostat_factor(R, s, it) : 1.0;
     if (!isfinite(U)) raise_status(status, ST_NONFINITE);
     o[RO_UPP] = u_pp;
     o[RO_UPM] = u_pm;
@@ -784,10 +829,15 @@ static FinishArgs finish_args(const DevState &s)
     return A;
 }
 
-template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st)
+template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st)
 {
-    auto kern = rescale ? k_kick_drift<T, true> : k_kick_drift<T, false>;
-    kern<<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.vel, s.acc, s.ntot, s.rep_out, drift_args(s));
+    k_kick_drift<T><<<pgrid(s.ntot), 256, 0, st>>>(s.reps, s.prep, s.vel, s.acc, s.ntot, drift_args(s));
+}
+
+template <typename T> void launch_rescale_drift(const DevState &s, const int *counters, cudaStream_t st)
+{
+    k_rescale_drift<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, s.nblk, s.vel, s.acc, s.kin_part,
+                                                counters + 7, drift_args(s));
 }
 
 void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
@@ -796,9 +846,11 @@ void launch_set_flags(int *flag, int n, int value, cudaStream_t st)
 }
 
 template <typename T>
-void launch_kick_finish(const DevState &s, int do_kick, double *ep_out, cudaStream_t st)
+void launch_kick_finish(const DevState &s, int do_kick, double *ep_out, cudaStream_t st, int *counters)
 {
-    k_kick_finish<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, finish_args(s), s.acc, do_kick, ep_out);
+    FinishArgs A = finish_args(s);
+    A.counters = counters;
+    k_kick_finish<T><<<s.nblk, PBLK, 0, st>>>(s.reps, s.nrep, A, s.acc, do_kick, ep_out);
 }
 
 template <typename T> void launch_finish_drift(const DevState &s, const DevState &next, cudaStream_t st)
@@ -874,8 +926,9 @@ void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double
 int gf_opt_blocks(int M) { return (int)((gf_triples(M) + GF_TRIPLES - 1) / GF_TRIPLES); }
 
 #define P3M_INST(T)                                                                             \
-    template void launch_kick_drift<T>(const DevState &, bool, cudaStream_t);                    \
-    template void launch_kick_finish<T>(const DevState &, int, double *, cudaStream_t);          \
+    template void launch_kick_drift<T>(const DevState &, cudaStream_t);                          \
+    template void launch_rescale_drift<T>(const DevState &, const int *, cudaStream_t);          \
+    template void launch_kick_finish<T>(const DevState &, int, double *, cudaStream_t, int *);   \
     template void launch_finish_drift<T>(const DevState &, const DevState &, cudaStream_t);      \
     template void launch_nqt<T>(const DevState &, const double *, const double *, int, int,      \
                                 double *, double *, const int *, int, cudaStream_t);            \

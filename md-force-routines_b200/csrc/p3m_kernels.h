@@ -120,10 +120,12 @@ template <typename T> void launch_efield_from_mesh(const DevState &s, int rep,
 void launch_gf_opt(double kappa, double alpha, int p, int m_alias, int M, double L,
                    double *G_k, double *a_part, cudaStream_t st);
 
-// rescale: the velocities still lack the last step's thermostat factor
-template <typename T> void launch_kick_drift(const DevState &s, bool rescale, cudaStream_t st);
+template <typename T> void launch_kick_drift(const DevState &s, cudaStream_t st);
+// counters: the step's index goes to counters[7], for launch_rescale_drift
 template <typename T> void launch_kick_finish(const DevState &s, int do_kick, double *ep_out,
-                                              cudaStream_t st);
+                                              cudaStream_t st, int *counters = nullptr);
+// the drift when the velocities still lack the last step's thermostat factor
+template <typename T> void launch_rescale_drift(const DevState &s, const int *counters, cudaStream_t st);
 // The end of a step and the drift of the next, whose flags are next's.
 template <typename T> void launch_finish_drift(const DevState &s, const DevState &next, cudaStream_t st);
 // Sums that k_step_reduce can take over from k_reduce_pp, k_reduce_pm and
