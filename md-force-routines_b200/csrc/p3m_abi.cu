@@ -1,9 +1,12 @@
 // C ABI of libp3m_b200: contexts, device buffers, the compat entry points that
 // mirror the reference's Python functions, and the device-resident stepper.
+#include <algorithm>
+#include <array>
 #include <cmath>
 #include <complex>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -260,27 +263,32 @@ static double build_pp_table64(const p3m_replica_desc &d, int N, double limit, d
     return worst;
 }
 
-// FP64 pair tables of all replicas with one interval count, the smallest that
-// keeps every replica's error within 4e-16 (a few units in the last place of
-// psi(0) = 1: below the rounding of the pair sums); 0 intervals when none
-// does. Replicas of equal parameters share the work.
-static int build_pp_tables64(const p3m_replica_desc *reps, int n_reps, std::vector<double2> &tab)
+// FP64 pair tables: each replica's with the smallest interval count that keeps
+// its error within 4e-16 (a few units in the last place of psi(0) = 1: below the
+// rounding of the pair sums), none where no count does -- by its own parameters
+// alone, so that a replica's terms do not depend on its batch. Replicas of equal
+// parameters share a table.
+static void build_pp_tables64(p3m_ctx *ctx, std::vector<double2> &tab)
 {
-    for (int N = 128; N <= PP64_MAX_N; N *= 2) {
-        tab.assign((size_t)n_reps * N * 4, make_double2(0.0, 0.0));
-        bool ok = true;
-        for (int r = 0; r < n_reps && ok; ++r) {
-            double2 *out = tab.data() + (size_t)r * N * 4;
-            int same = -1;
-            for (int q = 0; q < r && same < 0; ++q)
-                if (reps[q].kappa == reps[r].kappa && reps[q].alpha == reps[r].alpha && reps[q].rc == reps[r].rc) same = q;
-            if (same >= 0) memcpy(out, tab.data() + (size_t)same * N * 4, sizeof(double2) * N * 4);
-            else ok = build_pp_table64(reps[r], N, 4e-16, out) <= 4e-16;
+    DevState &s = ctx->s;
+    std::map<std::array<double, 3>, int> first;  // parameters -> replica
+    std::vector<double2> one((size_t)PP64_MAX_N * 4);
+    for (int r = 0; r < ctx->nrep; ++r) {
+        const p3m_replica_desc &d = ctx->desc[r];
+        RepDev &R = ctx->rh[r];
+        const auto seen = first.emplace(std::array<double, 3>{d.kappa, d.alpha, d.rc}, r);
+        if (!seen.second) {
+            R.pp64_n = ctx->rh[seen.first->second].pp64_n;
+            R.pp64_off = ctx->rh[seen.first->second].pp64_off;
+        } else {
+            for (int N = 128; N <= PP64_MAX_N && R.pp64_n == 0; N *= 2)
+                if (build_pp_table64(d, N, 4e-16, one.data()) <= 4e-16) R.pp64_n = N;
+            R.pp64_off = (long long)tab.size();
+            tab.insert(tab.end(), one.begin(), one.begin() + (size_t)R.pp64_n * 4);
         }
-        if (ok) return N;
+        s.pp64_max = std::max(s.pp64_max, R.pp64_n);
+        if (R.pp64_n == 0) ++s.pp64_direct;
     }
-    tab.clear();
-    return 0;
 }
 
 // Work items of the mesh passes of every replica: x-pass items, and either
@@ -591,6 +599,8 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     CKC(cudaEventCreateWithFlags(&ctx->ev_fin, cudaEventDisableTiming));
     CKC(cudaEventCreateWithFlags(&ctx->ev_red, cudaEventDisableTiming));
     CKC(cudaEventCreateWithFlags(&ctx->ev_asg, cudaEventDisableTiming));
+    std::vector<double2> tab64;
+    if (precision == P3M_FP64) build_pp_tables64(ctx, tab64);
     CKC(dalloc(&s.reps, n_reps));
     CKC(cudaMemcpy(s.reps, ctx->rh.data(), sizeof(RepDev) * n_reps, cudaMemcpyHostToDevice));
     {
@@ -599,13 +609,9 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
         CKC(dalloc(&s.pp_tables, tab.size()));
         CKC(cudaMemcpy(s.pp_tables, tab.data(), sizeof(float4) * tab.size(), cudaMemcpyHostToDevice));
     }
-    if (precision == P3M_FP64) {
-        std::vector<double2> tab;
-        s.pp64_n = build_pp_tables64(reps, n_reps, tab);
-        if (s.pp64_n > 0) {
-            CKC(dalloc(&s.pp_tables64, tab.size()));
-            CKC(cudaMemcpy(s.pp_tables64, tab.data(), sizeof(double2) * tab.size(), cudaMemcpyHostToDevice));
-        }
+    if (!tab64.empty()) {
+        CKC(dalloc(&s.pp_tables64, tab64.size()));
+        CKC(cudaMemcpy(s.pp_tables64, tab64.data(), sizeof(double2) * tab64.size(), cudaMemcpyHostToDevice));
     }
     CKC(dalloc(&s.pos, (size_t)3 * p));
     CKC(dalloc(&s.vel, (size_t)3 * p));
@@ -709,7 +715,7 @@ template <typename T> static void seq_pp(p3m_ctx *ctx, bool reduce = true, cudaS
 {
     if (!st) st = ctx->st;
     launch_pp<T>(ctx->s, st);
-    ctx->launches++;
+    ctx->launches += pp_kernel_count(ctx->s);
     if (reduce) {
         launch_reduce_pp(ctx->s, st);
         ctx->launches++;
@@ -888,7 +894,7 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more
     if (e == cudaSuccess && pairs_wait) e = cudaStreamWaitEvent(st, ctx->ev_asg, 0);
     if (e == cudaSuccess && sums_free) e = cudaStreamWaitEvent(st, sums_free, 0);
     launch_pp<T>(s, st);
-    ctx->launches++;
+    ctx->launches += pp_kernel_count(s);
     if (e == cudaSuccess && s.has_mesh) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
     if (e == cudaSuccess && rec) e = cudaStreamWaitEvent(st, ctx->ev_join3, 0);
     if (more && fuse) launch_finish_drift<T>(s, next, st);

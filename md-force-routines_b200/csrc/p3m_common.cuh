@@ -58,8 +58,8 @@ enum : int {
 #endif
 constexpr int PP_TABLE_N = P3M_PP_TABLE_N;  // FP32 pair table: cubic intervals on [0, rc]
 
-// Intervals of the FP64 pair table (degree-7 polynomials, 64 bytes each): the
-// smallest count that meets its error bound, 128 .. PP64_MAX_N.
+// Intervals of a replica's FP64 pair table (degree-7 polynomials, 64 bytes each):
+// the smallest count that meets its error bound, 128 .. PP64_MAX_N.
 constexpr int PP64_MAX_N = 512;
 
 // Per-replica constants. Offsets index the concatenated device arrays.
@@ -79,6 +79,8 @@ struct RepDev {
     int blk_off;           // offset of this replica's particle blocks (PBLK each)
     int pp_blk_off;        // offset of this replica's blocks in the PP force kernel
     int nq_blk_off;        // offset of this replica's blocks in the n(q,t) kernel
+    int pp64_n;            // intervals of its FP64 pair table (0: pair terms evaluated directly)
+    long long pp64_off;    // first coefficient pair of that table
     double L, kappa, alpha, rc, cellw, h, dt, t_desired, af, uf, kf;
     double skin, rcl;      // Verlet skin and list cutoff rc + skin
     double pbuf;           // inner-list buffer: the pair kernel reads the outer-list entries

@@ -55,8 +55,9 @@ struct DevState {
     double *pos_pref = nullptr;  // positions at the last inner-list build (ntot,3)
     double *prune_count = nullptr;  // per replica: inner-list builds between outer rebuilds
     float4 *pp_tables = nullptr; // FP32 pair tables: cubic of psi = phi r, [nrep][PP_TABLE_N]
-    double2 *pp_tables64 = nullptr;  // FP64 path: [nrep][4][pp64_n] coefficient pairs
-    int pp64_n = 0;              // intervals of the FP64 tables (0: pair terms evaluated directly)
+    double2 *pp_tables64 = nullptr;  // FP64 path: per table [4][intervals] coefficient pairs
+    int pp64_max = 0;            // intervals of the largest FP64 table (0: no replica has one)
+    int pp64_direct = 0;         // replicas without an FP64 table
     void *acc_pp = nullptr;      // V4<T> PP acceleration, cell-sorted order
     // brick sort
     int *brick_key = nullptr, *brick_rank = nullptr;  // per particle: brick, arrival rank in it
@@ -97,6 +98,8 @@ template <typename T> void launch_fix_cells(const DevState &s, cudaStream_t st);
 template <typename T> int launch_place_bricks(const DevState &s, cudaStream_t st);  // kernels launched
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st);
 template <typename T> void launch_pp(const DevState &s, cudaStream_t st);
+// kernels launch_pp launches: two for an FP64 batch with and without pair tables
+inline int pp_kernel_count(const DevState &s) { return s.pp64_max > 0 && s.pp64_direct > 0 ? 2 : 1; }
 int pp_particles_per_block(int tpi);
 void launch_reduce_pp(const DevState &s, cudaStream_t st);
 

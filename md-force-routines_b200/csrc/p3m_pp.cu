@@ -34,10 +34,10 @@
 // F/r = g/r^3 and phi = psi/r -- one table read per pair, and a force that is
 // exactly minus the gradient of the interpolated potential. FP32: cubics from
 // FP64 values. FP64: polynomials of degree 7 from extended-precision values,
-// with as many intervals as keep psi and g within a few 1e-16 of psi(0) = 1;
-// where the largest table does not reach that (very steep pair functions),
-// the reference's formula is evaluated directly, written with the shared
-// Gaussian factor
+// with as many intervals as keep psi and g within a few 1e-16 of psi(0) = 1,
+// each replica by itself, whatever its batch; for a replica whose largest
+// table does not reach that (a very steep pair function), the reference's
+// formula is evaluated directly, written with the shared Gaussian factor
 //   e^{+-kr} erfc(u+-) = erfcx(u+-) exp(-(a^2 r^2 + k^2/4a^2)),  u+- = ar +- k/2a,
 // using CUDA's exp and erfcx.
 #include "p3m_kernels.h"
@@ -328,8 +328,10 @@ __device__ __forceinline__ void pair_table64(double r2, double inv_h, int N, con
 }
 
 // FP64 forces from the lists: TPI threads per particle, Kahan-compensated
-// sums. TAB: pair terms from the table (tab_n intervals), branch-free, so the
-// loads and the dependent chains of a pass overlap; otherwise pair_direct.
+// sums. TAB: pair terms from the replica's table, branch-free, so the loads and
+// the dependent chains of a pass overlap; otherwise pair_direct. The blocks of
+// replicas of the other kind return at once (a batch with both is two
+// launches), so that neither kind pays for the other's registers.
 //
 // Bound: the table and coordinate reads through L1 (96 bytes a pair), then
 // the FP64 pipe; pair_direct's exp and two erfcx, some 250 FP64 instructions
@@ -339,7 +341,7 @@ template <int TPI, bool TAB>
 __global__ void __launch_bounds__(PPL_THREADS)
 k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict__ xq,
          const int *__restrict__ nnb, const int *__restrict__ nlist, int maxnb,
-         const double2 *__restrict__ tables, int tab_n, double4 *__restrict__ acc_out,
+         const double2 *__restrict__ tables, double4 *__restrict__ acc_out,
          double *__restrict__ u_part)
 {
     using T = double;
@@ -351,8 +353,10 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
     const int b = blockIdx.x;
     const int r = find_rep(b, nrep, [&](int k) { return reps[k].pp_blk_off; });
     const RepDev &R = reps[r];
+    const int tab_n = R.pp64_n;
+    if ((tab_n > 0) != TAB) return;  // block-uniform
     if constexpr (TAB) {
-        const double2 *src = tables + (long long)r * tab_n * 4;
+        const double2 *src = tables + R.pp64_off;
         for (int k = threadIdx.x; k < tab_n * 4; k += PPL_THREADS) cp_async16(ppl_tab64 + k, src + k);
         cp_async_wait_all();
         __syncthreads();
@@ -877,13 +881,13 @@ template <typename T, int TPI> static void launch_pp_tpi(const DevState &s, cuda
             s.reps, s.nrep, (const uint4 *)s.xq, s.nnb, s.nlist, s.maxnb, s.pp_tables,
             (float4 *)s.acc_pp, s.u_pp_part, pa);
     } else {
-        if (s.pp64_n > 0)
-            k_pp_f64<TPI, true><<<s.pp_nblk, PPL_THREADS, s.pp64_n * 4 * sizeof(double2), st>>>(
-                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, s.pp_tables64, s.pp64_n,
+        if (s.pp64_max > 0)
+            k_pp_f64<TPI, true><<<s.pp_nblk, PPL_THREADS, s.pp64_max * 4 * sizeof(double2), st>>>(
+                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, s.pp_tables64,
                 (double4 *)s.acc_pp, s.u_pp_part);
-        else
+        if (s.pp64_direct > 0)
             k_pp_f64<TPI, false><<<s.pp_nblk, PPL_THREADS, 0, st>>>(
-                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, nullptr, 0,
+                s.reps, s.nrep, (const Q *)s.xq, s.nnb, s.nlist, s.maxnb, nullptr,
                 (double4 *)s.acc_pp, s.u_pp_part);
     }
 }
