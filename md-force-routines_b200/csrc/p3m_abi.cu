@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "p3m_kernels.h"
+#include "p3m_pp_table.h"
 
 using namespace p3m;
 
@@ -212,62 +213,10 @@ static void build_pp_table(const p3m_replica_desc &d, float4 *out)
     }
 }
 
-// psi(r) and g(r) in extended precision, from the same expressions.
-static void pair_g_psi_l(long double r, long double k, long double a, long double *g, long double *psi)
-{
-    const long double up = a * r + 0.5L * k / a, um = a * r - 0.5L * k / a;
-    const long double ep = expl(k * r) * erfcl(up), em = expl(-k * r) * erfcl(um);
-    const long double gauss = expl(-a * a * r * r - 0.25L * k * k / (a * a));
-    *psi = 0.5L * (ep + em);
-    *g = 0.5L * (ep * (1.0L - k * r) + em * (1.0L + k * r)) +
-         2.0L * a * r * gauss / sqrtl(3.141592653589793238462643383279502884L);
-}
-
-// FP64 pair table of one replica with N intervals: psi on interval i as a
-// degree-7 polynomial in u in [-1/2, 1/2] about its middle, through eight
-// Chebyshev points (Newton's divided differences, expanded); out[k * N + i] =
-// coefficients 2k, 2k + 1. Returns the largest error of psi and of g = psi - r
-// psi' (as the kernel forms them) at points between the nodes, in units of
-// psi(0) = 1; stops early once it exceeds `limit`. Nodes are in extended
-// precision: psi' divides their noise by the interval width.
-static double build_pp_table64(const p3m_replica_desc &d, int N, double limit, double2 *out)
-{
-    constexpr int K = 8;
-    const long double h = (long double)d.rc / N;
-    long double x[K];
-    for (int j = 0; j < K; ++j) x[j] = 0.5L * cosl((2 * j + 1) * 3.141592653589793238462643383279502884L / (2 * K));
-    double worst = 0.0;
-    for (int i = 0; i < N; ++i) {
-        long double f[K], g, c[K] = {0};
-        for (int j = 0; j < K; ++j) pair_g_psi_l((i + 0.5L + x[j]) * h, d.kappa, d.alpha, &g, &f[j]);
-        for (int m = 1; m < K; ++m)
-            for (int j = K - 1; j >= m; --j) f[j] = (f[j] - f[j - 1]) / (x[j] - x[j - m]);
-        for (int m = K - 1; m >= 0; --m) {  // c = c (u - x[m]) + f[m]
-            for (int j = K - 1; j > 0; --j) c[j] = c[j - 1] - x[m] * c[j];
-            c[0] = f[m] - x[m] * c[0];
-        }
-        for (int k = 0; k < K / 2; ++k) out[k * N + i] = make_double2((double)c[2 * k], (double)c[2 * k + 1]);
-        for (int j = 0; j < 3; ++j) {  // the ends and the middle
-            const long double u = 0.5L * (j - 1), t = i + 0.5L + u;
-            long double p = 0.0L, dp = 0.0L, gt, pt;
-            for (int k = K - 1; k >= 0; --k) {
-                dp = dp * u + p;
-                p = p * u + (k % 2 ? out[k / 2 * N + i].y : out[k / 2 * N + i].x);
-            }
-            pair_g_psi_l(t * h, d.kappa, d.alpha, &gt, &pt);
-            const double e = (double)fmaxl(fabsl(p - pt), fabsl(p - t * dp - gt));
-            if (!(e <= limit)) return 1.0;
-            worst = fmax(worst, e);
-        }
-    }
-    return worst;
-}
-
-// FP64 pair tables: each replica's with the smallest interval count that keeps
-// its error within 4e-16 (a few units in the last place of psi(0) = 1: below the
-// rounding of the pair sums), none where no count does -- by its own parameters
-// alone, so that a replica's terms do not depend on its batch. Replicas of equal
-// parameters share a table.
+// FP64 pair tables: each replica's with the smallest interval count that meets
+// PP64_LIMIT, none where no count does -- by its own parameters alone, so that a
+// replica's terms do not depend on its batch. Replicas of equal parameters share
+// a table.
 static void build_pp_tables64(p3m_ctx *ctx, std::vector<double2> &tab)
 {
     DevState &s = ctx->s;
@@ -281,8 +230,8 @@ static void build_pp_tables64(p3m_ctx *ctx, std::vector<double2> &tab)
             R.pp64_n = ctx->rh[seen.first->second].pp64_n;
             R.pp64_off = ctx->rh[seen.first->second].pp64_off;
         } else {
-            for (int N = 128; N <= PP64_MAX_N && R.pp64_n == 0; N *= 2)
-                if (build_pp_table64(d, N, 4e-16, one.data()) <= 4e-16) R.pp64_n = N;
+            for (int N = PP64_MIN_N; N <= PP64_MAX_N && R.pp64_n == 0; N *= 2)
+                if (build_pp_table64(d.kappa, d.alpha, d.rc, N, PP64_LIMIT, &one[0].x) <= PP64_LIMIT) R.pp64_n = N;
             R.pp64_off = (long long)tab.size();
             tab.insert(tab.end(), one.begin(), one.begin() + (size_t)R.pp64_n * 4);
         }

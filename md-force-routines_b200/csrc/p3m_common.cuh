@@ -58,10 +58,6 @@ enum : int {
 #endif
 constexpr int PP_TABLE_N = P3M_PP_TABLE_N;  // FP32 pair table: cubic intervals on [0, rc]
 
-// Intervals of a replica's FP64 pair table (degree-7 polynomials, 64 bytes each):
-// the smallest count that meets its error bound, 128 .. PP64_MAX_N.
-constexpr int PP64_MAX_N = 512;
-
 // Per-replica constants. Offsets index the concatenated device arrays.
 struct RepDev {
     int n, p_off;          // particles, offset into particle arrays

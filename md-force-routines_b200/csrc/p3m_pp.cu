@@ -33,14 +33,15 @@
 //   g(r) = F(r) r^2 = -r^2 d(psi/r)/dr = psi - r psi',
 // F/r = g/r^3 and phi = psi/r -- one table read per pair, and a force that is
 // exactly minus the gradient of the interpolated potential. FP32: cubics from
-// FP64 values. FP64: polynomials of degree 7 from extended-precision values,
-// with as many intervals as keep psi and g within a few 1e-16 of psi(0) = 1,
-// each replica by itself, whatever its batch; for a replica whose largest
+// FP64 values. FP64: polynomials of degree 7 from extended-precision values
+// (p3m_pp_table.h), with as many intervals as keep psi and g within 4e-16 of
+// themselves, each replica by itself, whatever its batch; for one whose largest
 // table does not reach that (a very steep pair function), the reference's
 // formula is evaluated directly, written with the shared Gaussian factor
 //   e^{+-kr} erfc(u+-) = erfcx(u+-) exp(-(a^2 r^2 + k^2/4a^2)),  u+- = ar +- k/2a,
 // using CUDA's exp and erfcx.
 #include "p3m_kernels.h"
+#include "p3m_pp_table.h"
 
 namespace p3m {
 
@@ -305,15 +306,18 @@ constexpr int PPL_THREADS = 256;
 // FP64 pair terms of one entry from the table: tab[k * N + i] holds the
 // coefficients 2k, 2k + 1 of interval i (u in [-1/2, 1/2) about its middle),
 // so the 16-byte reads of a warp's lanes fall on random bank groups. Value and
-// derivative by one Horner recurrence; t = r / h, and g = p - t dp/du. The
-// caller passes r2 in (0, rc^2) (or rc^2, masked).
-__device__ __forceinline__ void pair_table64(double r2, double inv_h, int N, const double2 *tab,
-                                             double &f_over_r, double &phi)
+// derivative by one Horner recurrence; t = r / h, and g = p - t dp/du. Near the
+// cutoff psi falls by some 2 (alpha rc)^2 times r's relative change, so u is
+// formed without r's rounding: dr, what r misses of the root, and 1/h in two
+// parts. The caller passes r2 in (0, rc^2) (or rc^2, masked).
+__device__ __forceinline__ void pair_table64(double r2, double inv_h, double inv_h_lo, int N,
+                                             const double2 *tab, double &f_over_r, double &phi)
 {
     const double rinv = rsqrt(r2);
-    const double t = r2 * rinv * inv_h;
+    const double r = r2 * rinv, dr = 0.5 * rinv * fma(-r, r, r2);
+    const double t = r * inv_h;
     const int i = min((int)t, N - 1);
-    const double u = t - ((double)i + 0.5);
+    const double u = fma(r, inv_h, -((double)i + 0.5)) + fma(dr, inv_h, r * inv_h_lo);
     const double2 c67 = tab[3 * N + i], c45 = tab[2 * N + i], c23 = tab[N + i], c01 = tab[i];
     double p = c67.y, d = c67.y;
     p = fma(p, u, c67.x);
@@ -335,8 +339,9 @@ __device__ __forceinline__ void pair_table64(double r2, double inv_h, int N, con
 //
 // Bound: the table and coordinate reads through L1 (96 bytes a pair), then
 // the FP64 pipe; pair_direct's exp and two erfcx, some 250 FP64 instructions
-// a pair, bound it there before (1e4 particles, rc 5.9: 162 -> 51 us with two
-// lanes per particle, 84 -> 35 with eight; 1e5: 531 -> 218 with eight).
+// a pair, bound it there (1e4 particles, rc 6, direct / table: 164 / 52 us with
+// two lanes per particle, 91 / 43 with eight, where the 32 KB table is staged for
+// a quarter of the particles).
 template <int TPI, bool TAB>
 __global__ void __launch_bounds__(PPL_THREADS)
 k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict__ xq,
@@ -368,7 +373,7 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
     const double scd = R.L / Coord<T>::scale;
     const T sc = (T)scd, sc_lo = (T)(scd - (double)sc);
     const T rc2 = (T)(R.rc * R.rc);
-    const T inv_h = (T)(tab_n / R.rc);
+    const T inv_h = tab_n / R.rc, inv_h_lo = -fma(inv_h, R.rc, (double)-tab_n) / R.rc;
 
     T fx = 0, fy = 0, fz = 0, gx = 0, gy = 0, gz = 0;
     double u = 0.0;
@@ -412,7 +417,7 @@ k_pp_f64(const RepDev *__restrict__ reps, int nrep, const ulonglong4 *__restrict
                     const bool in = r2 < rc2 && r2 > (T)0;
                     if constexpr (TAB) {
                         T fr, ph;
-                        pair_table64(in ? r2 : rc2, inv_h, tab_n, ppl_tab64, fr, ph);
+                        pair_table64(in ? r2 : rc2, inv_h, inv_h_lo, tab_n, ppl_tab64, fr, ph);
                         fr = in ? fr : (T)0;
                         px += fr * dx;
                         py += fr * dy;
@@ -836,9 +841,12 @@ template <typename T> void configure_pp_kernels()
         set(k_pp_f32<4, PP_OUTER>); set(k_pp_f32<8, PP_OUTER>);
         set(k_pp_f32<1, PP_DYN>); set(k_pp_f32<2, PP_DYN>);
         set(k_pp_f32<4, PP_DYN>); set(k_pp_f32<8, PP_DYN>);
+    } else {
+        const int tab = (int)(PP64_MAX_N * PP64_COEF * sizeof(double));
+        auto set = [&](auto k) { cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tab); };
+        set(k_pp_f64<1, true>); set(k_pp_f64<2, true>);
+        set(k_pp_f64<4, true>); set(k_pp_f64<8, true>);
     }
-    // (the FP64 table, at most PP64_MAX_N intervals of 64 bytes, fits the default limit)
-    static_assert(PP64_MAX_N * 4 * sizeof(double2) <= 48 * 1024 - 1024, "FP64 table size");
 }
 
 template <typename T> void launch_build_lists(const DevState &s, cudaStream_t st)
