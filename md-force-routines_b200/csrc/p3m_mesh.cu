@@ -708,6 +708,10 @@ k_fft_z_green(const RepDev *__restrict__ reps, int nrep, const cplx<T> *__restri
 // registers between passes. Rows are M + 1 apart: lanes along z or along a row
 // fall on different banks; where lanes go along y to meet global memory, the
 // rows of a half warp are plane_row()'s, spaced to do the same.
+// The energy is summed by 32 consecutive tasks and then over those sums, the same
+// tree for either block size: a replica's energy does not depend on whether its
+// batch's planes share SMs (tests/test_gpu_batch_planes.py holds that for the
+// fields too).
 constexpr int PLANE_MAX = 64;
 
 __device__ __forceinline__ int plane_row(int g) { return ((g & 1) << 3) | ((g >> 1) & 7) | (g & ~15); }
@@ -761,24 +765,27 @@ __device__ __forceinline__ void plane_item(const RepDev &R, int kx, const cplx<T
     // z, pass 2; U_f, phi, -i kz phi; their inverse z transforms, pass 1
     const double wkx = (kx == 0 || kx == (M >> 1)) ? 1.0 : 2.0;
     const T twopi_L = (T)(6.283185307179586477 * R.inv_L);
-    double u = 0.0;
     for (int e = threadIdx.x; e < M * RA; e += NT) {
         const int s = e % M, k1 = e / M, y = s / RB + RA * (s % RB);
         T g[RB];
 #pragma unroll
         for (int k2 = 0; k2 < RB; ++k2) g[k2] = __ldg(green + lbase + (k1 + RA * k2) * M + y);
         cplx<T> x[RB], f[RB];
+        double u = 0.0;
 #pragma unroll
         for (int n2 = 0; n2 < RB; ++n2) x[n2] = A[(k1 * RB + n2) * LD + s];
         dft<T, RB, false>(x);
 #pragma unroll
         for (int k2 = 0; k2 < RB; ++k2) {
             const int n = k1 + RA * k2;
-            u += wkx * (double)g[k2] * ((double)x[k2].x * x[k2].x + (double)x[k2].y * x[k2].y);
+            const double xr = (double)x[k2].x, xi = (double)x[k2].y;
+            u = fma(wkx * (double)g[k2], fma(xr, xr, mul_rn(xi, xi)), u);
             x[k2] = make_c<T>(g[k2] * x[k2].x, g[k2] * x[k2].y);
             const T kz = (n == (M >> 1)) ? (T)0 : twopi_L * (T)freq(n, M);
             f[k2] = make_c<T>(kz * x[k2].y, -kz * x[k2].x);  // -i kz phi
         }
+        u = warp_sum(u);  // of 32 consecutive e
+        if ((threadIdx.x & 31) == 0) red[e >> 5] = u;
         dft<T, RB, true>(x);
         dft<T, RB, true>(f);
 #pragma unroll
@@ -873,8 +880,11 @@ __device__ __forceinline__ void plane_item(const RepDev &R, int kx, const cplx<T
 #pragma unroll
         for (int i = 0; i < RA; ++i) ek[nspec + lbase + z * M + j + RB * i] = x[i];
     }
-    const double ut = block_sum(u, red);
-    if (threadIdx.x == 0) *u_out = ut;
+    if (threadIdx.x < 32) {
+        static_assert(M * RA <= 32 * 32, "one lane per sum");
+        const double ut = warp_sum(threadIdx.x < M * RA / 32 ? red[threadIdx.x] : 0.0);
+        if (threadIdx.x == 0) *u_out = ut;
+    }
 }
 
 template <typename T, int NT>
