@@ -201,11 +201,19 @@ __device__ __forceinline__ void weights6(T x, T *w)
 //
 // FP64, B = 62: t rounded to a 64-bit integer, added as its low word and --
 // with the carry of that add -- its high word; the number of carries does not
-// depend on the order either. A contribution is kept to 2^-62 of the bound on
-// a node sum (156 unit charges: 2^-57), finer than an FP64 sum's rounding.
-// Shared memory has no 64-bit add (a
+// depend on the order either. Shared memory has no 64-bit add (a
 // compare-and-swap loop: 33 us for the 64 bricks of 1e4 particles, against
 // 14 with the two words; the ordered FP64 sum it replaced took 34).
+// The step 1/S is absolute: 2^-62 of the bound on a node sum, 2^-57 of the
+// charge for 156 equal ones, on nodes they hardly reach too (where the weights
+// themselves, from offsets that round at 2^-53 of x / h, are no better than some
+// 2^-48 of the charge). So that small charges keep theirs beside large ones,
+// those of a brick are taken in classes, each within a factor of 2^CLASS_BITS
+// of its largest, with a step and a pass over the tile of its own; the classes'
+// nodes are added in FP64, the largest first. A brick of one class pays a
+// minimum beside its maximum (nothing measurable), every further class its pass:
+// 1e4 particles on 64^3 14, 27 and 39 us with one, two and three classes; the
+// ordered FP64 sum took 39 on the same box whatever the charges.
 //
 // Bound: the shared-memory atomics (a warp's add every two cycles; 1280
 // bricks of 157 particles 50 -> 42 us without the second pass over positions
@@ -215,6 +223,7 @@ __device__ __forceinline__ void weights6(T x, T *w)
 // particles whose stencils reach it, and writes its planes -- no sums between
 // CTAs.
 constexpr int A_THREADS = 256;
+constexpr int CLASS_BITS = 4;
 constexpr float kRound = 12582912.0f;  // 1.5 * 2^23
 constexpr int kRoundBits = 0x4B400000;
 
@@ -246,119 +255,140 @@ k_assign(const RepDev *__restrict__ reps, int nrep, const int *__restrict__ bric
         const RepDev &R = reps[r];
         const int local = b - R.brick_off;
         const int p0 = brick_start[b], n = brick_start[b + 1] - p0;
-        double qmax = R.qmax;
-        if constexpr (sizeof(T) == 8) {  // the brick's own largest |q|
-            qmax = 0.0;
-            for (int k = threadIdx.x; k < n; k += A_THREADS) qmax = fmax(qmax, fabs((double)slot_q[p0 + k]));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) qmax = fmax(qmax, __shfl_xor_sync(0xffffffffu, qmax, o));
-            __syncthreads();  // the previous item is done with a_qmax
-            if (lane == 0) a_qmax[threadIdx.x >> 5] = qmax;
-            __syncthreads();
-            for (int k = 0; k < A_THREADS / 32; ++k) qmax = fmax(qmax, a_qmax[k]);
-        }
-        // S = 2^k with 0.17 n qmax S <= 2^B, k = B - ceil(log2(0.17 n qmax))
-        const double bound = fmax(0.17 * (double)(n > 0 ? n : 1) * qmax, 1e-300);
-        const long long bits = __double_as_longlong(bound);
-        const int ceil2 = (int)(bits >> 52) - 1023 + ((bits & 0xFFFFFFFFFFFFFll) != 0 ? 1 : 0);
-        constexpr int B = sizeof(T) == 4 ? 22 : 62, KMAX = sizeof(T) == 4 ? 100 : 1000;
-        const int kexp = max(-KMAX, min(B - ceil2, KMAX));
-        const double Sd = __longlong_as_double((long long)(kexp + 1023) << 52);
-        const T S = (T)Sd;
-        const double inv = __longlong_as_double((long long)(1023 - kexp) << 52);  // 1 / S
-        const int fb = max(0, min(16, 30 - (32 - __clz(n))));  // n < 2^(32 - clz n)
-        const float F = (float)(1 << fb);
-        __syncthreads();
-        for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
-            thi[k] = 0;
-            tlo[k] = 0;
-        }
-        __syncthreads();
-        for (int c0 = p0; c0 < p0 + n; c0 += A_THREADS) {
-            // The lanes of a warp add at the same offsets from their
-            // particles' stencil bases: lanes whose bases share a shared-memory
-            // bank conflict on every atomic. The chunk's particles (of those
-            // that reach this item's planes) are ranked by bank and dealt
-            // round-robin to the warps. Integer sums do not depend on which
-            // thread adds what.
-            const int c = c0 + threadIdx.x;
-            int bank = 0, rank = 0;
-            bool use = false;
-            if (c < p0 + n) {
-                const int pb = unpack_base(slot_pt[c].w);  // -1: filed under brick 0 and flagged
-                const int lz = (pb >> 8) & 15;
-                use = pb >= 0 && (!SPLIT || (lz + HALO >= z0 && lz < z0 + np));
-                bank = (((lz * TILE + ((pb >> 4) & 15)) * TILE) + (pb & 15)) & 31;
-            }
-            __syncthreads();  // the previous chunk is done with a_src
-            a_src[threadIdx.x] = -1;
-            if (threadIdx.x < 32) a_cnt[threadIdx.x] = 0;
-            __syncthreads();
-            if (use) rank = atomicAdd(&a_cnt[bank], 1);
-            const int nch = __syncthreads_count(use);
-            if (threadIdx.x < 32) {  // exclusive scan of the bank counts
-                const int v = a_cnt[lane];
-                int x = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += t;
+        // classes of charges (FP64): |q| in (low, high], the first without a bound
+        double high = 1e308;
+        bool more = false, first = true;
+        do {
+            double qmax = R.qmax, qmin = 1e308, low = 0.0;
+            if constexpr (sizeof(T) == 8) {  // the class's largest |q|, and the thread's smallest left
+                qmax = 0.0;
+                for (int k = threadIdx.x; k < n; k += A_THREADS) {
+                    const double q = fabs((double)slot_q[p0 + k]);
+                    if (q > high) continue;  // an earlier class's
+                    qmax = fmax(qmax, q);
+                    if (q > 0.0) qmin = fmin(qmin, q);
                 }
-                a_cnt[lane] = x - v;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) qmax = fmax(qmax, __shfl_xor_sync(0xffffffffu, qmax, o));
+                __syncthreads();  // the previous item is done with a_qmax
+                if (lane == 0) a_qmax[threadIdx.x >> 5] = qmax;
+                __syncthreads();
+                for (int k = 0; k < A_THREADS / 32; ++k) qmax = fmax(qmax, a_qmax[k]);
+                low = qmax * (1.0 / (1 << CLASS_BITS));
+            }
+            // S = 2^k with 0.17 n qmax S <= 2^B, k = B - ceil(log2(0.17 n qmax))
+            const double bound = fmax(0.17 * (double)(n > 0 ? n : 1) * qmax, 1e-300);
+            const long long bits = __double_as_longlong(bound);
+            const int ceil2 = (int)(bits >> 52) - 1023 + ((bits & 0xFFFFFFFFFFFFFll) != 0 ? 1 : 0);
+            constexpr int B = sizeof(T) == 4 ? 22 : 62, KMAX = sizeof(T) == 4 ? 100 : 1000;
+            const int kexp = max(-KMAX, min(B - ceil2, KMAX));
+            const double Sd = __longlong_as_double((long long)(kexp + 1023) << 52);
+            const T S = (T)Sd;
+            const double inv = __longlong_as_double((long long)(1023 - kexp) << 52);  // 1 / S
+            const int fb = max(0, min(16, 30 - (32 - __clz(n))));  // n < 2^(32 - clz n)
+            const float F = (float)(1 << fb);
+            // (the previous pass is done with the tile)
+            if constexpr (sizeof(T) == 8) more = __syncthreads_or(qmin <= low);
+            else __syncthreads();
+            for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
+                thi[k] = 0;
+                tlo[k] = 0;
             }
             __syncthreads();
-            if (use) {
-                const int q = a_cnt[bank] + rank, nw = (nch + 31) >> 5;
-                a_src[(q % nw) * 32 + q / nw] = c;
-            }
-            __syncthreads();
-            const int p = a_src[threadIdx.x];
-            if (p < 0) continue;
-            const typename V4<T>::t v = slot_pt[p];
-            const int pb = unpack_base(v.w), lz = pb >> 8;
-            T wx[6], wy[6], wz[6];
-            weights6<T>(v.x, wx);
-            weights6<T>(v.y, wy);
-            weights6<T>(v.z, wz);
-            const T qs = slot_q[p] * S;
-            const int base = ((lz - z0) * TILE + ((pb >> 4) & 15)) * TILE + (pb & 15);
+            for (int c0 = p0; c0 < p0 + n; c0 += A_THREADS) {
+                // The lanes of a warp add at the same offsets from their
+                // particles' stencil bases: lanes whose bases share a shared-memory
+                // bank conflict on every atomic. The chunk's particles (of those
+                // that reach this item's planes) are ranked by bank and dealt
+                // round-robin to the warps. Integer sums do not depend on which
+                // thread adds what.
+                const int c = c0 + threadIdx.x;
+                int bank = 0, rank = 0;
+                bool use = false;
+                if (c < p0 + n) {
+                    const int pb = unpack_base(slot_pt[c].w);  // -1: filed under brick 0 and flagged
+                    const int lz = (pb >> 8) & 15;
+                    use = pb >= 0 && (!SPLIT || (lz + HALO >= z0 && lz < z0 + np));
+                    if (sizeof(T) == 8 && (more || !first)) {
+                        const double q = fabs((double)slot_q[c]);
+                        use = use && q > low && q <= high;
+                    }
+                    bank = (((lz * TILE + ((pb >> 4) & 15)) * TILE) + (pb & 15)) & 31;
+                }
+                __syncthreads();  // the previous chunk is done with a_src
+                a_src[threadIdx.x] = -1;
+                if (threadIdx.x < 32) a_cnt[threadIdx.x] = 0;
+                __syncthreads();
+                if (use) rank = atomicAdd(&a_cnt[bank], 1);
+                const int nch = __syncthreads_count(use);
+                if (threadIdx.x < 32) {  // exclusive scan of the bank counts
+                    const int v = a_cnt[lane];
+                    int x = v;
 #pragma unroll
-            for (int g = 0; g < 6; ++g) {
-                if (SPLIT && (unsigned)(lz + g - z0) >= (unsigned)np) continue;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(0xffffffffu, x, o);
+                        if (lane >= o) x += t;
+                    }
+                    a_cnt[lane] = x - v;
+                }
+                __syncthreads();
+                if (use) {
+                    const int q = a_cnt[bank] + rank, nw = (nch + 31) >> 5;
+                    a_src[(q % nw) * 32 + q / nw] = c;
+                }
+                __syncthreads();
+                const int p = a_src[threadIdx.x];
+                if (p < 0) continue;
+                const typename V4<T>::t v = slot_pt[p];
+                const int pb = unpack_base(v.w), lz = pb >> 8;
+                T wx[6], wy[6], wz[6];
+                weights6<T>(v.x, wx);
+                weights6<T>(v.y, wy);
+                weights6<T>(v.z, wz);
+                const T qs = slot_q[p] * S;
+                const int base = ((lz - z0) * TILE + ((pb >> 4) & 15)) * TILE + (pb & 15);
 #pragma unroll
-                for (int a = 0; a < 6; ++a) {
-                    const T qzy = qs * wz[g] * wy[a];
-                    const int row = base + (g * TILE + a) * TILE;
+                for (int g = 0; g < 6; ++g) {
+                    if (SPLIT && (unsigned)(lz + g - z0) >= (unsigned)np) continue;
 #pragma unroll
-                    for (int cx = 0; cx < 6; ++cx) {
-                        const T t = mul_rn(qzy, wx[cx]);
-                        if constexpr (sizeof(T) == 4) {
-                            const float hb = (t - 0.5f) + kRound;    // floor(t), as a float
-                            const int hi = __float_as_int(hb) - kRoundBits;
-                            const float frac = t - (hb - kRound);      // in [0, 1], exact
-                            const int lo = __float_as_int(frac * F + kRound) - kRoundBits;
-                            atomicAdd(thi + row + cx, hi);
-                            atomicAdd(tlo + row + cx, lo);
-                        } else {
-                            const long long i = __double2ll_rn(t);
-                            const unsigned lo = (unsigned)i;
-                            const unsigned old = atomicAdd((unsigned *)tlo + row + cx, lo);
-                            atomicAdd(thi + row + cx, (int)(i >> 32) + (old + lo < lo ? 1 : 0));
+                    for (int a = 0; a < 6; ++a) {
+                        const T qzy = qs * wz[g] * wy[a];
+                        const int row = base + (g * TILE + a) * TILE;
+#pragma unroll
+                        for (int cx = 0; cx < 6; ++cx) {
+                            const T t = mul_rn(qzy, wx[cx]);
+                            if constexpr (sizeof(T) == 4) {
+                                const float hb = (t - 0.5f) + kRound;    // floor(t), as a float
+                                const int hi = __float_as_int(hb) - kRoundBits;
+                                const float frac = t - (hb - kRound);      // in [0, 1], exact
+                                const int lo = __float_as_int(frac * F + kRound) - kRoundBits;
+                                atomicAdd(thi + row + cx, hi);
+                                atomicAdd(tlo + row + cx, lo);
+                            } else {
+                                const long long i = __double2ll_rn(t);
+                                const unsigned lo = (unsigned)i;
+                                const unsigned old = atomicAdd((unsigned *)tlo + row + cx, lo);
+                                atomicAdd(thi + row + cx, (int)(i >> 32) + (old + lo < lo ? 1 : 0));
+                            }
                         }
                     }
                 }
             }
-        }
-        __syncthreads();
-        T *dst = tiles + R.tile_off + (long long)local * TILE3 + z0 * TILE * TILE;
-        // exact as integers, rounded once by the conversion
-        const T unit = sizeof(T) == 4 ? (T)(inv / (double)F) : (T)inv;
-        for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
-            if constexpr (sizeof(T) == 4)
-                dst[k] = (float)(((long long)thi[k] << fb) + tlo[k]) * unit;
-            else
-                dst[k] = (T)(((long long)thi[k] << 32) | (unsigned)tlo[k]) * unit;
-        }
+            __syncthreads();
+            T *dst = tiles + R.tile_off + (long long)local * TILE3 + z0 * TILE * TILE;
+            // exact as integers, rounded once by the conversion
+            const T unit = sizeof(T) == 4 ? (T)(inv / (double)F) : (T)inv;
+            for (int k = threadIdx.x; k < nnode; k += A_THREADS) {
+                if constexpr (sizeof(T) == 4)
+                    dst[k] = (float)(((long long)thi[k] << fb) + tlo[k]) * unit;
+                else {
+                    const T v = (T)(((long long)thi[k] << 32) | (unsigned)tlo[k]) * unit;
+                    dst[k] = first ? v : dst[k] + v;
+                }
+            }
+            high = low;
+            first = false;
+        } while (more);
     }
 }
 
