@@ -138,16 +138,31 @@ static cudaError_t valloc(void **p, size_t bytes)
 }
 
 // Scratch of one call, from the device's stream-ordered pool: several buffers
-// in one allocation on stream st, freed on it again. The runtime keeps a freed
-// block for the next call and returns it to the system at the program's next
-// synchronisation, so calls in a row do not pay for mapping memory (a
-// cudaMalloc / cudaFree pair: 0.6 ms each), and nothing is held by the library.
+// in one allocation on stream st, freed on it again. The pool keeps a freed block
+// for the next call until the program next synchronises, so calls in a row do not
+// pay for mapping memory (a cudaMalloc / cudaFree pair: 0.6 ms each). A caller with
+// a fixed memory budget must not find large blocks gone meanwhile: where the pool
+// holds more than kPoolKeep, the call waits for its (finished) stream, which
+// gives the freed blocks back to the system before it returns.
+static const unsigned long long kPoolKeep = 64ull << 20;
+
 struct CallScratch {
     cudaStream_t st;
     char *base = nullptr;
     size_t used = 0;
     explicit CallScratch(cudaStream_t s) : st(s) {}
-    ~CallScratch() { if (base) cudaFreeAsync(base, st); }
+    ~CallScratch()
+    {
+        if (!base) return;
+        cudaFreeAsync(base, st);
+        int dev = 0;
+        cudaMemPool_t pool;
+        unsigned long long held = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetMemPool(&pool, dev) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+            held > kPoolKeep)
+            cudaStreamSynchronize(st);
+    }
     CallScratch(const CallScratch &) = delete;
     CallScratch &operator=(const CallScratch &) = delete;
     static size_t pad(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
@@ -2172,22 +2187,24 @@ extern "C" int p3m_pm_error(int device, int count, const double *n, const double
     if (rc != P3M_OK) return rc;
     // partial sums of every set, [set][2][block]
     const size_t stride = 2 * (size_t)maxb;
-    double *d_part = nullptr;
     cudaStream_t st = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&d_part, (size_t)count * stride * sizeof(double), st);
-    for (int i = 0; e == cudaSuccess && i < count; ++i) {
-        double *q = d_part + (size_t)i * stride;
-        launch_pm_error(kappa[i], alpha[i], p, m_alias, M[i], box[i], q, q + maxb, st);
-        e = cudaGetLastError();
-    }
     std::vector<double> h;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
-        h.resize((size_t)count * stride);
-        e = cudaMemcpyAsync(h.data(), d_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
+        CallScratch scr(st);  // (given back before its stream goes)
+        e = scr.reserve(CallScratch::pad((size_t)count * stride * sizeof(double)));
+        double *d_part = e == cudaSuccess ? scr.take<double>((size_t)count * stride) : nullptr;
+        for (int i = 0; e == cudaSuccess && i < count; ++i) {
+            double *q = d_part + (size_t)i * stride;
+            launch_pm_error(kappa[i], alpha[i], p, m_alias, M[i], box[i], q, q + maxb, st);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) {
+            h.resize((size_t)count * stride);
+            e = cudaMemcpyAsync(h.data(), d_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (d_part) cudaFreeAsync(d_part, st);
     if (st) cudaStreamDestroy(st);
     if (e != cudaSuccess) return fail(nullptr, P3M_ECUDA, "p3m_pm_error", cudaGetErrorString(e));
     for (int i = 0; i < count; ++i) {
