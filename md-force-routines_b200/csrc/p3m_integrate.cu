@@ -741,7 +741,7 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
             o[0] = k * km;
             o[1] = km * km;
             o[2] = up * up;
-            o[3] = exp(-km * km * inv4a2);
+            o[3] = km != 0.0 ? exp(-km * km * inv4a2) : 1.0;  // (1/alpha^2 may overflow)
         }
     }
     __syncwarp();
@@ -765,7 +765,7 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
         num += __shfl_xor_sync(0xffffffffu, num, o);
         den += __shfl_xor_sync(0xffffffffu, den, o);
     }
-    num *= four_pi * exp(-kappa_sq * inv4a2);
+    num *= four_pi * (kappa_sq != 0.0 ? exp(-kappa_sq * inv4a2) : 1.0);
     double g = 0.0, acontrib = 0.0;
     if (have && k_sq != 0.0) {
         g = num / ((den * den) * k_sq);
