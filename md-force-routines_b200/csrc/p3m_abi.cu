@@ -687,14 +687,16 @@ template <typename T> static void seq_pp(p3m_ctx *ctx, bool reduce = true, cudaS
 }
 
 template <typename T>
-static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr, cudaEvent_t assigned = nullptr,
-                   cudaEvent_t sums_free = nullptr)
+static cudaError_t seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr,
+                          cudaEvent_t assigned = nullptr, cudaEvent_t sums_free = nullptr)
 {
     if (!st) st = ctx->st;
     DevState &s = ctx->s;
+    cudaError_t e = cudaSuccess;
     launch_assign<T>(s, st);
-    if (assigned) cudaEventRecord(assigned, st);
-    if (sums_free) cudaStreamWaitEvent(st, sums_free, 0);
+    if (assigned) e = cudaEventRecord(assigned, st);
+    if (e == cudaSuccess && sums_free) e = cudaStreamWaitEvent(st, sums_free, 0);
+    if (e != cudaSuccess) return e;
     launch_fft_forward<T>(s, st);
     if (reduce) {
         launch_reduce_pm(s, st);
@@ -703,6 +705,7 @@ static void seq_pm(p3m_ctx *ctx, bool reduce = true, cudaStream_t st = nullptr, 
     launch_fft_inverse<T>(s, st);
     launch_gather<T>(s, st);
     ctx->launches += 2 + fft_kernel_count(s);
+    return e;
 }
 
 // Compute the influence function of every replica that has none yet.
@@ -739,8 +742,8 @@ template <typename T> static int seq_force(p3m_ctx *ctx)
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
         if (e == cudaSuccess) {
             ctx->launches += launch_place_bricks<T>(s, st2);
-            seq_pm<T>(ctx, true, st2);
-            e = cudaEventRecord(ctx->ev_join, st2);
+            e = seq_pm<T>(ctx, true, st2);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_join, st2);
         }
     }
     launch_scan_cells(s, st);
@@ -834,8 +837,8 @@ static int seq_step(p3m_ctx *ctx, int mode, int record_nqt, int k = 0, bool more
             e = cudaStreamWaitEvent(st2, ctx->ev_fork, 0);
             if (e == cudaSuccess) {
                 ctx->launches += launch_place_bricks<T>(s, st2);
-                seq_pm<T>(ctx, false, st2, pairs_wait ? ctx->ev_asg : nullptr, sums_free);
-                e = cudaEventRecord(ctx->ev_join, st2);
+                e = seq_pm<T>(ctx, false, st2, pairs_wait ? ctx->ev_asg : nullptr, sums_free);
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_join, st2);
             }
         }
         if (e == cudaSuccess && rec) {  // the new positions are final: ring row counters[3]
@@ -1122,7 +1125,7 @@ static int do_pm(p3m_ctx *ctx, const double *pos, const double *Z, double *acc, 
     RET(h2d(ctx, s.pos, pos, sizeof(double) * 3 * s.ntot));
     RET(upload_charge(ctx, Z));
     seq_sort<T>(ctx, true);
-    seq_pm<T>(ctx);
+    CK(seq_pm<T>(ctx));
     launch_combine<T>(s, 0, 1, 0, s.acc, ctx->ep, ctx->st);
     ctx->launches++;
     if (rho) {
