@@ -532,12 +532,15 @@ extern "C" int p3m_create(const p3m_replica_desc *reps, int n_reps, int precisio
     plan_mesh_passes(ctx);
     s.nblk = blk;
     s.max_mesh = maxm;
-    // Threads per particle, from step times (FP32, us per step with 1 / 2 / 4 / 8):
-    // 2e3 particles 61 / 54 / 54 / 53, 1e4 71 / 67 / 74 / 70, 1e5 335 / 318 /
+    // Threads per particle, from step times (us per step with 1 / 2 / 4 / 8).
+    // FP32: 2e3 particles 61 / 54 / 54 / 53, 1e4 71 / 67 / 74 / 70, 1e5 335 / 318 /
     // 340 / 364, 2e5 in 20 replicas 456 / 442 / 469 / 554, 1e6 2270 / 2107 /
-    // 2217 / 2698: four while two would leave most SMs without a block, then
-    // two -- one, though it fills the SMs from 7.6e4 particles on, ends with a
-    // longer last wave of longer blocks.
+    // 2217 / 2698. FP64: 1e3 82 / 55 / 44 / 43, 2e3 136 / 85 / 63 / 53, 1e4 112 /
+    // 71 / 72 / 77, 4e4 197 / 166 / 160 / 170, 1e5 430 / 415 / 427 / 462. Four
+    // while two would leave most SMs without a block, then two -- one, though it
+    // fills the SMs from 7.6e4 particles on, ends with a longer last wave of longer
+    // blocks. (Alone the FP64 pair loop is fastest with eight up to 1e4 particles;
+    // there those blocks crowd the mesh branch of a step.)
     plan_lists(ctx, -1.0, p >= 148 * 64 ? 2 : 4);
 
     auto cleanup = [&](int code) {

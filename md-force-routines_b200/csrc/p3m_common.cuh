@@ -29,15 +29,15 @@ __host__ __device__ constexpr int pencil_log(int logM) { return logM >= 8 ? 4 : 
 __host__ __device__ constexpr int fft_ra(int logM) { return logM >= 7 ? 16 : (logM == 6 ? 8 : 4); }
 __host__ __device__ constexpr int fft_rb(int logM) { return (1 << logM) / fft_ra(logM); }
 constexpr int TWIDDLE_N = 480;
-// Complex lines per item of the x passes (two real rows each): 32, or M/2 for
-// M = 32, so each radix pass has a group for every one of 256 threads; 16 at
-// M = 256, where the shorter items balance the last wave (FFT 0.576 against
-// 0.587 ms at 256^3; at 64^3 16 lines measured 0.144 against 0.130).
 // PP cells are at least (rc + skin) / D wide (D, the cell divisor of a
 // context: 1 or 2), so the neighbours of a particle lie in the (2 D + 1)^3
 // cells around its own.
 constexpr int CELL_DIV_MAX = 2;
-__host__ __device__ constexpr int cell_stencil(int d) { return (2 * d + 1) * (2 * d + 1) * (2 * d + 1); }
+// Complex lines per item of the x passes (two real rows each), log2: 32, or M/2
+// for M = 32, so that the 256 threads have short DFTs of both passes; 16 at M =
+// 256, where shorter items fill the SMs more evenly (FP32, all FFT passes of a
+// step, 16 / 32 lines: 347 / 381 us at 256^3, but 73 / 61 at 128^3 and 130 / 102
+// for 20 meshes of 64^3).
 __host__ __device__ constexpr int x_lines_log(int logM)
 {
     return logM >= 8 ? 4 : (logM - 1 < 5 ? logM - 1 : 5);

@@ -1067,9 +1067,10 @@ constexpr int GTILE = TILE * TILE * GTX;
 // gather_mode 1 takes NC = 1 up to GATHER_SPLIT_MAX bricks (measured, us alone
 // / step with a CTA per brick against three: 8 bricks 16.5 / 51.8 - 8.3 /
 // 46.5, 64 bricks 12.4 / 66.1 - 8.3 / 62.8, FP64 18.5 / 93.1 - 12.4 / 87.5,
-// 512 bricks 28.8 / 310.0 - 26.7 / 308.3) and NC = 3 beyond (step, as the
-// kernel is now: 1280 bricks 403.0 - 402.9, 2056 633.4 - 632.9, 4096 1751 -
-// 1770).
+// 512 bricks 28.8 / 310.0 - 26.7 / 308.3) and NC = 3 beyond (step, medians of
+// six runs from one state: 1280 bricks 395.9 - 396.0, 2048 603.8 - 610, 4096
+// 1711 - 1729; an autotuner run, which compares single timings, may pick either
+// up to 2048).
 constexpr int GATHER_SPLIT_MAX = 512;
 
 template <typename T, int NB, int NC>

@@ -138,7 +138,7 @@ k_build_lists(const RepDev *__restrict__ reps, int nrep, const int *__restrict__
         // the home cell's centre in the integer coordinates
         const U ox = Coord<T>::q(((double)cx + 0.5) / nc), oy = Coord<T>::q(((double)cy + 0.5) / nc),
                 oz = Coord<T>::q(((double)cz + 0.5) / nc);
-        __syncthreads();  // the previous cell is done with pre, nstart and stage
+        __syncthreads();  // the previous cell is done with pre, the row arrays and stage
         // pre = exclusive prefix sum over the rows (one warp holds them all)
         if (tid < 32) {
             int n = 0;

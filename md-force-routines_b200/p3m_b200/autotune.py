@@ -9,10 +9,10 @@ What it searches (p3m_tuning of the C ABI):
   125-cell stencil of small cells, or 27 larger cells whose candidates are
   staged once for many particles);
 * the FFT tiles of meshes up to 64^3: the fused y/z plane kernel (a whole kx
-  plane per CTA) or the y and z pencil passes (16 lines per CTA);
+  plane per CTA) or the y and z pencil passes (32 lines per CTA, 16 at 256^3);
 * the force gather: a CTA per mesh brick with one or two field-tile buffers
   (copy/compute overlap against CTAs per SM), or a CTA per brick and field
-  component (three times the work items);
+  component (three times the work items; what up to 512 bricks take anyway);
 * on the FP32 path, inner lists (dynamic pruning): the pair kernel reads the
   Verlet entries closer than rc + prune_buf and rebuilds those lists itself
   every few steps, which makes larger skins (rarer Verlet rebuilds) cheap.

@@ -19,6 +19,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 COUNTS = {
     # test_gpu_batch_fp64.py
     (0.1, 0.46, 2.975): 128, (0.0, 0.9, 2.975): 256, (6.0, 0.85, 2.975): 512, (40.0, 1.5, 2.975): 0,
+    # test_gpu_pp_table.py, with the four above
+    (1.0, 0.6, 2.975): 128, (3.0, 0.45, 2.975): 256,
     # test_gpu_pp_pair.py
     (0.5, 0.72, 5.0): 512, (2.0, 0.72, 4.9): 512, (0.0, 0.75, 4.8): 512, (3.0, 0.65, 5.1): 512,
     (1.0, 0.3, 3.3): 128, (9.0, 0.6, 5.3): 1024,
