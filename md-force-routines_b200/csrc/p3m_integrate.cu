@@ -682,7 +682,7 @@ k_nqt_reduce(const RepDev *__restrict__ reps, int nrep, int nblk,
 // products or sums of one factor per axis, tabulated per triple; what is left
 // per alias is a division. GF_LANES lanes share a triple: lane a takes the
 // aliases az = a, a + GF_LANES, ... and a fixed shuffle tree adds them.
-// One mesh of 64^3 with three aliases takes 26 us; with every point and an
+// One mesh of 64^3 with three aliases takes 28 us; with every point and an
 // exponential per alias it took 717.
 constexpr int GF_MAXA = 15;    // 2 * m_alias + 1 <= 15
 constexpr int GF_LANES = 8;
@@ -696,6 +696,35 @@ static __host__ __device__ long long gf_triples(int M)
     return U * (U + 1) * (U + 2) / 6;
 }
 
+// exp(-(x / 2 alpha)^2): the rounding of the argument, which the exponential
+// would multiply by the argument's size, is carried beside it. A Gaussian of
+// zero also where x / alpha overflows.
+__device__ __forceinline__ double gauss_factor(double x, double alpha)
+{
+    const double q = x / alpha, s = 0.25 * q * q;
+    if (s >= 800.0) return 0.0;
+    const double rest = fma(-q, alpha, x) / alpha;  // q + rest = x / alpha
+    return exp(-s) * (1.0 - (fma(0.25 * q, q, -s) + 0.5 * q * rest));
+}
+
+// (sin x / x)^n. Around zero, the central aliases: from 1 - sin x / x, a short
+// series, whose rounding is relative to that small difference -- the quotient's
+// own would be raised to the n-th power.
+__device__ __forceinline__ double sinc_power(double x, int n)
+{
+    if (fabs(x) <= 1.6) {
+        const double t = x * x;
+        double w = 1.0;
+#pragma unroll
+        for (int i = 12; i > 1; --i) w = fma(-t * (1.0 / (2 * i * (2 * i + 1))), w, 1.0);
+        return exp(n * log1p(-t * (1.0 / 6.0) * w));
+    }
+    const double v = sin(x) / x;
+    double up = 1.0;
+    for (int q = 0; q < n; ++q) up *= v;
+    return up;
+}
+
 __global__ void __launch_bounds__(GF_THREADS)
 k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__restrict__ G_k,
          double *__restrict__ a_part)
@@ -707,7 +736,7 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
     const double h = L / M;
     const int mid = M / 2;  // (M - 1) / 2 for odd M
     const int na = 2 * m + 1;
-    const double kappa_sq = kappa * kappa, inv4a2 = 0.25 / (alpha * alpha);
+    const double kappa_sq = kappa * kappa;
     const int tl = threadIdx.x / GF_LANES, lane = threadIdx.x % GF_LANES;
     const long long t = blockIdx.x * (long long)GF_TRIPLES + tl;
     const bool have = t < gf_triples(M);
@@ -734,14 +763,11 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
         k_sq += k * k;
         for (int a = lane; a < na; a += GF_LANES) {
             const double km = two_pi * (s + (double)(a - m) * M) / L;
-            const double v = km != 0.0 ? sin(0.5 * km * h) / (0.5 * km * h) : 1.0;
-            double up = 1.0;
-            for (int q = 0; q < p; ++q) up *= v;
             double *o = tab[tl][d][a];
             o[0] = k * km;
             o[1] = km * km;
-            o[2] = up * up;
-            o[3] = km != 0.0 ? exp(-km * km * inv4a2) : 1.0;  // (1/alpha^2 may overflow)
+            o[2] = sinc_power(0.5 * km * h, 2 * p);
+            o[3] = gauss_factor(km, alpha);
         }
     }
     __syncwarp();
@@ -765,7 +791,7 @@ k_gf_opt(double kappa, double alpha, int p, int m, int M, double L, double *__re
         num += __shfl_xor_sync(0xffffffffu, num, o);
         den += __shfl_xor_sync(0xffffffffu, den, o);
     }
-    num *= four_pi * (kappa_sq != 0.0 ? exp(-kappa_sq * inv4a2) : 1.0);
+    num *= four_pi * gauss_factor(kappa, alpha);
     double g = 0.0, acontrib = 0.0;
     if (have && k_sq != 0.0) {
         g = num / ((den * den) * k_sq);
