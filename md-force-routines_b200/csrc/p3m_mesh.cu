@@ -60,7 +60,7 @@ __device__ __forceinline__ int freq(int n, int M) { return n < (M >> 1) ? n : n 
 //
 // Bound: the x passes by the latency of their tile and spectrum reads, the y
 // and z passes by L2 and, at 256^3, HBM (the inverse y pass moves 404 MB in 65
-// us, 6.2 TB/s). Radix-2 passes of three stages through shared memory in
+// us, 6.2 TB/s, some four fifths of it HBM's). Radix-2 passes of three stages through shared memory in
 // bit-reversed order, which this replaced, moved each element through it eight
 // times a line (two now). All passes of a step, before / after, FP32: one 64^3
 // mesh 26 / 19 us, 20 of them 125 / 93, 128^3 85 / 54, 256^3 573 / 330; FP64
